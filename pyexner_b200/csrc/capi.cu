@@ -299,11 +299,13 @@ struct Geometry {
     int band_rows = 0, nstrips = 0, nbands = 0, grid = 0;
 };
 
-// Tallest band of the stage kernel's default geometry (tuning knob; float32 Gaussian bed:
-// 160 and 192 measured alike at 8192^2, 160 ahead of 192 at 4096^2)
-#ifndef PXB_STAGE_MAX_ROWS
-#define PXB_STAGE_MAX_ROWS 176
-#endif
+// Tiles of the stage kernel: warps side by side and on top of one another, rows in shared
+// memory (owned rows of the tallest band and two on each side), launch shape.
+struct StageGeometry {
+    int wx = 1, wy = 1, srows = 0, band_rows = 0, nstrips = 0, nbands = 0, grid = 0, threads = 0;
+    size_t smem = 0;
+};
+
 // CFL work items per resident warp and the shortest band that rule may give (tuning knobs;
 // 4 and 64 against 2 and 32: the same at 2048^2, 10 % faster CFL at 8192^2 with bedload
 // everywhere, where the cubic's cost varies from item to item)
@@ -314,31 +316,83 @@ struct Geometry {
 #define PXB_CFL_MIN_ROWS 64
 #endif
 
-Geometry stage_geometry(int ny, int nx, int esize, int resident_warps, int want_rows) {
-    Geometry g;
-    const int sout = pxb_stage_strip_out(esize);
-    g.nstrips = std::max(1, (nx - 3 + sout - 1) / sout);
-    int rows = want_rows;
-    if (rows <= 0) {
-        // k rounds of items, each with about one item per resident warp (the work queue
-        // hands out the items beyond the first), for the smallest k whose bands are at most
-        // PXB_STAGE_MAX_ROWS tall: a whole number of rounds leaves no partial last round
-        // with idle SMs, and on large grids several rounds of shorter bands keep the
-        // concurrently active items close together in memory (halos shared through L2)
-        const int ipb = pxb_stage_items_per_band(g.nstrips), span = ny - 1;
-        int k = 1, bands = std::max(1, resident_warps / ipb);
-        while ((span + bands - 1) / bands > PXB_STAGE_MAX_ROWS) bands = std::max(1, ++k * resident_warps / ipb);
-        rows = std::max(8, (span + bands - 1) / bands);
-    }
-    g.band_rows = rows;
-    g.nbands = std::max(1, (ny - 1 + rows - 1) / rows);
-    const int items = pxb_stage_items_per_band(g.nstrips) * g.nbands;
-    // Unless the grid is small, launch exactly the resident capacity: every SM then holds
-    // the same number of blocks (a grid a little below capacity is spread unevenly by the
-    // block scheduler), and the kernel's work queue hands out the items beyond one per warp.
-    const int need = std::max(1, (items + 3) / 4), cap = std::max(1, resident_warps / 4);
-    g.grid = need >= cap / 4 ? cap : need;
+// Dynamic shared memory a stage block may ask for (of 227 KB a block can have; the budget
+// instantiation also has 1 KB of its own).
+constexpr size_t STAGE_SMEM_MAX = 224 * 1024;
+
+cudaError_t allow_smem(int dtype, bool mpm, bool mask, pxb::StageUse use) {
+    return dtype == PXB_F64 ? pxb::stage_allow_smem<double>(mpm, mask, use, STAGE_SMEM_MAX)
+                            : pxb::stage_allow_smem<float>(mpm, mask, use, STAGE_SMEM_MAX);
+}
+
+// Tiles of the stage kernel on an ny x nx grid: wx warps side by side, wy on top of one
+// another, bands of about `rows` rows.
+StageGeometry stage_tiles(int ny, int nx, int esize, int wx, int wy, int rows) {
+    StageGeometry g;
+    g.wx = wx;
+    g.wy = wy;
+    g.nstrips = pxb::stage_strips(nx, wx);
+    // bands of at least two rows (a ring row and its donors' row share a tile) that fit in
+    // shared memory
+    const size_t cap = STAGE_SMEM_MAX / esize;
+    while (rows > 2 && pxb::stage_smem_elems(wx, rows + 5) > cap) --rows;
+    g.nbands = std::max(1, std::min(ny / 2, (ny + rows - 1) / rows));
+    g.band_rows = (ny + g.nbands - 1) / g.nbands;
+    g.srows = g.band_rows + 4;
+    g.smem = pxb::stage_smem_elems(wx, g.srows) * esize;
+    g.threads = 32 * wx * wy;
+    g.grid = g.nstrips * g.nbands;
     return g;
+}
+
+// Estimated time of `grid` tiles of this shape, all with `srows` shared rows, in units of
+// the issue slots one warp takes for one row.  Every warp marches over its share of the
+// tile's rows and EXTRA more (the face row shared with the warp below, first loads,
+// barriers, stores); with few warps a scheduler loses slots (FEW) and a row takes at least
+// LATENCY; a wave of blocks costs START more.  The last, partial wave costs its busiest SM's
+// blocks, less (down to TAIL) the emptier it is.  The constants are fitted to timed sweeps
+// of 15 to 50 tilings each at 21 sizes from 48^2 to 8192^2 (float32) and 10 from 64^2 to
+// 2048^2 (float64): the tiling picked is within 2 % of the fastest of its sweep on average.
+double stage_cost(const StageGeometry& g, int esize, int sm_count) {
+    const bool f64 = esize == 8;
+    const double LATENCY = f64 ? 4 : 6.5, START = f64 ? 6 : 4, FEW = f64 ? 0.2 : 1.4, EXTRA = f64 ? 2 : 4, TAIL = f64 ? 0.5 : 0.3;
+    const int sm_threads = pxb::stage_max_threads(esize) * pxb::stage_min_blocks(esize);
+    // 196 KB is the largest shared-memory carveout below all of it: the L1 cache keeps 60 KB
+    // (three blocks of 67 KB, which leave it 28 KB, are 4 % slower at 8192^2 than of 64 KB)
+    const int resident = std::max(1, (int)std::min<size_t>(sm_threads / g.threads, (size_t)(196 * 1024) / (g.smem + 1024)));
+    const double per_sm = (double)g.grid / sm_count, share = (double)g.srows / g.wy + EXTRA;
+    auto wave = [&](double blocks) {  // co-resident blocks of one SM
+        const double warps = blocks * g.threads / 128.0;  // per scheduler
+        return std::max((warps + FEW) * share, share * LATENCY) + START;
+    };
+    const double full = std::floor(per_sm / resident), rem = per_sm - full * resident;
+    double t = full * wave(resident);
+    if (rem > 1e-9) t += wave(std::ceil(rem)) * (full > 0 ? TAIL + (1 - TAIL) * rem / resident : 1.0);
+    return t;
+}
+
+// Block shapes (warps side by side, on top of one another) the tilings are chosen from.
+constexpr int STAGE_SHAPES[][2] = {{1, 4}, {1, 8}, {2, 4}, {4, 2}, {2, 6}, {3, 4}};
+
+// The cheapest tiling of a grid by stage_cost; want_rows > 0 asks for that band height.
+StageGeometry stage_geometry(int ny, int nx, int esize, int sm_count, int want_rows) {
+    StageGeometry best;
+    double best_cost = 0;
+    for (const auto& sh : STAGE_SHAPES) {
+        if (32 * sh[0] * sh[1] > pxb::stage_max_threads(esize)) continue;
+        int last = 0;
+        for (int rows = want_rows > 0 ? want_rows : 64; rows >= (want_rows > 0 ? want_rows : 4); --rows) {
+            const StageGeometry g = stage_tiles(ny, nx, esize, sh[0], sh[1], rows);
+            if (g.nbands == last) continue;
+            last = g.nbands;
+            const double cost = stage_cost(g, esize, sm_count);
+            if (best.grid == 0 || cost < best_cost) {
+                best = g;
+                best_cost = cost;
+            }
+        }
+    }
+    return best;
 }
 
 Geometry cfl_geometry(int ny, int nx, int resident_warps) {
@@ -500,13 +554,18 @@ void fill_sed(pxb::SedTable<T>& S, const double* seds, int nsed) {
     S.one_minus_por = (T)(1.0 - por_sum / nsed);
     S.inv_one_minus_por = (T)(1.0 / (1.0 - por_sum / nsed));
     S.n_p_mix = (T)(std::pow(d50f_sum / nsed, 1.0 / 6.0) / 21.1);
+    double move = 0;
     for (int k = 0; k < nsed; ++k) {
         const double frac = seds[0 * nsed + k], d50 = seds[1 * nsed + k], dens = seds[2 * nsed + k];
         const double s = dens / 1000.0;
         const double np_ = std::pow(d50, 1.0 / 6.0) / 21.1;
         S.k_theta[k] = (T)(np_ * np_ / ((s - 1.0) * d50));
         S.k_g1[k] = (T)(8.0 * frac * (np_ * (np_ * np_)) * std::sqrt(9.81) / (s - 1.0));
+        // a threshold that is not positive lets every wet cell move
+        const double q = np_ * np_ / ((s - 1.0) * d50) / (0.9999 * seds[5 * nsed + k]);
+        move = std::max(move, q > 0 && std::isfinite(q) ? q * q * q : HUGE_VAL);
     }
+    S.k_move = (T)move;
 }
 
 struct PlanCommon {
@@ -679,7 +738,7 @@ struct pxb_re_plan {
     int nsed = 0;
     int mpm = 0;
     const uint8_t* nodata = nullptr;
-    Geometry stage[8];  // by (mpm, mask, avg) variant: band geometry from its occupancy
+    StageGeometry stage;
     int want_rows = 0;
     pxb::SedTable<float> sedf;
     pxb::SedTable<double> sedd;
@@ -710,7 +769,7 @@ struct pxb_re_ens {
     int dtype = 0, mpm = 0, nm = 0;
     int band_rows = 0;
     int sm_count = 0;
-    int bps[2] = {1, 1};  // resident stage blocks per SM: plain, averaged
+    StageGeometry tile;  // wx, wy and shared rows common to the members
     bool has_mask = false;
     std::vector<EnsMember> m;
     std::vector<void*> owned;           // zero nodata planes of members without one
@@ -842,18 +901,17 @@ int re_stage_impl(pxb_re_plan* P, const pxb_re_fields* in, const pxb_re_fields* 
     a.dt = (const T*)dt;
     a.ring = P->c.ring;
     a.sed = sed_of<T>(P);
-    const int v = (P->mpm ? 4 : 0) | (P->nodata ? 2 : 0) | (avg ? 1 : 0);
-    const Geometry& g = P->stage[v];
-    a.band_rows = g.band_rows;
+    const StageGeometry& g = P->stage;
+    a.wx = g.wx;
+    a.srows = g.srows;
     a.nstrips = g.nstrips;
     a.nbands = g.nbands;
     a.err = &P->c.scr->err;
-    a.queue = P->c.scr->queue;
-    const long long nitems = (long long)pxb_stage_items_per_band(g.nstrips) * g.nbands;
+    const long long nitems = g.grid;
     const bool bud = bud_w > 0.0 && P->bud_acc && P->bud_part;
     if (bud && nitems > P->bud_items) return fail(PXB_ERR_ARG, "budget partials smaller than the band geometry");
     if (bud) a.bud = P->bud_part;
-    PXB_CUDA(pxb::launch_re_stage<T>(a, P->mpm != 0, P->nodata != nullptr, avg != nullptr, g.grid, s));
+    PXB_CUDA(pxb::launch_re_stage<T>(a, P->mpm != 0, P->nodata != nullptr, avg != nullptr, g.grid, g.threads, g.smem, s));
     if (bud)
         PXB_CUDA(pxb::launch_budget_stage<T>(P->bud_part, (int)nitems, (const T*)dt, bud_w * P->c.dx, P->bud_acc, s));
     return PXB_OK;
@@ -989,18 +1047,10 @@ int re_init_impl(pxb_re_plan* P, const pxb_re_fields* f, cudaStream_t s) {
 // averaged with a; a is not written); the fastest is kept for every variant.
 template <class T>
 int re_autotune_impl(pxb_re_plan* P, const pxb_re_fields* A, const pxb_re_fields* B, cudaStream_t s, int32_t* out) {
-    const bool f64 = P->c.dtype == PXB_F64;
-    auto set_rows = [&](int rows) {
-        for (int v = 0; v < 8; ++v) {
-            const bool mpm = v & 4, hm = v & 2, avg = v & 1;
-            const int bps = f64 ? pxb::re_stage_blocks_per_sm<double>(mpm, hm, avg)
-                                : pxb::re_stage_blocks_per_sm<float>(mpm, hm, avg);
-            P->stage[v] = stage_geometry(P->c.ny, P->c.nx, f64 ? 8 : 4, std::max(1, bps) * 4 * P->c.sm_count, rows);
-        }
-    };
+    auto set_rows = [&](int rows) { P->stage = stage_geometry(P->c.ny, P->c.nx, (int)sizeof(T), P->c.sm_count, rows); };
     set_rows(0);
-    const int r0 = P->stage[(P->mpm ? 4 : 0) | (P->nodata ? 2 : 0)].band_rows;
-    std::vector<int> cand = {r0, 2 * r0, 3 * r0, 4 * r0, 8, 16, 24, 32, 48, 64, 96, 128, 192, 256};
+    const int r0 = P->stage.band_rows;
+    std::vector<int> cand = {r0, 2 * r0, 8, 12, 16, 24, 32, 48, 64, 96};
     std::vector<int> uniq;
     for (int c : cand)
         if (c >= 8 && c <= std::max(8, P->c.ny) && std::find(uniq.begin(), uniq.end(), c) == uniq.end())
@@ -1223,10 +1273,11 @@ pxb::REStageArgs<T> ens_stage_args(const pxb_re_ens* E, int k, const pxb_re_fiel
     a.dt = (const T*)E->dt + k;
     a.ring = mb.ring;
     a.sed = ens_sed<T>(E);
-    a.band_rows = E->band_rows;
-    const int sout = pxb_stage_strip_out((int)sizeof(T));
-    a.nstrips = std::max(1, (mb.nx - 3 + sout - 1) / sout);
-    a.nbands = std::max(1, (mb.ny - 1 + E->band_rows - 1) / E->band_rows);
+    const StageGeometry g = stage_tiles(mb.ny, mb.nx, (int)sizeof(T), E->tile.wx, E->tile.wy, E->band_rows);
+    a.wx = g.wx;
+    a.srows = E->tile.srows;
+    a.nstrips = g.nstrips;
+    a.nbands = g.nbands;
     a.err = &E->scr[k].err;
     return a;
 }
@@ -1236,6 +1287,27 @@ template <class T>
 int ens_build_stage_tables(pxb_re_ens* E) {
     std::vector<pxb::REStageArgs<T>> t[4];
     std::vector<int> base(1, 0);
+    // the block shape by the cost of all members' tiles together; the tallest band of any
+    // member sizes the shared memory
+    double best_cost = 0;
+    E->tile = StageGeometry();
+    for (const auto& sh : STAGE_SHAPES) {
+        if (32 * sh[0] * sh[1] > pxb::stage_max_threads((int)sizeof(T))) continue;
+        StageGeometry all;
+        for (const EnsMember& mb : E->m) {
+            const StageGeometry g = stage_tiles(mb.ny, mb.nx, (int)sizeof(T), sh[0], sh[1], E->band_rows);
+            const int grid = all.grid + g.grid, srows = std::max(all.srows, g.srows);
+            all = g;
+            all.grid = grid;
+            all.srows = srows;
+        }
+        all.smem = pxb::stage_smem_elems(all.wx, all.srows) * sizeof(T);
+        const double cost = stage_cost(all, (int)sizeof(T), E->sm_count);
+        if (E->tile.grid == 0 || cost < best_cost) {
+            E->tile = all;
+            best_cost = cost;
+        }
+    }
     for (int k = 0; k < E->nm; ++k) {
         const EnsMember& mb = E->m[(size_t)k];
         pxb_re_fields b_noG = mb.b;  // SSPRK2 stage 1 in MPM mode: G is recomputed by stage 2
@@ -1245,7 +1317,7 @@ int ens_build_stage_tables(pxb_re_ens* E) {
         t[2].push_back(ens_stage_args<T>(E, k, &mb.b, &mb.a, &mb.a, &mb.a));
         t[3].push_back(ens_stage_args<T>(E, k, &mb.a, &b_noG, nullptr, &mb.a));
         const pxb::REStageArgs<T>& a = t[0].back();
-        base.push_back(base.back() + pxb_stage_items_per_band(a.nstrips) * a.nbands);
+        base.push_back(base.back() + a.nstrips * a.nbands);
     }
     for (int v = 0; v < 4; ++v) {
         if (!E->st_args[v]) PXB_CUDA(cudaMalloc(&E->st_args[v], sizeof(pxb::REStageArgs<T>) * E->nm));
@@ -1308,10 +1380,7 @@ int ens_stage_launch(pxb_re_ens* E, int v, cudaStream_t s) {
     a.args = (const pxb::REStageArgs<T>*)E->st_args[v];
     a.base = E->st_base;
     a.nmembers = E->nm;
-    a.queue = E->scr[0].queue;
-    const bool avg = v == 2;
-    const int grid = std::max(1, std::min((E->st_total + 3) / 4, std::max(1, E->bps[avg ? 1 : 0]) * E->sm_count));
-    PXB_CUDA(pxb::launch_ens_stage<T>(a, E->mpm != 0, E->has_mask, avg, grid, s));
+    PXB_CUDA(pxb::launch_ens_stage<T>(a, E->mpm != 0, E->has_mask, v == 2, E->st_total, E->tile.threads, E->tile.smem, s));
     return PXB_OK;
 }
 
@@ -1393,7 +1462,7 @@ int ens_run_impl(pxb_re_ens* E, int nsteps, int scheme, double cfl, void* dt_log
 // Candidate band heights timed on stage 1 (a -> b) of the current states; keeps the fastest.
 template <class T>
 int ens_autotune_impl(pxb_re_ens* E, cudaStream_t s, int32_t* out) {
-    static const int cand[] = {8, 12, 16, 24, 32, 48, 64, 96, 128, 160, 192, 256};
+    static const int cand[] = {8, 12, 16, 24, 32, 48, 64, 96};
     int st = ens_build_cfl_tables<T>(E, 0.5, nullptr);
     if (st != PXB_OK) return st;
     st = ens_cfl_launch<T>(E, 0, s);  // a dt to run the stage with (the states are not touched)
@@ -2146,11 +2215,13 @@ int re_plan_create(const pxb_re_config* cfg, DevArena* A, pxb_re_plan** out) {
         fill_sed_dual(P->sedD, P->seds.data(), nullptr, P->nsed);
     }
     const bool f64 = cfg->dtype == PXB_F64;
-    for (int v = 0; v < 8; ++v) {
-        const bool mpm = v & 4, hm = v & 2, avg = v & 1;
-        const int bps = f64 ? pxb::re_stage_blocks_per_sm<double>(mpm, hm, avg)
-                            : pxb::re_stage_blocks_per_sm<float>(mpm, hm, avg);
-        P->stage[v] = stage_geometry(cfg->ny, cfg->nx, f64 ? 8 : 4, std::max(1, bps) * 4 * P->c.sm_count, cfg->band_rows);
+    P->stage = stage_geometry(cfg->ny, cfg->nx, f64 ? 8 : 4, P->c.sm_count, cfg->band_rows);
+    const cudaError_t es = allow_smem(cfg->dtype, cfg->mpm != 0, cfg->nodata != nullptr, pxb::STAGE_PLAN);
+    if (es != cudaSuccess) {
+        if (!P->c.ws) cudaFree(P->gen);
+        P->c.release();
+        delete P;
+        return fail(PXB_ERR_CUDA, std::string("stage kernel shared memory: ") + cudaGetErrorString(es));
     }
     const int cb = f64 ? pxb::re_cfl_blocks_per_sm<double>(cfg->nodata != nullptr)
                        : pxb::re_cfl_blocks_per_sm<float>(cfg->nodata != nullptr);
@@ -2284,10 +2355,9 @@ int pxb_re_set_budget(pxb_re_plan* P, double* acc_dev) {
         return fail(PXB_ERR_UNSUPPORTED, "the volume budget is built into the fused stage path only");
     if (acc_dev && ((uintptr_t)acc_dev & 7u)) return fail(PXB_ERR_ARG, "acc_dev must be 8-byte aligned");
     if (acc_dev && !P->bud_part) {
-        // every band geometry the plan can take: bands of one row at least
-        const int nstrips = std::max(1, (P->c.nx - 3 + pxb_stage_strip_out((int)P->c.esize()) - 1) /
-                                            pxb_stage_strip_out((int)P->c.esize()));
-        const long long items = (long long)pxb_stage_items_per_band(nstrips) * P->c.ny;
+        // every tiling the plan can take: one warp wide, bands of one row at least
+        const long long items = (long long)pxb::stage_strips(P->c.nx, 1) * P->c.ny;
+        PXB_CUDA(allow_smem(P->c.dtype, P->mpm != 0, P->nodata != nullptr, pxb::STAGE_BUDGET));
         PXB_CUDA(cudaMalloc(&P->bud_part, sizeof(double) * 2 * (size_t)items));
         P->bud_items = items;
     }
@@ -2407,7 +2477,7 @@ int pxb_re_ens_create(const pxb_re_ens_config* cfg, pxb_re_ens** out) {
     E->dtype = cfg->dtype;
     E->mpm = cfg->mpm;
     E->nm = cfg->nmembers;
-    E->band_rows = cfg->band_rows > 0 ? cfg->band_rows : 64;
+    E->band_rows = cfg->band_rows > 0 ? cfg->band_rows : 40;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&E->sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
@@ -2476,9 +2546,8 @@ int pxb_re_ens_create(const pxb_re_ens_config* cfg, pxb_re_ens** out) {
         cudaMalloc(&E->dt, es * E->nm) != cudaSuccess || cudaMemset(E->dt, 0, es * E->nm) != cudaSuccess ||
         cudaStreamCreateWithFlags(&E->cap, cudaStreamNonBlocking) != cudaSuccess)
         return bail(fail(PXB_ERR_CUDA, "ensemble scratch"));
-    for (int v = 0; v < 2; ++v)
-        E->bps[v] = E->dtype == PXB_F64 ? pxb::ens_stage_blocks_per_sm<double>(E->mpm != 0, E->has_mask, v == 1)
-                                        : pxb::ens_stage_blocks_per_sm<float>(E->mpm != 0, E->has_mask, v == 1);
+    if (allow_smem(E->dtype, E->mpm != 0, E->has_mask, pxb::STAGE_ENSEMBLE) != cudaSuccess)
+        return bail(fail(PXB_ERR_CUDA, "stage kernel shared memory"));
     int st = E->dtype == PXB_F64 ? ens_build_stage_tables<double>(E) : ens_build_stage_tables<float>(E);
     if (st != PXB_OK) return bail(st);
     *out = E;

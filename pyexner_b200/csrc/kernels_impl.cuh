@@ -1,52 +1,62 @@
 // Launchers shared by the float and double translation units.
 #pragma once
+#include <type_traits>
+
 #include "pxb_launch.h"
 
 namespace pxb {
 
-template <class T, bool MPM, bool HM, bool AVG>
-static cudaError_t stage_variant(const REStageArgs<T>& a, int grid, cudaStream_t s) {
-    // the budget variant only when its partial array is set (the others carry no budget code)
-    if (a.bud) re_stage_kernel<T, MPM, HM, AVG, true><<<grid, 128, 0, s>>>(a);
-    else re_stage_kernel<T, MPM, HM, AVG, false><<<grid, 128, 0, s>>>(a);
-    return cudaGetLastError();
-}
-
-template <class T>
-cudaError_t launch_re_stage(const REStageArgs<T>& a, bool mpm, bool hm, bool avg, int grid, cudaStream_t s) {
-    const int key = (mpm ? 4 : 0) | (hm ? 2 : 0) | (avg ? 1 : 0);
-    switch (key) {
-        case 0: return stage_variant<T, false, false, false>(a, grid, s);
-        case 1: return stage_variant<T, false, false, true>(a, grid, s);
-        case 2: return stage_variant<T, false, true, false>(a, grid, s);
-        case 3: return stage_variant<T, false, true, true>(a, grid, s);
-        case 4: return stage_variant<T, true, false, false>(a, grid, s);
-        case 5: return stage_variant<T, true, false, true>(a, grid, s);
-        case 6: return stage_variant<T, true, true, false>(a, grid, s);
-        default: return stage_variant<T, true, true, true>(a, grid, s);
+// Calls f with the compile-time flags (MPM, mask, averaged) of a stage kernel.
+template <class F>
+static cudaError_t stage_dispatch(bool mpm, bool hm, bool avg, F f) {
+    using std::false_type;
+    using std::true_type;
+    switch ((mpm ? 4 : 0) | (hm ? 2 : 0) | (avg ? 1 : 0)) {
+        case 0: return f(false_type{}, false_type{}, false_type{});
+        case 1: return f(false_type{}, false_type{}, true_type{});
+        case 2: return f(false_type{}, true_type{}, false_type{});
+        case 3: return f(false_type{}, true_type{}, true_type{});
+        case 4: return f(true_type{}, false_type{}, false_type{});
+        case 5: return f(true_type{}, false_type{}, true_type{});
+        case 6: return f(true_type{}, true_type{}, false_type{});
+        default: return f(true_type{}, true_type{}, true_type{});
     }
 }
 
-template <class T, bool MPM, bool HM, bool AVG>
-static int stage_occ() {
-    int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, re_stage_kernel<T, MPM, HM, AVG>, 128, 0);
-    return n;
+template <class T>
+cudaError_t launch_re_stage(const REStageArgs<T>& a, bool mpm, bool hm, bool avg, int grid, int threads, size_t smem,
+                            cudaStream_t s) {
+    return stage_dispatch(mpm, hm, avg, [&](auto M, auto H, auto A) {
+        constexpr bool m = decltype(M)::value, h = decltype(H)::value, v = decltype(A)::value;
+        // the budget variant only when its partial array is set (the others carry no budget code)
+        if (a.bud) re_stage_kernel<T, m, h, v, true><<<grid, threads, smem, s>>>(a);
+        else re_stage_kernel<T, m, h, v, false><<<grid, threads, smem, s>>>(a);
+        return cudaGetLastError();
+    });
 }
 
 template <class T>
-int re_stage_blocks_per_sm(bool mpm, bool hm, bool avg) {
-    const int key = (mpm ? 4 : 0) | (hm ? 2 : 0) | (avg ? 1 : 0);
-    switch (key) {
-        case 0: return stage_occ<T, false, false, false>();
-        case 1: return stage_occ<T, false, false, true>();
-        case 2: return stage_occ<T, false, true, false>();
-        case 3: return stage_occ<T, false, true, true>();
-        case 4: return stage_occ<T, true, false, false>();
-        case 5: return stage_occ<T, true, false, true>();
-        case 6: return stage_occ<T, true, true, false>();
-        default: return stage_occ<T, true, true, true>();
-    }
+cudaError_t launch_ens_stage(const EnsStageArgs<T>& a, bool mpm, bool hm, bool avg, int grid, int threads, size_t smem,
+                             cudaStream_t s) {
+    return stage_dispatch(mpm, hm, avg, [&](auto M, auto H, auto A) {
+        constexpr bool m = decltype(M)::value, h = decltype(H)::value, v = decltype(A)::value;
+        ens_stage_kernel<T, m, h, v><<<grid, threads, smem, s>>>(a);
+        return cudaGetLastError();
+    });
+}
+
+template <class T>
+cudaError_t stage_allow_smem(bool mpm, bool hm, StageUse use, size_t bytes) {
+    cudaError_t e = cudaSuccess;
+    for (int avg = 0; avg < 2 && e == cudaSuccess; ++avg)
+        e = stage_dispatch(mpm, hm, avg != 0, [&](auto M, auto H, auto A) {
+            constexpr bool m = decltype(M)::value, h = decltype(H)::value, v = decltype(A)::value;
+            const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+            if (use == STAGE_PLAN) return cudaFuncSetAttribute(re_stage_kernel<T, m, h, v, false>, at, (int)bytes);
+            if (use == STAGE_BUDGET) return cudaFuncSetAttribute(re_stage_kernel<T, m, h, v, true>, at, (int)bytes);
+            return cudaFuncSetAttribute(ens_stage_kernel<T, m, h, v>, at, (int)bytes);
+        });
+    return e;
 }
 
 template <class T>
@@ -78,49 +88,6 @@ cudaError_t launch_bc(const BcArgs<T>& a, cudaStream_t s) {
     bc_gather_kernel<T><<<g, 256, 0, s>>>(a);
     bc_scatter_kernel<T><<<g, 256, 0, s>>>(a);
     return cudaGetLastError();
-}
-
-template <class T, bool MPM, bool HM, bool AVG>
-static cudaError_t ens_variant(const EnsStageArgs<T>& a, int grid, cudaStream_t s) {
-    ens_stage_kernel<T, MPM, HM, AVG><<<grid, 128, 0, s>>>(a);
-    return cudaGetLastError();
-}
-
-template <class T>
-cudaError_t launch_ens_stage(const EnsStageArgs<T>& a, bool mpm, bool hm, bool avg, int grid, cudaStream_t s) {
-    const int key = (mpm ? 4 : 0) | (hm ? 2 : 0) | (avg ? 1 : 0);
-    switch (key) {
-        case 0: return ens_variant<T, false, false, false>(a, grid, s);
-        case 1: return ens_variant<T, false, false, true>(a, grid, s);
-        case 2: return ens_variant<T, false, true, false>(a, grid, s);
-        case 3: return ens_variant<T, false, true, true>(a, grid, s);
-        case 4: return ens_variant<T, true, false, false>(a, grid, s);
-        case 5: return ens_variant<T, true, false, true>(a, grid, s);
-        case 6: return ens_variant<T, true, true, false>(a, grid, s);
-        default: return ens_variant<T, true, true, true>(a, grid, s);
-    }
-}
-
-template <class T, bool MPM, bool HM, bool AVG>
-static int ens_occ() {
-    int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ens_stage_kernel<T, MPM, HM, AVG>, 128, 0);
-    return n;
-}
-
-template <class T>
-int ens_stage_blocks_per_sm(bool mpm, bool hm, bool avg) {
-    const int key = (mpm ? 4 : 0) | (hm ? 2 : 0) | (avg ? 1 : 0);
-    switch (key) {
-        case 0: return ens_occ<T, false, false, false>();
-        case 1: return ens_occ<T, false, false, true>();
-        case 2: return ens_occ<T, false, true, false>();
-        case 3: return ens_occ<T, false, true, true>();
-        case 4: return ens_occ<T, true, false, false>();
-        case 5: return ens_occ<T, true, false, true>();
-        case 6: return ens_occ<T, true, true, false>();
-        default: return ens_occ<T, true, true, true>();
-    }
 }
 
 template <class T>
@@ -185,15 +152,15 @@ cudaError_t launch_roe_cfl(const CflArgs<T>& a, int grid, cudaStream_t s) {
 }
 
 #define PXB_INSTANTIATE(T)                                                                              \
-    template cudaError_t launch_re_stage<T>(const REStageArgs<T>&, bool, bool, bool, int, cudaStream_t); \
-    template int re_stage_blocks_per_sm<T>(bool, bool, bool);                                           \
+    template cudaError_t launch_re_stage<T>(const REStageArgs<T>&, bool, bool, bool, int, int, size_t, cudaStream_t); \
+    template cudaError_t stage_allow_smem<T>(bool, bool, StageUse, size_t);                             \
     template cudaError_t launch_re_cfl<T>(const CflArgs<T>&, bool, int, cudaStream_t);                  \
     template int re_cfl_blocks_per_sm<T>(bool);                                                         \
     template cudaError_t launch_re_init<T>(const InitArgs<T>&, cudaStream_t);                           \
     template cudaError_t launch_bc<T>(const BcArgs<T>&, cudaStream_t);                                  \
     template cudaError_t launch_re_general<T>(const GenArgs<T>&, int, cudaStream_t);                    \
-    template cudaError_t launch_ens_stage<T>(const EnsStageArgs<T>&, bool, bool, bool, int, cudaStream_t); \
-    template int ens_stage_blocks_per_sm<T>(bool, bool, bool);                                          \
+    template cudaError_t launch_ens_stage<T>(const EnsStageArgs<T>&, bool, bool, bool, int, int, size_t, \
+                                             cudaStream_t);                                             \
     template cudaError_t launch_ens_cfl<T>(const EnsCflArgs<T>&, bool, int, cudaStream_t);              \
     template cudaError_t launch_set_time<T>(CflScratch*, double, cudaStream_t);                         \
     template cudaError_t launch_roe_stage<T>(const RoeArgs<T>&, bool, cudaStream_t);                    \

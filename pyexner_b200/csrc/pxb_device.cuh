@@ -115,7 +115,12 @@ __device__ __forceinline__ HCell<T> make_hcell(T h, T hu, T hv, T zb, T z, T nb)
 // Roe-Exner fluctuations of one face (roe_exner.py:312-533).  YF selects the y-face
 // orientation (normal (0,-1): normal velocity -v, tangential u); otherwise (1,0).
 // Outputs upwP (to cell j) and upwM (to cell i) in (h, hu, hv).
-template <class T, bool YF>
+// WARP: every lane of the warp evaluates a face, so warp votes may skip work.  Where every
+// face is subcritical (both cells and the Roe state: |u| < c), no entropy fix applies, the
+// first wave goes to cell i and the third to cell j: the speeds u -+ c of the cells and the
+// wave split are left out (the same bits but for the sign of zeros; measured on the float32
+// 2048^2 Gaussian bed together with the sediment vote of the stage kernel).
+template <class T, bool YF, bool WARP = false>
 __device__ __forceinline__ void roe_exner_face(const HCell<T>& I, const HCell<T>& J, T dx, T P[3], T M[3]) {
     const T uhi = YF ? -I.v : I.u, vhi = YF ? I.u : I.v;
     const T uhj = YF ? -J.v : J.u, vhj = YF ? J.u : J.v;
@@ -134,20 +139,19 @@ __device__ __forceinline__ void roe_exner_face(const HCell<T>& I, const HCell<T>
         ut = (uhi * I.sq + uhj * J.sq) / den;
         vt = (vhi * I.sq + vhj * J.sq) / den;
     }
+    bool sub = false;
+    if constexpr (WARP) sub = __all_sync(FULL, fabs(uhi) < I.c && fabs(uhj) < J.c && fabs(ut) < ct);
     const T l1r = ut - ct;
     const T l3r = ut + ct;
     // Harten-Hyman (roe_exner.py:357-371); the VEL_TOL guard only in the lambda_3 speed
     T l1 = l1r, lE1 = T(0);
-    const T ei = uhi - I.c, ej = uhj - J.c;
-    const bool m1 = (ei < T(0)) && (ej > T(0));
     T l3 = l3r, lE3 = T(0);
-    const T fi = uhi + I.c, fj = uhj + J.c;
-    const bool m3 = (fi < T(0)) && (fj > T(0));
-    // transonic faces are rare: the float build skips the block for the whole warp
-    // when no lane needs it (all lanes evaluate every face, so the vote is safe)
-    bool need = true;
-    if constexpr (is_f32<T>()) need = __any_sync(FULL, m1 || m3);
-    if (need) {
+    bool m1 = false, m3 = false;
+    if (!sub) {
+        const T ei = uhi - I.c, ej = uhj - J.c;
+        m1 = (ei < T(0)) && (ej > T(0));
+        const T fi = uhi + I.c, fj = uhj + J.c;
+        m3 = (fi < T(0)) && (fj > T(0));
         if (m1) {
             const T t = ei * (ej - l1r) / (ej - ei);
             lE1 = l1r - t;
@@ -194,30 +198,36 @@ __device__ __forceinline__ void roe_exner_face(const HCell<T>& I, const HCell<T>
         //   upwP = (A1 + A3, A1 l1 + A3 l3, (A1 + A3) vt + [ut > 0] w2 ct)
         //   upwM = the same with T_k - A_k and [ut <= 0].
         // (b1, w2c, e1, e3 are rounded products, so each sum below has one product to fuse)
-        // When no face of the warp needs the entropy fix (the vote above; lambda_E = 0) the
-        // e_k terms are dropped for the whole warp; they add only zeros then (the sign of a
-        // zero flux component may differ, which no update can see).
         const float w1 = __fmaf_rn(l1, a1, -b1), w2c = mul_rn(ut * a2, ct), w3 = __fmaf_rn(l3, a3, -b3);
-        float A1, A3, B1, B3;
-        if (need) {
-            const float e1 = mul_rn(lE1, a1), e3 = mul_rn(lE3, a3);
-            A1 = (l1 > 0.f ? w1 : 0.f) + (lE1 > 0.f ? e1 : 0.f);
-            A3 = (l3 > 0.f ? w3 : 0.f) + (lE3 > 0.f ? e3 : 0.f);
-            B1 = (w1 + e1) - A1;
-            B3 = (w3 + e3) - A3;
-        } else {
-            A1 = l1 > 0.f ? w1 : 0.f;
-            A3 = l3 > 0.f ? w3 : 0.f;
-            B1 = w1 - A1;  // as (w1 + e1) - A1, NaN included
-            B3 = w3 - A3;
-        }
         const bool s2 = ut > 0.f;
-        p0 = A1 + A3;
-        p1 = sum2(A1, l1, A3, l3);
+        if (sub) {  // A1 = 0, A3 = w3
+            p0 = w3;
+            p1 = mul_rn(w3, l3);
+            n0 = w1;
+            n1 = mul_rn(w1, l1);
+        } else {
+            const float e1 = mul_rn(lE1, a1), e3 = mul_rn(lE3, a3);
+            const float A1 = (l1 > 0.f ? w1 : 0.f) + (lE1 > 0.f ? e1 : 0.f);
+            const float A3 = (l3 > 0.f ? w3 : 0.f) + (lE3 > 0.f ? e3 : 0.f);
+            const float B1 = (w1 + e1) - A1;
+            const float B3 = (w3 + e3) - A3;
+            p0 = A1 + A3;
+            p1 = sum2(A1, l1, A3, l3);
+            n0 = B1 + B3;
+            n1 = sum2(B1, l1, B3, l3);
+        }
         p2 = __fmaf_rn(p0, vt, s2 ? w2c : 0.f);
-        n0 = B1 + B3;
-        n1 = sum2(B1, l1, B3, l3);
         n2 = __fmaf_rn(n0, vt, s2 ? 0.f : w2c);
+    } else if (sub) {  // the terms of the split below that remain, in its order
+        const T w1 = l1 * a1 - b1, w2c = ut * a2 * ct, w3 = l3 * a3 - b3;
+        n0 = w1;
+        n1 = w1 * l1;
+        n2 = w1 * vt;
+        p0 = w3;
+        p1 = w3 * l3;
+        p2 = w3 * vt;
+        if (ut > T(0)) p2 = w2c + p2;
+        else if (ut <= T(0)) n2 = n2 + w2c;
     } else {
     {
         const T w = l1 * a1 - b1;
@@ -353,11 +363,32 @@ struct SedTable {
     int n;
     T one_minus_por;  // 1 - mean(porosity)
     T n_p_mix;        // (mean(d50*frac))^(1/6) / 21.1   (compute_n)
+    T k_move;         // max over the classes of (n_p^2 / ((s-1) d50) / (0.9999 theta_c))^3 (mpm_may_move)
     // float path only: folded constants
     T k_theta[PXB_MAX_SED];  // n_p^2 / ((s-1) d50)
     T k_g1[PXB_MAX_SED];     // frac * n_p^3 sqrt(g) / (s-1) * 8
     T inv_one_minus_por;
 };
+
+// Whether a cell may lie above the Shields threshold of any class (false: its grass factor
+// is 0).  theta = k |u|^2 h^(-1/3) > theta_c is tested as |u|^6 (k / theta_c)^3 > h, with
+// theta_c lowered by 1e-4 (k_move; the rounding of the test is below 1e-5), so that no cell
+// the full evaluation would give a grass factor is missed.  A NaN velocity may move.
+template <class T>
+__device__ __forceinline__ bool mpm_may_move(T h, T hu, T hv, const SedTable<T>& S) {
+    T um;
+    if constexpr (is_f32<T>()) {
+        const float rs = f_rsqrt(h);
+        const float r = rs * rs;
+        const float u = hu * r, v = hv * r;
+        um = fsum2(u, u, v, v);
+    } else {
+        const T r = T(1) / h;
+        const T u = hu * r, v = hv * r;
+        um = u * u + v * v;
+    }
+    return h > T(DRY_TOL) && !(um * um * um * S.k_move <= h);
+}
 
 // Meyer-Peter & Mueller grass factor of one cell (roe_exner.py:85-130).
 template <class T>
@@ -365,21 +396,11 @@ __device__ __forceinline__ T mpm_grass(T h, T hu, T hv, bool nodata, const SedTa
     if constexpr (is_f32<T>()) {
         // G = sum_k frac n_p^3 sqrt(g)/((s-1) sqrt h) * 8 sqrt(dth)/(th^1.5 + 1e-5) * dth
         const float hc = clamp_lo(h, float(DRY_TOL));
+        // Below the Shields threshold in every lane and class G is 0 (and 0 for a NaN depth
+        // or velocity): such warps return before the refinement
+        if (!__any_sync(FULL, mpm_may_move(h, hu, hv, S))) return 0.f;
         float rs = f_rsqrt(hc);
         float rcb = f_ex2(-0.33333333333f * f_lg2(hc));  // h^(-1/3)
-        {
-            // Below the Shields threshold in every lane and class G is 0.  The unrefined
-            // theta (relative error under 1e-5) decides it with a 1e-4 margin, so such warps
-            // return before the refinement; the full evaluation gives the same 0 there (and
-            // 0 for a NaN depth or velocity too).
-            const float r0 = rs * rs;
-            const float u0 = hu * r0, v0 = hv * r0;
-            const float q0 = fsum2(u0, u0, v0, v0) * rcb;
-            bool above = false;
-#pragma unroll 1
-            for (int k = 0; k < S.n; ++k) above = above || (S.k_theta[k] * q0 > 0.9999f * S.s[k].thc);
-            if (!__any_sync(FULL, above)) return 0.f;
-        }
         // one Newton step each: the threshold (theta - theta_c)^1.5 amplifies errors in theta
         rs = rs * (1.5f - 0.5f * hc * rs * rs);
         const float r = rs * rs;

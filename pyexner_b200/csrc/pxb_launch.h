@@ -26,9 +26,13 @@ cudaError_t launch_label_fill(int ny, int nx, int npoly, const uint8_t* labels, 
                               long long* cells, cudaStream_t s);
 
 template <class T>
-cudaError_t launch_re_stage(const REStageArgs<T>& a, bool mpm, bool has_mask, bool avg, int grid, cudaStream_t s);
+cudaError_t launch_re_stage(const REStageArgs<T>& a, bool mpm, bool has_mask, bool avg, int grid, int threads,
+                            size_t smem, cudaStream_t s);
+// Allows both stages' kernels of one (mpm, mask) kind, of a plan, of its budget runs or of
+// an ensemble, as much dynamic shared memory as a tile may ask for.
+enum StageUse { STAGE_PLAN = 0, STAGE_BUDGET = 1, STAGE_ENSEMBLE = 2 };
 template <class T>
-int re_stage_blocks_per_sm(bool mpm, bool has_mask, bool avg);
+cudaError_t stage_allow_smem(bool mpm, bool has_mask, StageUse use, size_t bytes);
 template <class T>
 cudaError_t launch_re_cfl(const CflArgs<T>& a, bool has_mask, int grid, cudaStream_t s);
 template <class T>
@@ -70,9 +74,8 @@ cudaError_t launch_dual_pack(int ny, int nx, long long pitch, const double* v, c
                              cudaStream_t s);
 cudaError_t launch_dual_unpack(int ny, int nx, long long pitch, const Dual* in, double* v, double* t, cudaStream_t s);
 template <class T>
-cudaError_t launch_ens_stage(const EnsStageArgs<T>& a, bool mpm, bool has_mask, bool avg, int grid, cudaStream_t s);
-template <class T>
-int ens_stage_blocks_per_sm(bool mpm, bool has_mask, bool avg);
+cudaError_t launch_ens_stage(const EnsStageArgs<T>& a, bool mpm, bool has_mask, bool avg, int grid, int threads,
+                             size_t smem, cudaStream_t s);
 template <class T>
 cudaError_t launch_ens_cfl(const EnsCflArgs<T>& a, bool has_mask, int grid, cudaStream_t s);
 template <class T>

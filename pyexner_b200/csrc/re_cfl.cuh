@@ -26,7 +26,6 @@ struct CflScratch {
     int pad;
     double t_step;               // simulation time at the start of the current step
     double t_next;               // t_step + dt: the time the next dt is added to
-    unsigned int queue[2];       // stage kernel work queue: items handed out, blocks finished
     unsigned int cfl_queue;      // CFL kernel work queue: items handed out (reset by the last block)
     unsigned int pad2;
 };

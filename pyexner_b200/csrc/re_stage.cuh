@@ -5,58 +5,86 @@
 // boundary handlers -> grass factor (:85-140) -> Exner update (:665-717) -> boundary
 // handlers, and for the second SSPRK2 stage the 0.5/0.5 combination (SSPRK2.py:40).
 //
-// Layout of the work: a warp owns a strip of 32 x CPT columns (3 halo | owned | 3 halo;
-// CPT consecutive columns per lane, one by default, two as a float32 build knob) and
-// marches down a band of rows.  Each iteration consumes one new row, copied into the
-// warp's shared buffer by cp.async during the previous iteration (together with the
-// partner-state values the averaging stage stores in this one), and advances a software
-// pipeline held in registers:
-//   A  row r   : cell precompute, x-face fluxes (east neighbour by shuffle), y-face (r-1|r)
-//   B  row r-1 : hydro update (all four faces known)
-//   C  row r-2 : momentum corrections (needs updated depths of rows r-3..r-1)
-//   D  row r-3 : first boundary application on ring cells (donors in rows r-4..r-2)
-//   E  row r-3 : grass factor, Exner cell, Exner x-faces and y-face (r-4|r-3)
-//   F  row r-4 : z_b update
-//   G  row r-5 : second boundary application on z_b and G, then the z_b / G stores
-// Hydro fields are stored after D (the second application leaves them unchanged for
-// the layouts the host accepts).  Every face is evaluated once per warp; the only
-// redundant work is the 6 halo columns of each strip and 6 halo rows of each band.
-// Warp votes skip work whose result is known for the whole warp: the entropy-fix terms
-// without a transonic face, the momentum corrections where every cell is wet, the Exner
-// block where no cell of the two rows carries sediment (see the phases below).
+// Layout of the work: a block computes one tile, a strip of 30 wx - 4 owned columns by a
+// band of owned rows, in two phases with the updated h, hu, hv of the tile (two halo rows
+// and columns on each side) in shared memory between them:
+//   1  hydro faces and update: its warps stand wx side by side and wy on top of one
+//      another; a warp holds 32 columns, of which the inner 30 get both of their x-faces
+//      from shuffles (side-by-side warps overlap by two columns), and marches down its
+//      share of the rows with the north face's fluctuation in registers
+//   C  momentum corrections, only where some cell of the tile is dry (or masked), and the
+//      first boundary application, only in tiles with ring cells, in shared memory
+//   2  grass factor, Exner cells, faces and z_b update, the same march, then the stores;
+//      ring cells are finished last, from their donors' values in shared memory (second
+//      boundary application)
+// A face between two warps' row shares is evaluated by both; every other face of a tile
+// is evaluated once.  Warp votes skip work whose result is known for the whole warp: the
+// entropy fix and the wave split where every face is subcritical, the activity masks where
+// every cell is wet, the grass factor and the Exner update where no cell near the warp's
+// carries sediment.
+//
+// Bound by instruction issue (82 % of issue slots in the plain float32 stage at 4096^2,
+// DRAM at 35 %).  The tile replaced a warp that marched down a band with all phases in one
+// register pipeline: that needed 118 registers (16 warps per SM, 74 % of issue slots),
+// moved 35 values a row between pipeline stages, repeated 1.41 times the cells (32 columns
+// for 26) and ran 11 rows before its first store, which set the time of small grids.
+// Measured, before -> after, us per SSPRK2 step with the CFL reduction (float32):
+// 48^2 51.5 -> 23, 256^2 53.6 -> 26.7, 512^2 60.7 -> 35, 1024^2 105 -> 66, 2048^2 252 ->
+// 203, 8192^2 3200 -> 2550; with bedload in every cell 2048^2 328 -> 309.
 #pragma once
-#include <type_traits>
-
 #include "pxb_device.cuh"
 
-// Resident 128-thread blocks per SM the float32 build is register-limited to, for the
-// plain stage and the averaging second SSPRK2 stage (tuning knobs, measured on the
-// 2048^2 and 8192^2 Gaussian-bed cases): 4 (128 registers, no spills) with one column
-// per lane; 5 (96 registers) is 1% faster at 8192^2 and 4% slower at 2048^2, where fewer
-// resident warps mean taller bands and fewer redundant halo rows.  With two columns per
-// lane the state needs about 200 registers: 3 blocks (168, some spills) or 2.
-#ifndef PXB_STAGE_MIN_BLOCKS
-#define PXB_STAGE_MIN_BLOCKS (PXB_STAGE_CPT_F32 == 2 ? 3 : 4)
+// Threads of the largest block and resident blocks of that size per SM the stage kernels
+// are register-limited to.  float32: 2 x 384 threads (80 registers, a few spilled bytes);
+// 2 x 512 (64 registers, 56 B of spills) is 5 % slower at 2048^2 and 10 % at 8192^2.
+// float64: 2 x 256 (128 registers); 3 x 256 is 5 % slower with bedload everywhere and 25 %
+// without, 2 x 384 like it, 4 x 256 (64 registers, 1.2 KB of spills) 30 to 50 % slower.
+#ifndef PXB_STAGE_THREADS_F32
+#define PXB_STAGE_THREADS_F32 384
 #endif
-#ifndef PXB_STAGE_MIN_BLOCKS_AVG
-#define PXB_STAGE_MIN_BLOCKS_AVG (PXB_STAGE_CPT_F32 == 2 ? 3 : 4)
+#ifndef PXB_STAGE_BLOCKS_F32
+#define PXB_STAGE_BLOCKS_F32 2
 #endif
-// float64 state (twice the registers per value): 3 blocks (168 registers, a few hundred
-// bytes of spills) measured 12 % faster than 5 (96 registers, 2.8 KB of spills) and than
-// 2 (no spills, too few warps) at 2048^2
-#ifndef PXB_STAGE_MIN_BLOCKS_F64
-#define PXB_STAGE_MIN_BLOCKS_F64 3
+#ifndef PXB_STAGE_THREADS_F64
+#define PXB_STAGE_THREADS_F64 256
 #endif
-// Unroll factor of the steady row loop (tuning knob).
-#ifndef PXB_STAGE_UNROLL
-#define PXB_STAGE_UNROLL 1
+#ifndef PXB_STAGE_BLOCKS_F64
+#define PXB_STAGE_BLOCKS_F64 2
 #endif
-#define PXB_PRAGMA(x) _Pragma(#x)
-#define PXB_UNROLL(n) PXB_PRAGMA(unroll n)
-#define PXB_STAGE_BOUNDS(T, AVG) \
-    (sizeof(T) == 8 ? PXB_STAGE_MIN_BLOCKS_F64 : ((AVG) ? PXB_STAGE_MIN_BLOCKS_AVG : PXB_STAGE_MIN_BLOCKS))
+// Rows of the averaging stage whose partner values are loaded together, one batch ahead of
+// the batch being stored (and the first before the block's barrier): 3 against 2 and 4 is
+// 1 to 3 % faster at 8192^2; without the batch ahead the averaging stage took 1410 us there
+// instead of 1210.
+#ifndef PXB_STAGE_BATCH
+#define PXB_STAGE_BATCH 3
+#endif
 
 namespace pxb {
+
+constexpr int stage_max_threads(int esize) { return esize == 8 ? PXB_STAGE_THREADS_F64 : PXB_STAGE_THREADS_F32; }
+constexpr int stage_min_blocks(int esize) { return esize == 8 ? PXB_STAGE_BLOCKS_F64 : PXB_STAGE_BLOCKS_F32; }
+
+// Columns of a tile with wx warps side by side: all (raw), and owned by an inner strip.
+static inline constexpr __host__ __device__ int stage_cols(int wx) { return 30 * wx + 2; }
+static inline constexpr __host__ __device__ int stage_owned(int wx) { return 30 * wx - 4; }
+// Strips of a grid: the first owns three columns more (no halo to its west), the last up
+// to three more; every strip but the first starts where its left neighbour's ends.
+static inline __host__ __device__ int stage_strips(int nx, int wx) {
+    const int oc = stage_owned(wx);
+    return nx > 6 + oc ? (nx - 6 + oc - 1) / oc : 1;
+}
+// First row of band b: bands differ by at most one row (and have at least two: the host
+// asks for at most ny / 2 bands).
+static inline __host__ __device__ int stage_band_row(int ny, int nbands, int b) {
+    return (int)(((long long)ny * b) / nbands);
+}
+// Shared memory of a block, in elements: h, hu, hv of srows x cols cells, and for ring
+// cells five values per slot (first application: h, hu, hv, then z_b and G) and z_b, G of
+// the four outermost rows and columns.
+static inline __host__ __device__ size_t stage_smem_elems(int wx, int srows) {
+    const size_t pw = stage_cols(wx);
+    return 3 * pw * srows + 12 * (pw + srows);
+}
 
 template <class T>
 struct REStageArgs {
@@ -70,13 +98,12 @@ struct REStageArgs {
     const T* dt;
     const pxb_ring_recipe* ring;              // null when there are no handlers
     SedTable<T> sed;
-    int band_rows, nstrips, nbands;
+    int wx, srows, nstrips, nbands;  // tiles: warps side by side, shared rows, strips, bands
     int* err;
-    unsigned int* queue;  // {next dynamic item, finished blocks}, zero between launches
-    // Volume budget (null: off): per work item, the outflow through the outer boundary of
-    // the physical cells (rows and columns 1 .. n-2) of water (sum of the mass fluxes of
-    // the boundary faces) and of sediment (Exner fluxes), in the state's flux units; item
-    // k writes bud[2k], bud[2k+1] on every launch.
+    // Volume budget (null: off): per tile, the outflow through the outer boundary of the
+    // physical cells (rows and columns 1 .. n-2) of water (sum of the mass fluxes of the
+    // boundary faces) and of sediment (Exner fluxes), in the state's flux units; tile k
+    // writes bud[2k], bud[2k+1] on every launch.
     double* bud;
 };
 
@@ -87,31 +114,14 @@ __device__ __forceinline__ void cp_async_elem(T* smem, const T* gmem) {
     if constexpr (sizeof(T) == 4) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
     else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
 }
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 // cp.async of 16 bytes with zero fill: the first src_bytes (0-16) bytes are read, the
 // rest of the 16 is set to zero; with src_bytes = 0 nothing is read.
 __device__ __forceinline__ void cp_async16_zfill(unsigned smem, const void* gmem, unsigned src_bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem), "l"(gmem), "r"(src_bytes) : "memory");
 }
-static_assert(sizeof(pxb_ring_recipe) == 48, "ring recipes are copied as three 16-byte chunks");
-
-// Fields of the second boundary application (z_b and G donors) packed into one word by
-// the first: flags bits 3-4 and the four offsets (each in [-1, 1]) biased by 8.
-__device__ __forceinline__ unsigned pack_zg(unsigned flags, int zdy, int zdx, int gdy, int gdx) {
-    return (flags & 24u) | ((unsigned)(zdy + 8) << 8) | ((unsigned)(zdx + 8) << 12) | ((unsigned)(gdy + 8) << 16) |
-           ((unsigned)(gdx + 8) << 20);
-}
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-
-template <class T>
-__device__ __forceinline__ T pick_row(int dy, T above, T mid, T below) {
-    return dy < 0 ? above : (dy > 0 ? below : mid);
-}
 
 template <class T>
 __device__ __forceinline__ HCell<T> shfl_down_hcell(const HCell<T>& p) {
@@ -140,852 +150,556 @@ __device__ __forceinline__ ECell<T> shfl_down_ecell(const ECell<T>& p) {
     return q;
 }
 
-// Donor values of the boundary passes for the CPT columns of this lane: column k takes
-// the value at (row q+dy[k], column +dxo[k]) with dy, dxo in [-1, 1].  The candidates
-// are this lane's own columns and the last column of the west lane / first column of
-// the east lane (one shuffle each); the row is chosen by the receiver.  Donors lie in
-// another row only for cells of the first and last rows (plan creation checks it), so
-// elsewhere (dyrow false) only the middle row is fetched.
-template <int CPT, class T>
-__device__ __forceinline__ T pick_col(const T (&cand)[CPT + 2], int s) {
-    T v = cand[0];
-#pragma unroll
-    for (int t = 1; t < CPT + 2; ++t) v = (s == t) ? cand[t] : v;
-    return v;
-}
+// One row of this lane's column as read from HBM.
+template <class T>
+struct RawCell {
+    T h, hu, hv, zb, z, nb;
+    bool m;
+};
 
-template <int CPT, class T>
-__device__ __forceinline__ void donor_candidates(const T (&x)[CPT], T (&cd)[CPT + 2]) {
-    cd[0] = __shfl_up_sync(FULL, x[CPT - 1], 1);
-#pragma unroll
-    for (int k = 0; k < CPT; ++k) cd[k + 1] = x[k];
-    cd[CPT + 1] = __shfl_down_sync(FULL, x[0], 1);
-}
+// The SSPRK2 partner's values of one cell.
+template <class T>
+struct Partner {
+    T h, hu, hv, zb, G;
+};
 
-template <int CPT, class T>
-__device__ __forceinline__ void fetch_donor(bool dyrow, const int (&dy)[CPT], const int (&dxo)[CPT],
-                                            const T (&above)[CPT], const T (&mid)[CPT], const T (&below)[CPT],
-                                            T (&out)[CPT]) {
-    T cm[CPT + 2];
-    donor_candidates<CPT>(mid, cm);
-    if (!dyrow) {
-#pragma unroll
-        for (int k = 0; k < CPT; ++k) out[k] = pick_col<CPT>(cm, k + dxo[k] + 1);
-        return;
-    }
-    T ca[CPT + 2], cbl[CPT + 2];
-    donor_candidates<CPT>(above, ca);
-    donor_candidates<CPT>(below, cbl);
-#pragma unroll
-    for (int k = 0; k < CPT; ++k) {
-        const int s = k + dxo[k] + 1;
-        out[k] = pick_row(dy[k], pick_col<CPT>(ca, s), pick_col<CPT>(cm, s), pick_col<CPT>(cbl, s));
-    }
-}
-
-// CPT consecutive elements of a shared row buffer laid out by column (lane * CPT + k).
-template <int CPT, class T>
-__device__ __forceinline__ void read_cols(const T* rowp, int lane, T (&v)[CPT]) {
-    if constexpr (CPT == 2 && sizeof(T) == 4) {
-        const float2 t = *reinterpret_cast<const float2*>(rowp + 2 * lane);
-        v[0] = t.x;
-        v[1] = t.y;
-    } else {
-#pragma unroll
-        for (int k = 0; k < CPT; ++k) v[k] = rowp[CPT * lane + k];
-    }
-}
-
-// One work item (a strip of one band) of a stage; the single-grid kernel and the
-// ensemble kernel (ens.cuh) both loop over items and call this.  Each lane owns CPT
-// consecutive columns (pxb_stage_cpt): a strip is 32 * CPT columns, 3 halo | owned | 3
-// halo.  Neighbour values inside a lane are plain registers; across lanes one shuffle
-// moves the first (east) or last (west) column.
-// A block's shared buffer of the stage kernel (TAG: 0 row copies, 1 partner copies),
-// one object for every instantiation of re_stage_item with these dimensions, so that
-// the interior and the boundary instantiations in one kernel share it.
-template <class T, int TAG, int D0, int D1, int D2, int D3>
-__device__ __forceinline__ T (&stage_smem())[D0][D1][D2][D3] {
-    __shared__ __align__(16) T buf[D0][D1][D2][D3];
-    return buf;
-}
-
-// INTERIOR: the instantiation for items away from the grid's boundary (no boundary strip
-// or row), which carries none of the boundary-recipe code.
-template <class T, bool MPM, bool HAS_MASK, bool AVG, bool BUD = false, bool INTERIOR = false>
-__device__ __forceinline__ void re_stage_item(const REStageArgs<T>& a, const int item, bool& bad) {
-    constexpr int CPT = pxb_stage_cpt((int)sizeof(T));
-    constexpr int W = 32 * CPT;
-    const int lane = threadIdx.x & 31;
+// One tile.  INTERIOR: the instantiation for tiles away from the grid's boundary (inner
+// strips of inner bands): every column lies inside the grid and no cell whose Exner
+// update the tile needs is a ring cell, so it carries neither column tests nor boundary
+// code.  The results do not depend on the tiling.
+template <class T, bool MPM, bool HAS_MASK, bool AVG, bool BUD, bool INTERIOR>
+__device__ __forceinline__ void re_stage_tile(const REStageArgs<T>& a, const int tile, T* const S, bool& bad) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int wx = a.wx, wy = (int)(blockDim.x >> 5) / wx;
+    const int iy = warp / wx, ix = warp - iy * wx;
     const int ny = a.ny, nx = a.nx;
     const unsigned upitch = (unsigned)a.pitch;  // planes are < 2^31 elements (checked at plan creation)
     const T dt = *a.dt;
     const T dx = a.dx;
     const T dtdx = dt / dx;  // float path only
     const T DRY = T(DRY_TOL);
+    const int band = tile / a.nstrips, strip = tile - band * a.nstrips;
+    const bool first_strip = strip == 0, last_strip = strip == a.nstrips - 1;
+    const int pw = stage_cols(wx), sr = a.srows;
+    const int cstart = strip * stage_owned(wx);  // column of index 0
+    const int idx = 30 * ix + lane, c = cstart + idx;
+    const bool colok = INTERIOR || c < nx;
+    const bool has_e = lane < 31 && (INTERIOR || c + 1 < nx);
+    // owned columns by index, and the lane of the column's one owner
+    const int lo = first_strip ? 0 : 3, hi = last_strip ? nx - 1 - cstart : pw - 4;
+    const bool lane_in = (lane >= 1 && lane <= 30) || (idx == 0) || (idx == pw - 1);
+    const bool out_col = lane_in && idx >= lo && idx <= hi;
+    const bool near_col = lane_in && idx >= lo - 1 && idx <= hi + 1 && colok;  // owned or next to one
+    const int R0 = stage_band_row(ny, a.nbands, band), R1 = stage_band_row(ny, a.nbands, band + 1);
+    const int H0 = max(0, R0 - 2), H1 = min(ny, R1 + 2);  // rows of the hydro update
+    const int K0 = max(0, R0 - 1), K1 = min(ny, R1 + 1);  // rows of the Exner cells
+    T* const Sh = S;
+    T* const Su = S + (size_t)pw * sr;
+    T* const Sv = S + 2 * (size_t)pw * sr;
+    auto sidx = [&](int r, int k) __attribute__((always_inline)) { return (r - (R0 - 2)) * pw + k; };
+    // Budget: a face counts once, in the tile that owns its row (x-faces; y-faces (r-1|r)
+    // by row r) and the lane that owns the column.  The outflow of a face with left cell I
+    // (west / north side) is F = h_I u_n,I + upwM_0, the flux whose differences the
+    // fluctuations of roe_exner.py:597-606 telescope to; F leaves the physical cells
+    // through the east / south boundary and enters them through the west / north one.
+    // Exner: the upwind face flux of roe_exner.py:708-715.
+    double budh = 0.0, budz = 0.0;
+
+    // ================= phase 1: hydro faces and update of rows H0 .. H1-1
+    // the outermost index columns miss a face unless the grid ends there: they stay zero,
+    // as do the columns beyond the grid
+    const bool whole = INTERIOR ? (lane >= 1 && lane <= 30) : colok && ((lane >= 1 && lane <= 30) || c == 0 || c == nx - 1);
+    bool dry = false;
     {
-        const int ipb = pxb_stage_items_per_band(a.nstrips);
-        const int band = item / ipb;
-        const int kb = item - band * ipb;
-        int strip = kb - 1, half = -1;  // half: 0 / 1 = upper / lower half of a boundary strip
-        if (ipb == 1) strip = 0;
-        else if (kb < 2) { strip = 0; half = kb; }
-        else if (kb >= a.nstrips) { strip = a.nstrips - 1; half = kb - a.nstrips; }
-        const bool last_strip = !INTERIOR && strip == a.nstrips - 1;
-        const int cb = strip * (W - 2 * PXB_HALO) - PXB_HALO + CPT * lane;  // column of this lane's first element
-        bool colok[CPT], has_e[CPT], out_col[CPT], interior_col[CPT];
-#pragma unroll
-        for (int k = 0; k < CPT; ++k) {
-            const int c = cb + k, j = CPT * lane + k;
-            // an interior strip lies inside the grid's columns 1 .. nx-2 (it is neither the
-            // first nor the last strip, and every strip but the last ends two columns
-            // short of column nx - 1)
-            colok[k] = INTERIOR || ((c >= 0) && (c < nx));
-            has_e[k] = colok[k] && (INTERIOR || c + 1 < nx) && (j < W - 1);
-            out_col[k] = colok[k] && j >= PXB_HALO && (j < W - PXB_HALO || last_strip);
-            interior_col[k] = INTERIOR || ((c >= 1) && (c <= nx - 2));
-        }
-        const int B0 = band * a.band_rows;
-        const int B1 = (band == a.nbands - 1) ? ny : B0 + a.band_rows;
-        const int Bm = B0 + (B1 - B0 + 1) / 2;
-        const int R0 = half == 1 ? Bm : B0;
-        const int R1 = half == 0 ? Bm : B1;
-        const int L0 = max(0, R0 - 3), L1 = min(ny, R1 + 3);
-        // boundary recipes can only apply in the first/last strip or on rows 0 / ny-1
-        const bool bc_strip = !INTERIOR && (a.ring != nullptr) && (strip == 0 || last_strip);
-        const bool bc_rows = !INTERIOR && (a.ring != nullptr) && (R0 == 0 || R1 == ny);
-        // Budget: only items that own boundary faces of physical cells add to the lane slots.
-        // A face counts once: in the item that owns its row (x-faces; y-faces (r-1|r) by row
-        // r) and, for columns, by the lane that owns the column.  The outflow of a face with
-        // left cell I (west / north side) is F = h_I u_n,I + upwM_0, the flux whose
-        // differences the fluctuations of roe_exner.py:597-606 telescope to; F leaves the
-        // physical cells through the east / south boundary and enters them through the west
-        // / north one.  Exner: the upwind face flux of roe_exner.py:708-715.
-        // (BUD: the budget instantiation, launched only when a.bud is set)
-        __shared__ double budbuf[4][BUD ? 2 : 1][BUD ? 32 : 1];
-        const bool bud_item = BUD && (bc_strip || bc_rows);
-        if constexpr (BUD) {
-            budbuf[threadIdx.x >> 5][0][lane] = 0.0;
-            budbuf[threadIdx.x >> 5][1][lane] = 0.0;
-        }
-
-        // ---- carried pipeline state, per column
-        HCell<T> pA[CPT];
-        T hA[CPT], huA[CPT], hvA[CPT], ztA[CPT];
-        T xfA[CPT][3], nfA[CPT][3];
-        T hr3[CPT], hr2[CPT], hur2[CPT], hvr2[CPT], zt3[CPT], zt2[CPT];
-        unsigned mwin[CPT];  // bit i = nodata of row r-1-i
-        T zin1[CPT], zin2[CPT], zin3[CPT], zin4[CPT];
-        T gin1[CPT], gin2[CPT], gin3[CPT], gin4[CPT];
-        T hf4h[CPT], hf4u[CPT], hf4v[CPT], hf3h[CPT], hf3u[CPT], hf3v[CPT];
-        ECell<T> e4[CPT];
-        T xe4[CPT], fn4[CPT];
-        T zbp6[CPT], zbp5[CPT], gg6[CPT], gg5[CPT];
-#pragma unroll
-        for (int k = 0; k < CPT; ++k) {
-            pA[k] = make_hcell(T(0), T(0), T(0), T(0), T(0), T(0));
-            hA[k] = huA[k] = hvA[k] = ztA[k] = T(0);
-#pragma unroll
-            for (int m = 0; m < 3; ++m) xfA[k][m] = nfA[k][m] = T(0);
-            hr3[k] = hr2[k] = hur2[k] = hvr2[k] = zt3[k] = zt2[k] = T(0);
-            mwin[k] = 0u;
-            zin1[k] = zin2[k] = zin3[k] = zin4[k] = T(0);
-            gin1[k] = gin2[k] = gin3[k] = gin4[k] = T(0);
-            hf4h[k] = hf4u[k] = hf4v[k] = hf3h[k] = hf3u[k] = hf3v[k] = T(0);
-            e4[k] = make_ecell(T(0), T(0), T(0), T(0), T(0));
-            xe4[k] = fn4[k] = T(0);
-            zbp6[k] = zbp5[k] = gg6[k] = gg5[k] = T(0);
-        }
-
-        // Row r+1 is fetched while row r is computed: the loads of one iteration are in
-        // flight during the ~thousand instructions of the previous one.  In float32 they
-        // are cp.async copies into this warp's shared buffer (no registers held); in
-        // float64 (measured: faster there) plain loads into registers.
-        constexpr bool ASYNC_ROWS = is_f32<T>();
-        constexpr int NP = MPM ? 6 : 7;
-        auto& rbuf = stage_smem<T, 0, 4, ASYNC_ROWS ? 2 : 1, ASYNC_ROWS ? NP : 1, ASYNC_ROWS ? W : 1>();
-        T(*rb)[ASYNC_ROWS ? NP : 1][ASYNC_ROWS ? W : 1] = rbuf[threadIdx.x >> 5];
-        T nh[CPT], nhu[CPT], nhv[CPT], nzb[CPT], nz[CPT], nnb[CPT], ng[CPT];
-        bool nm[CPT];
-#pragma unroll
-        for (int k = 0; k < CPT; ++k) {
-            nh[k] = nhu[k] = nhv[k] = nzb[k] = nz[k] = nnb[k] = ng[k] = T(0);
-            nm[k] = false;
-        }
-        auto load_row = [&](int rr) __attribute__((always_inline)) {
-            const int b = rr & 1;
-#pragma unroll
-            for (int k = 0; k < CPT; ++k) {
-                const bool ok = rr < L1 && colok[k];
-                const unsigned i = (unsigned)rr * upitch + (unsigned)(cb + k);
-                if constexpr (!ASYNC_ROWS) {
-                    if (ok) {
-                        nh[k] = __ldg(a.h + i);
-                        nhu[k] = __ldg(a.hu + i);
-                        nhv[k] = __ldg(a.hv + i);
-                        nzb[k] = __ldg(a.zb + i);
-                        nz[k] = __ldg(a.z + i);
-                        nnb[k] = __ldg(a.nb + i);
-                        if (!MPM) ng[k] = __ldg(a.G + i);
-                        if (HAS_MASK) nm[k] = __ldg(a.nodata + i) != 0;
-                    } else {
-                        nh[k] = nhu[k] = nhv[k] = nzb[k] = nz[k] = nnb[k] = ng[k] = T(0);
-                        nm[k] = false;
-                    }
-                } else {
-                    const int e = CPT * lane + k;
-                    if (ok) {
-                        cp_async_elem(&rb[b][0][e], a.h + i);
-                        cp_async_elem(&rb[b][1][e], a.hu + i);
-                        cp_async_elem(&rb[b][2][e], a.hv + i);
-                        cp_async_elem(&rb[b][3][e], a.zb + i);
-                        cp_async_elem(&rb[b][4][e], a.z + i);
-                        cp_async_elem(&rb[b][5][e], a.nb + i);
-                        if constexpr (!MPM) cp_async_elem(&rb[b][NP - 1][e], a.G + i);
-                        if (HAS_MASK) nm[k] = __ldg(a.nodata + i) != 0;
-                    } else {
-#pragma unroll
-                        for (int pl = 0; pl < NP; ++pl) rb[b][pl][e] = T(0);
-                        nm[k] = false;
-                    }
-                }
-            }
-        };
-        load_row(L0);
-        // Averaging stage: the partner state's values of the cells stored in iteration r
-        // (rows r-3 and r-5).  In float32 they are copied asynchronously into this warp's
-        // shared buffer during iteration r-1, so they cost neither registers nor a wait at
-        // the store; in float64 (measured: the shared-buffer form is slower there) they
-        // are loaded into registers at the start of iteration r.  Only the owning lane
-        // reads and then writes these cells, so both are safe when the output aliases the
-        // partner.
-        constexpr bool ASYNC_PARTNER = AVG && is_f32<T>();
-        auto& pbuf = stage_smem<T, 1, 4, ASYNC_PARTNER ? 2 : 1, 5, ASYNC_PARTNER ? W : 1>();
-        T(*pb)[5][ASYNC_PARTNER ? W : 1] = pbuf[threadIdx.x >> 5];
-        auto partner_copy = [&](const int rr) __attribute__((always_inline)) {  // the rows stored in iteration rr
-            const int q0 = rr - 3, p0 = rr - 5;
-            const int b = rr & 1;
-#pragma unroll
-            for (int k = 0; k < CPT; ++k) {
-                const int e = CPT * lane + k;
-                if (q0 >= L0 && q0 < L1 && q0 >= R0 && q0 < R1 && out_col[k]) {
-                    const unsigned i = (unsigned)q0 * upitch + (unsigned)(cb + k);
-                    cp_async_elem(&pb[b][0][e], a.ah + i);
-                    cp_async_elem(&pb[b][1][e], a.ahu + i);
-                    cp_async_elem(&pb[b][2][e], a.ahv + i);
-                }
-                if (p0 >= L0 && p0 < L1 && p0 >= R0 && p0 < R1 && out_col[k]) {
-                    const unsigned i = (unsigned)p0 * upitch + (unsigned)(cb + k);
-                    cp_async_elem(&pb[b][3][e], a.azb + i);
-                    if (a.oG) cp_async_elem(&pb[b][4][e], a.aG + i);
-                }
-            }
-        };
-        if constexpr (ASYNC_PARTNER) partner_copy(L0);
-        cp_async_commit();
-        // Boundary recipes of the side columns (first / last strip, rows other than the
-        // first and last): the recipe of the ring cell of the row that the first boundary
-        // application treats in iteration r (q = r-3) is copied into this warp's shared
-        // buffer during iteration r-1 (one slot per side), so no recipe load is waited on
-        // inside the pipeline; the first and last rows, where every column is a ring cell,
-        // read theirs directly.  The first application leaves the z_b / G fields of the
-        // second (row p = r-5, two iterations later) in a packed word.  Float32 only, as
-        // the row copies.
-        constexpr bool ASYNC_RECIPES = ASYNC_ROWS && !INTERIOR;
-        __shared__ __align__(16) pxb_ring_recipe rcbuf[4][ASYNC_RECIPES ? 2 : 1][2];
-        __shared__ unsigned zgbuf[4][ASYNC_RECIPES ? 4 : 1][ASYNC_RECIPES ? W : 1];
-        pxb_ring_recipe(*rcb)[2] = rcbuf[threadIdx.x >> 5];
-        unsigned(*zgb)[ASYNC_RECIPES ? W : 1] = zgbuf[threadIdx.x >> 5];
-        auto recipe_copy = [&](const int rr) __attribute__((always_inline)) {  // the recipes used in iteration rr
-            const int qn = rr - 3;
-            if (bc_strip && qn >= L0 && qn < L1 && qn != 0 && qn != ny - 1) {
-#pragma unroll
-                for (int k = 0; k < CPT; ++k) {
-                    const int c = cb + k;
-                    if (c == 0 || c == nx - 1) {
-                        const char* src = reinterpret_cast<const char*>(a.ring + ring_slot(qn, c, ny, nx));
-                        char* dst = reinterpret_cast<char*>(&rcb[rr & 1][c == 0 ? 0 : 1]);
-                        cp_async16(dst, src);
-                        cp_async16(dst + 16, src + 16);
-                        cp_async16(dst + 32, src + 32);
-                    }
-                }
-            }
-        };
-
-        // One pipeline iteration.  In the steady state (rows L0+5 .. L1-1) every phase has
-        // valid rows, so the row checks compile away.
-        auto iterate = [&](const int r, auto steady_tag) __attribute__((always_inline)) {
-            constexpr bool S = decltype(steady_tag)::value;
-            const bool rowA = S || r < L1;
-            // ================= A: row r (prefetched), x-faces of row r, y-face (r-1 | r)
-            T h_r[CPT], hu_r[CPT], hv_r[CPT], zb_r[CPT], z_r[CPT], nb_r[CPT], g_r[CPT];
-            if constexpr (ASYNC_ROWS) {
-                cp_async_wait<0>();  // row r (and the partner rows stored in this iteration)
-                const int rbb = r & 1;
-                read_cols<CPT>(rb[rbb][0], lane, h_r);
-                read_cols<CPT>(rb[rbb][1], lane, hu_r);
-                read_cols<CPT>(rb[rbb][2], lane, hv_r);
-                read_cols<CPT>(rb[rbb][3], lane, zb_r);
-                read_cols<CPT>(rb[rbb][4], lane, z_r);
-                read_cols<CPT>(rb[rbb][5], lane, nb_r);
-                if constexpr (!MPM) {
-                    read_cols<CPT>(rb[rbb][NP - 1], lane, g_r);
-                } else {
-#pragma unroll
-                    for (int k = 0; k < CPT; ++k) g_r[k] = T(0);
-                }
+        if (lane_in && !whole)
+            for (int r = H0 + iy; r < H1; r += wy) Sh[sidx(r, idx)] = Su[sidx(r, idx)] = Sv[sidx(r, idx)] = T(0);
+        const int n = H1 - H0;
+        const int q0 = H0 + n * iy / wy, q1 = H0 + n * (iy + 1) / wy;
+        auto load = [&](int r) __attribute__((always_inline)) {
+            RawCell<T> x;
+            if (colok && r >= 0 && r < ny) {
+                const unsigned i = (unsigned)r * upitch + (unsigned)c;
+                x.h = __ldg(a.h + i);
+                x.hu = __ldg(a.hu + i);
+                x.hv = __ldg(a.hv + i);
+                x.zb = __ldg(a.zb + i);
+                x.z = __ldg(a.z + i);
+                x.nb = __ldg(a.nb + i);
+                x.m = HAS_MASK ? __ldg(a.nodata + i) != 0 : false;
             } else {
-#pragma unroll
-                for (int k = 0; k < CPT; ++k) {
-                    h_r[k] = nh[k], hu_r[k] = nhu[k], hv_r[k] = nhv[k], zb_r[k] = nzb[k];
-                    z_r[k] = nz[k], nb_r[k] = nnb[k], g_r[k] = ng[k];
-                }
+                x.h = x.hu = x.hv = x.zb = x.z = x.nb = T(0);
+                x.m = false;
             }
-            bool m_r[CPT];
+            return x;
+        };
+        if (q0 < q1) {
+            int r = max(q0 - 1, 0);  // the row above the share gives its first north face
+            RawCell<T> cur = load(r), nxt = load(r + 1);
+            HCell<T> p = make_hcell(cur.h, cur.hu, cur.hv, cur.zb, cur.z, cur.nb);
+            T nP[3] = {T(0), T(0), T(0)};
+            for (; r < q1; ++r) {
+                const HCell<T> ps = make_hcell(nxt.h, nxt.hu, nxt.hv, nxt.zb, nxt.z, nxt.nb);
+                const T h_r = cur.h, hu_r = cur.hu, hv_r = cur.hv;
+                const bool m_r = cur.m;
+                cur = nxt;
+                if (r + 2 <= q1) nxt = load(r + 2);  // in flight during this row's faces
+                // pr.h = max(h, DRY_TOL) > DRY_TOL exactly when h > DRY_TOL (false for NaN).
+                // Where every cell of row r is wet (and, with a mask plane, no cell of rows r
+                // and r+1 is nodata), all of its x-faces and south faces are active and need no
+                // masks (inner tiles; the two outer lanes' missing faces enter no cell that is
+                // kept).
+                const bool wet = p.h > DRY;
+                const bool allwet = INTERIOR && __all_sync(FULL, wet && !(HAS_MASK && (m_r || cur.m)));
+                T yP[3] = {T(0), T(0), T(0)}, yM[3] = {T(0), T(0), T(0)};
+                if (r + 1 < ny) {
+                    roe_exner_face<T, true, true>(p, ps, dx, yP, yM);
+                    if (!allwet) {
+                        const bool act = colok && (wet || ps.h > DRY) && !(HAS_MASK && (m_r || cur.m));
 #pragma unroll
-            for (int k = 0; k < CPT; ++k) m_r[k] = nm[k];
-            load_row(r + 1);
-            if constexpr (ASYNC_PARTNER) partner_copy(r + 1);
-            if constexpr (ASYNC_RECIPES) recipe_copy(r + 1);
-            cp_async_commit();
-            T pah[CPT], pahu[CPT], pahv[CPT], pazb[CPT], paG[CPT];
-#pragma unroll
-            for (int k = 0; k < CPT; ++k) pah[k] = pahu[k] = pahv[k] = pazb[k] = paG[k] = T(0);
-            if constexpr (!ASYNC_PARTNER && AVG) {
-                const int q0 = r - 3, p0 = r - 5;
-#pragma unroll
-                for (int k = 0; k < CPT; ++k) {
-                    if ((S || (q0 >= L0 && q0 < L1)) && q0 >= R0 && q0 < R1 && out_col[k]) {
-                        const unsigned i = (unsigned)q0 * upitch + (unsigned)(cb + k);
-                        pah[k] = a.ah[i];
-                        pahu[k] = a.ahu[i];
-                        pahv[k] = a.ahv[i];
-                    }
-                    if ((S || (p0 >= L0 && p0 < L1)) && p0 >= R0 && p0 < R1 && out_col[k]) {
-                        const unsigned i = (unsigned)p0 * upitch + (unsigned)(cb + k);
-                        pazb[k] = a.azb[i];
-                        if (a.oG) paG[k] = a.aG[i];
-                    }
-                }
-            }
-            HCell<T> pr[CPT];
-            T zt_r[CPT];
-#pragma unroll
-            for (int k = 0; k < CPT; ++k) {
-                pr[k] = make_hcell(h_r[k], hu_r[k], hv_r[k], zb_r[k], z_r[k], nb_r[k]);
-                zt_r[k] = z_r[k] + zb_r[k];
-            }
-            T xf[CPT][3];
-#pragma unroll
-            for (int k = 0; k < CPT; ++k) xf[k][0] = xf[k][1] = xf[k][2] = T(0);
-            // In the prologue / drain iterations of a band the faces of invalid rows are
-            // skipped for the whole warp (r is warp-uniform); their results would be masked.
-            if (S || rowA) {
-                HCell<T> pe[CPT];
-                bool me[CPT];
-#pragma unroll
-                for (int k = 0; k + 1 < CPT; ++k) { pe[k] = pr[k + 1]; me[k] = m_r[k + 1]; }
-                pe[CPT - 1] = shfl_down_hcell(pr[0]);
-                me[CPT - 1] = HAS_MASK ? (__shfl_down_sync(FULL, (int)m_r[0], 1) != 0) : false;
-                T P[CPT][3], M[CPT][3];
-                bool xact[CPT];
-#pragma unroll
-                for (int k = 0; k < CPT; ++k) {
-                    // pr.h = max(h, DRY_TOL) > DRY_TOL exactly when h > DRY_TOL (false for NaN)
-                    xact[k] = rowA && has_e[k] && ((pr[k].h > DRY) || (pe[k].h > DRY)) && !(m_r[k] || me[k]);
-                    roe_exner_face<T, false>(pr[k], pe[k], dx, P[k], M[k]);
-#pragma unroll
-                    for (int m = 0; m < 3; ++m) {
-                        P[k][m] = xact[k] ? P[k][m] : T(0);
-                        M[k][m] = xact[k] ? M[k][m] : T(0);
-                    }
-                    if (bud_item && xact[k] && out_col[k] && r >= R0 && r < R1 && r >= 1 && r <= ny - 2 &&
-                        (cb + k == 0 || cb + k == nx - 2)) {
-                        const double F = (double)mul_rn(pr[k].h, pr[k].u) + (double)M[k][0];
-                        if constexpr (BUD) budbuf[threadIdx.x >> 5][0][lane] += cb + k == 0 ? -F : F;
-                    }
-                }
-                // upwP of the west face of column k: own column k-1, or the west lane's last
-                // (lane 0 has no west face in the warp).  P and M are zero on inactive faces,
-                // and the sums start at +0, so adding them unconditionally gives the same bits
-                // as adding only the active ones.
-                T wP[CPT][3];
-#pragma unroll
-                for (int k = 1; k < CPT; ++k)
-#pragma unroll
-                    for (int m = 0; m < 3; ++m) wP[k][m] = P[k - 1][m];
-#pragma unroll
-                for (int m = 0; m < 3; ++m) {
-                    const T w = __shfl_up_sync(FULL, P[CPT - 1][m], 1);
-                    wP[0][m] = lane > 0 ? w : T(0);
-                }
-                // scatter order of roe_exner.py:599-600: east upwM first, then west upwP
-#pragma unroll
-                for (int k = 0; k < CPT; ++k) {
-#pragma unroll
-                    for (int m = 0; m < 3; ++m) xf[k][m] = (xf[k][m] + M[k][m]) + wP[k][m];
-                }
-            }
-            T yP[CPT][3], yM[CPT][3];
-#pragma unroll
-            for (int k = 0; k < CPT; ++k)
-#pragma unroll
-                for (int m = 0; m < 3; ++m) yP[k][m] = yM[k][m] = T(0);
-            if (S || (rowA && r - 1 >= L0)) {
-#pragma unroll
-                for (int k = 0; k < CPT; ++k) {
-                    const bool yact = rowA && (S || r - 1 >= L0) && colok[k] && ((hA[k] > DRY) || (h_r[k] > DRY)) &&
-                                      !((mwin[k] & 1u) || m_r[k]);
-                    roe_exner_face<T, true>(pA[k], pr[k], dx, yP[k], yM[k]);
-#pragma unroll
-                    for (int m = 0; m < 3; ++m) {
-                        yP[k][m] = yact ? yP[k][m] : T(0);
-                        yM[k][m] = yact ? yM[k][m] : T(0);
-                    }
-                    if (bud_item && (r == 1 || r == ny - 1) && r >= R0 && r < R1) {
-                        const int c = cb + k;
-                        if (out_col[k] && yact && c >= 1 && c <= nx - 2) {
-                            // y-faces have the normal (0, -1): u_n = -v
-                            const double F = -(double)mul_rn(pA[k].h, pA[k].v) + (double)yM[k][0];
-                            if constexpr (BUD) budbuf[threadIdx.x >> 5][0][lane] += r == 1 ? -F : F;
+                        for (int m = 0; m < 3; ++m) {
+                            yP[m] = act ? yP[m] : T(0);
+                            yM[m] = act ? yM[m] : T(0);
+                        }
+                        if constexpr (BUD && !INTERIOR) {
+                            const int rs = r + 1;  // the face (r | r+1) counts with row r+1
+                            if (act && out_col && (rs == 1 || rs == ny - 1) && rs >= R0 && rs < R1 && rs >= q0 && rs < q1 &&
+                                c >= 1 && c <= nx - 2) {
+                                // y-faces have the normal (0, -1): u_n = -v
+                                const double F = -(double)mul_rn(p.h, p.v) + (double)yM[0];
+                                budh += rs == 1 ? -F : F;
+                            }
                         }
                     }
                 }
-            }
-
-            // ================= B: hydro update of row r-1
-            T hr1[CPT], hur1[CPT], hvr1[CPT];
+                if (r >= q0) {
+                    const HCell<T> pe = shfl_down_hcell(p);
+                    const bool me = HAS_MASK ? (__shfl_down_sync(FULL, (int)m_r, 1) != 0) : false;
+                    T P[3], M[3];
+                    roe_exner_face<T, false, true>(p, pe, dx, P, M);
+                    if (!allwet) {
+                        const bool act = has_e && (wet || pe.h > DRY) && !(HAS_MASK && (m_r || me));
 #pragma unroll
-            for (int k = 0; k < CPT; ++k) {
-                hr1[k] = hur1[k] = hvr1[k] = T(0);
-                if (S || (r - 1 >= L0 && r - 1 < L1)) {
-                    T f0 = xfA[k][0], f1 = xfA[k][1], f2 = xfA[k][2];
-                    f0 = f0 + yM[k][0]; f1 = f1 + yM[k][1]; f2 = f2 + yM[k][2];    // south face upwM
-                    f0 = f0 + nfA[k][0]; f1 = f1 + nfA[k][1]; f2 = f2 + nfA[k][2];  // north face upwP
+                        for (int m = 0; m < 3; ++m) {
+                            P[m] = act ? P[m] : T(0);
+                            M[m] = act ? M[m] : T(0);
+                        }
+                        if constexpr (BUD && !INTERIOR) {
+                            if (act && out_col && r >= R0 && r < R1 && r >= 1 && r <= ny - 2 && (c == 0 || c == nx - 2)) {
+                                const double F = (double)mul_rn(p.h, p.u) + (double)M[0];
+                                budh += c == 0 ? -F : F;
+                            }
+                        }
+                    }
+                    // scatter order of roe_exner.py:597-602: east upwM, west upwP, south upwM,
+                    // north upwP (lane 0 has no west face in the warp; inactive faces add zeros)
+                    T f[3];
+#pragma unroll
+                    for (int m = 0; m < 3; ++m) {
+                        const T w = __shfl_up_sync(FULL, P[m], 1);
+                        f[m] = (T(0) + M[m]) + ((INTERIOR || lane > 0) ? w : T(0));
+                        f[m] = f[m] + yM[m];
+                        f[m] = f[m] + nP[m];
+                    }
+                    T h1, u1, v1;
                     if constexpr (is_f32<T>()) {
-                        hr1[k] = hA[k] - dtdx * f0;
-                        hur1[k] = huA[k] - dtdx * f1;
-                        hvr1[k] = hvA[k] - dtdx * f2;
+                        h1 = h_r - dtdx * f[0];
+                        u1 = hu_r - dtdx * f[1];
+                        v1 = hv_r - dtdx * f[2];
                     } else {
-                        hr1[k] = hA[k] - dt * f0 / dx;
-                        hur1[k] = huA[k] - dt * f1 / dx;
-                        hvr1[k] = hvA[k] - dt * f2 / dx;
+                        h1 = h_r - dt * f[0] / dx;
+                        u1 = hu_r - dt * f[1] / dx;
+                        v1 = hv_r - dt * f[2] / dx;
+                    }
+                    if (whole) {
+                        const int k = sidx(r, idx);
+                        Sh[k] = h1;
+                        Su[k] = u1;
+                        Sv[k] = v1;
+                        dry = dry || !(h1 > DRY) || (HAS_MASK && m_r);
                     }
                 }
+                nP[0] = yP[0];
+                nP[1] = yP[1];
+                nP[2] = yP[2];
+                p = ps;
             }
+        }
+    }
 
-            // ================= C: momentum corrections of row r-2
-            T hf2h[CPT], hf2u[CPT], hf2v[CPT];
-            // Where every cell of the warp is wet and its north / south neighbours are not
-            // dry (no nodata mask), no correction applies: a warp vote skips the tests and
-            // their shuffles.  Exact: NaN depths fail the vote, as they fail `active`.
-            bool allwet = false;
-            if constexpr (!HAS_MASK) {
-                bool dry = false;
+    // The averaging stage's partner values of this lane's cells of the first rows it will
+    // store, in flight across the barrier and the tests that follow.
+    constexpr int U = PXB_STAGE_BATCH;
+    const int p0 = R0 + (R1 - R0) * iy / wy, p1 = R0 + (R1 - R0) * (iy + 1) / wy;  // rows of phase 2
+    auto partner = [&](int p) __attribute__((always_inline)) {
+        Partner<T> q{};
+        if (AVG && out_col && p < p1) {
+            const unsigned i = (unsigned)p * upitch + (unsigned)c;
+            q.h = a.ah[i];
+            q.hu = a.ahu[i];
+            q.hv = a.ahv[i];
+            q.zb = a.azb[i];
+            if (a.oG) q.G = a.aG[i];
+        }
+        return q;
+    };
+    Partner<T> qn[U];
 #pragma unroll
-                for (int k = 0; k < CPT; ++k)
-                    dry = dry || (colok[k] && (!(hr2[k] > DRY) || (hr3[k] < DRY) || (hr1[k] < DRY)));
-                allwet = !__any_sync(FULL, dry);
+    for (int u = 0; u < U; ++u) qn[u] = partner(p0 + u);
+
+    // ================= momentum corrections (roe_exner.py:14-62) of rows K0 .. K1-1
+    // Where every cell of the tile is wet and none is nodata no correction applies.  A NaN
+    // depth fails `h > DRY`, as it fails `active`.
+    dry = __syncthreads_or(dry) != 0;
+    if (dry) {
+        const int n = K1 - K0;
+        const int q0 = K0 + n * iy / wy, q1 = K0 + n * (iy + 1) / wy;
+        if (near_col && (INTERIOR || (c >= 1 && c <= nx - 2))) {
+            for (int r = max(q0, 1); r < min(q1, ny - 1); ++r) {
+                const unsigned i = (unsigned)r * upitch + (unsigned)c;
+                const int k = sidx(r, idx);
+                const T hc = Sh[k], hE = Sh[k + 1], hW = Sh[k - 1], hN = Sh[k - pw], hS = Sh[k + pw];
+                auto zt = [&](unsigned j) __attribute__((always_inline)) { return __ldg(a.z + j) + __ldg(a.zb + j); };
+                auto nod = [&](unsigned j) __attribute__((always_inline)) { return HAS_MASK && __ldg(a.nodata + j) != 0; };
+                const T eta = hc + zt(i);
+                const bool stop_u = ((hE < DRY) && (eta < zt(i + 1))) || ((hW < DRY) && (eta < zt(i - 1))) || nod(i + 1) || nod(i - 1);
+                const bool stop_v = ((hN < DRY) && (eta < zt(i - upitch))) || ((hS < DRY) && (eta < zt(i + upitch))) ||
+                                    nod(i - upitch) || nod(i + upitch);
+                const bool active = (hc > DRY) && !nod(i);
+                if (!active || stop_u) Su[k] = T(0);
+                if (!active || stop_v) Sv[k] = T(0);
             }
-            if (allwet) {
-#pragma unroll
-                for (int k = 0; k < CPT; ++k) {
-                    const bool ok = S || (r - 2 >= L0 && r - 2 < L1);
-                    hf2h[k] = ok ? hr2[k] : T(0);
-                    hf2u[k] = ok ? hur2[k] : T(0);
-                    hf2v[k] = ok ? hvr2[k] : T(0);
-                }
+        }
+        __syncthreads();
+    }
+
+    // ================= first boundary application, on the ring cells of rows K0 .. K1-1
+    // Ring slots of the tile: row 0 by index, row ny-1 by index, column 0 by row, column
+    // nx-1 by row (the corners belong to the rows).  The recipes map values from before the
+    // application, so the new values are gathered before any is written.
+    const bool ring_tile = !INTERIOR;
+    const int nslots = 2 * (pw + sr);
+    T* const slot_v = S + 3 * (size_t)pw * sr;         // gathered h, hu, hv; then rows / columns of z_b, G
+    T* const slot_zb = slot_v + 8 * (size_t)(pw + sr);  // z_b and G of the ring cells after the application
+    T* const slot_g = slot_zb + nslots;
+    auto slot_cell = [&](int k, int& r, int& j) __attribute__((always_inline)) {  // false: not a ring cell of this tile
+        bool ok;
+        if (k < 2 * pw) {
+            r = k < pw ? 0 : ny - 1;
+            j = k < pw ? k : k - pw;
+            ok = k < pw ? R0 == 0 : R1 == ny;
+        } else {
+            const int s = k - 2 * pw;
+            r = R0 - 2 + (s < sr ? s : s - sr);
+            j = s < sr ? -cstart : nx - 1 - cstart;
+            ok = r >= max(K0, 1) && r < min(K1, ny - 1) && (s < sr ? first_strip : last_strip);
+        }
+        return ok && j >= lo - 1 && j <= hi + 1 && cstart + j < nx;
+    };
+    auto recipe = [&](int r, int j) __attribute__((always_inline)) {
+        pxb_ring_recipe rc{};
+        if (a.ring) rc = a.ring[ring_slot(r, cstart + j, ny, nx)];
+        return rc;
+    };
+    // h, hu, hv of a ring cell by its recipe from the shared values
+    auto apply_hydro = [&](const pxb_ring_recipe& rc, int k0, T& h, T& hu, T& hv) __attribute__((always_inline)) {
+        h = (rc.flags & 1u) ? Sh[k0 + rc.h_dy * pw + rc.h_dx] : Sh[k0];
+        hu = Su[k0];
+        hv = Sv[k0];
+        if (rc.flags & 2u) {
+            if (rc.flags & 4u) {
+                hu = T(rc.m[0]);
+                hv = T(rc.m[1]);
             } else {
-                const int q2 = r - 2;
-                T hE[CPT], hW[CPT], zE[CPT], zW[CPT];
-                bool m2[CPT], mE[CPT], mW[CPT];
-#pragma unroll
-                for (int k = 0; k < CPT; ++k) m2[k] = HAS_MASK && ((mwin[k] >> 1) & 1u);
-#pragma unroll
-                for (int k = 0; k + 1 < CPT; ++k) { hE[k] = hr2[k + 1]; zE[k] = zt2[k + 1]; mE[k] = m2[k + 1]; }
-#pragma unroll
-                for (int k = 1; k < CPT; ++k) { hW[k] = hr2[k - 1]; zW[k] = zt2[k - 1]; mW[k] = m2[k - 1]; }
-                hE[CPT - 1] = __shfl_down_sync(FULL, hr2[0], 1);
-                zE[CPT - 1] = __shfl_down_sync(FULL, zt2[0], 1);
-                hW[0] = __shfl_up_sync(FULL, hr2[CPT - 1], 1);
-                zW[0] = __shfl_up_sync(FULL, zt2[CPT - 1], 1);
-                mE[CPT - 1] = HAS_MASK ? (__shfl_down_sync(FULL, (int)m2[0], 1) != 0) : false;
-                mW[0] = HAS_MASK ? (__shfl_up_sync(FULL, (int)m2[CPT - 1], 1) != 0) : false;
-#pragma unroll
-                for (int k = 0; k < CPT; ++k) {
-                    hf2h[k] = hf2u[k] = hf2v[k] = T(0);
-                    if (S || (q2 >= L0 && q2 < L1)) {
-                        hf2h[k] = hr2[k];
-                        hf2u[k] = hur2[k];
-                        hf2v[k] = hvr2[k];
-                        if (interior_col[k] && q2 >= 1 && q2 <= ny - 2) {
-                            const bool mN = HAS_MASK && ((mwin[k] >> 2) & 1u);
-                            const bool mS = HAS_MASK && (mwin[k] & 1u);
-                            const T eta = hr2[k] + zt2[k];
-                            const bool stop_u = ((eta < zE[k]) && (hE[k] < DRY)) || ((eta < zW[k]) && (hW[k] < DRY)) || mE[k] || mW[k];
-                            const bool stop_v = ((eta < zt3[k]) && (hr3[k] < DRY)) || ((eta < ztA[k]) && (hr1[k] < DRY)) || mN || mS;
-                            const bool active = (hr2[k] > DRY) && !m2[k];
-                            hf2u[k] = (active && !stop_u) ? hur2[k] : T(0);
-                            hf2v[k] = (active && !stop_v) ? hvr2[k] : T(0);
-                        }
-                    }
-                }
+                const int kd = k0 + rc.m_dy * pw + rc.m_dx;
+                const T du = Su[kd], dv = Sv[kd];
+                hu = sum2(T(rc.m[0]), du, T(rc.m[1]), dv);
+                hv = sum2(T(rc.m[2]), du, T(rc.m[3]), dv);
             }
+        }
+    };
+    if (ring_tile) {
+        for (int k = threadIdx.x; k < nslots; k += blockDim.x) {
+            int r, j;
+            if (!slot_cell(k, r, j)) continue;
+            const pxb_ring_recipe rc = recipe(r, j);
+            apply_hydro(rc, sidx(r, j), slot_v[k], slot_v[nslots + k], slot_v[2 * nslots + k]);
+            const unsigned i = (unsigned)r * upitch + (unsigned)(cstart + j);
+            slot_zb[k] = __ldg(a.zb + ((rc.flags & 8u) ? i + (unsigned)((int)rc.zb_dy * (int)upitch + rc.zb_dx) : i));
+            if (!MPM) slot_g[k] = __ldg(a.G + ((rc.flags & 16u) ? i + (unsigned)((int)rc.g_dy * (int)upitch + rc.g_dx) : i));
+        }
+        __syncthreads();
+        for (int k = threadIdx.x; k < nslots; k += blockDim.x) {
+            int r, j;
+            if (!slot_cell(k, r, j)) continue;
+            const int s = sidx(r, j);
+            Sh[s] = slot_v[k];
+            Su[s] = slot_v[nslots + k];
+            Sv[s] = slot_v[2 * nslots + k];
+        }
+        __syncthreads();
+    }
 
-            // ================= D: boundary passes for the hydro fields of row q = r-3
-            // The first pass maps pre-boundary values (HF, input z_b / G) of the donors; the
-            // stored h, hu, hv are the second pass, which maps first-pass values: a donor in
-            // the same row contributes its first-pass value, a donor in another row is never
-            // a hydro boundary cell (checked at plan creation), so its value is HF.
-            const int q = r - 3;
-            const bool rowD = S || ((q >= L0) && (q < L1));
-            T hbh[CPT], hbu[CPT], hbv[CPT], zb1[CPT], gb1[CPT], sbh[CPT], sbu[CPT], sbv[CPT];
-#pragma unroll
-            for (int k = 0; k < CPT; ++k) {
-                hbh[k] = sbh[k] = hf3h[k];
-                hbu[k] = sbu[k] = hf3u[k];
-                hbv[k] = sbv[k] = hf3v[k];
-                zb1[k] = zin3[k];
-                gb1[k] = gin3[k];
-            }
-            if (rowD && (bc_strip || (bc_rows && (q == 0 || q == ny - 1)))) {
-                unsigned flags[CPT];
-                int hdy[CPT], hdx[CPT], mdy[CPT], mdx[CPT], zdy[CPT], zdx[CPT], gdy[CPT], gdx[CPT];
-                T m0[CPT], m1[CPT], m2c[CPT], m3[CPT];
-                bool anyf = false;
-#pragma unroll
-                for (int k = 0; k < CPT; ++k) {
-                    flags[k] = 0u;
-                    hdy[k] = hdx[k] = mdy[k] = mdx[k] = zdy[k] = zdx[k] = gdy[k] = gdx[k] = 0;
-                    m0[k] = m1[k] = m2c[k] = m3[k] = T(0);
-                    auto take = [&](const pxb_ring_recipe& rc) __attribute__((always_inline)) {
-                        flags[k] = rc.flags;
-                        hdy[k] = rc.h_dy; hdx[k] = rc.h_dx; mdy[k] = rc.m_dy; mdx[k] = rc.m_dx;
-                        zdy[k] = rc.zb_dy; zdx[k] = rc.zb_dx; gdy[k] = rc.g_dy; gdx[k] = rc.g_dx;
-                        m0[k] = T(rc.m[0]); m1[k] = T(rc.m[1]); m2c[k] = T(rc.m[2]); m3[k] = T(rc.m[3]);
-                    };
-                    const int c = cb + k;
-                    bool direct = true;
-                    if constexpr (ASYNC_RECIPES) {
-                        if (q != 0 && q != ny - 1) {  // side rows: the ring column's recipe, copied in iteration r-1
-                            direct = false;
-                            if (c == 0 || c == nx - 1) take(rcb[r & 1][c == 0 ? 0 : 1]);
-                        }
-                    }
-                    if (direct) {
-                        const int slot = colok[k] ? ring_slot(q, c, ny, nx) : -1;
-                        if (slot >= 0) take(a.ring[slot]);
-                    }
-                    if constexpr (ASYNC_RECIPES) zgb[r & 3][CPT * lane + k] = pack_zg(flags[k], zdy[k], zdx[k], gdy[k], gdx[k]);
-                    anyf = anyf || (flags[k] != 0u);
-                }
-                if (__any_sync(FULL, anyf)) {
-                    const bool dyrow = (q == 0) || (q == ny - 1);
-                    T vh[CPT], vu[CPT], vv[CPT], vz[CPT];
-                    fetch_donor<CPT>(dyrow, hdy, hdx, hf4h, hf3h, hf2h, vh);
-                    fetch_donor<CPT>(dyrow, mdy, mdx, hf4u, hf3u, hf2u, vu);
-                    fetch_donor<CPT>(dyrow, mdy, mdx, hf4v, hf3v, hf2v, vv);
-                    fetch_donor<CPT>(dyrow, zdy, zdx, zin4, zin3, zin2, vz);
-#pragma unroll
-                    for (int k = 0; k < CPT; ++k) {
-                        if (flags[k] & 1u) hbh[k] = vh[k];
-                        if (flags[k] & 2u) {
-                            if (flags[k] & 4u) { hbu[k] = m0[k]; hbv[k] = m1[k]; }
-                            else { hbu[k] = sum2(m0[k], vu[k], m1[k], vv[k]); hbv[k] = sum2(m2c[k], vu[k], m3[k], vv[k]); }
-                        }
-                        if (flags[k] & 8u) zb1[k] = vz[k];
-                    }
-                    if (!MPM) {
-                        T vg[CPT];
-                        fetch_donor<CPT>(dyrow, gdy, gdx, gin4, gin3, gin2, vg);
-#pragma unroll
-                        for (int k = 0; k < CPT; ++k)
-                            if (flags[k] & 16u) gb1[k] = vg[k];
-                    }
-                    // second pass
-                    T wh[CPT], wu[CPT], wv[CPT];
-                    fetch_donor<CPT>(dyrow, hdy, hdx, hf4h, hbh, hf2h, wh);
-                    fetch_donor<CPT>(dyrow, mdy, mdx, hf4u, hbu, hf2u, wu);
-                    fetch_donor<CPT>(dyrow, mdy, mdx, hf4v, hbv, hf2v, wv);
-#pragma unroll
-                    for (int k = 0; k < CPT; ++k) {
-                        sbh[k] = hbh[k];
-                        sbu[k] = hbu[k];
-                        sbv[k] = hbv[k];
-                        if (flags[k] & 1u) sbh[k] = wh[k];
-                        if ((flags[k] & 2u) && !(flags[k] & 4u)) {
-                            sbu[k] = sum2(m0[k], wu[k], m1[k], wv[k]);
-                            sbv[k] = sum2(m2c[k], wu[k], m3[k], wv[k]);
-                        }
-                    }
-                }
-            }
+    // z_b and G of the four outermost rows (0, 1, ny-2, ny-1) by index and the four
+    // outermost columns by row, for the second application
+    T* const edge_z = slot_v;
+    T* const edge_g = slot_v + 4 * (pw + sr);
 
-            // ================= E: grass factor, Exner cell and faces of row q
-            bool mq[CPT], mq1[CPT];
-#pragma unroll
-            for (int k = 0; k < CPT; ++k) {
-                mq[k] = HAS_MASK && ((mwin[k] >> 2) & 1u);
-                mq1[k] = HAS_MASK && ((mwin[k] >> 3) & 1u);
+    // ================= phase 2: Exner update and stores of rows R0 .. R1-1
+    {
+        // Final values of a cell of row p: stored, unless it is a ring cell (those are
+        // finished last); tiles at the boundary also keep z_b and G of the outermost rows
+        // and columns for that.
+        auto finish = [&](int p, T oh, T ou, T ov, T zo, T go, const Partner<T>& q) __attribute__((always_inline)) {
+            if (!out_col) return;
+            if (!INTERIOR) {
+                if (p <= 1) { edge_z[p * pw + idx] = zo; edge_g[p * pw + idx] = go; }
+                if (p >= ny - 2) {
+                    const int w = (4 - (ny - p)) * pw + idx;  // ny-2 -> 2, ny-1 -> 3
+                    edge_z[w] = zo;
+                    edge_g[w] = go;
+                }
+                const int w = 4 * pw + p - (R0 - 2);
+                if (c <= 1) { edge_z[w + c * sr] = zo; edge_g[w + c * sr] = go; }
+                if (c >= nx - 2) {
+                    edge_z[w + (4 - (nx - c)) * sr] = zo;
+                    edge_g[w + (4 - (nx - c)) * sr] = go;
+                }
+                if (p == 0 || p == ny - 1 || c == 0 || c == nx - 1) return;
             }
-            ECell<T> e3[CPT];
-            T xe3[CPT], Fy[CPT];
-#pragma unroll
-            for (int k = 0; k < CPT; ++k) {
-                e3[k] = ECell<T>{};
-                xe3[k] = Fy[k] = T(0);
+            const unsigned i = (unsigned)p * upitch + (unsigned)c;
+            if (AVG) {
+                oh = T(0.5) * q.h + T(0.5) * oh;
+                ou = T(0.5) * q.hu + T(0.5) * ou;
+                ov = T(0.5) * q.hv + T(0.5) * ov;
+                zo = T(0.5) * q.zb + T(0.5) * zo;
+                go = T(0.5) * q.G + T(0.5) * go;
             }
-            if (S || rowD) {  // warp-uniform: row q is outside the band's rows in some prologue / drain iterations
-#pragma unroll
-                for (int k = 0; k < CPT; ++k) {
-                    const T Gq = MPM ? mpm_grass(hbh[k], hbu[k], hbv[k], mq[k], a.sed) : const_grass(hbh[k], gb1[k], mq[k]);
-                    e3[k] = make_ecell(hbh[k], hbu[k], hbv[k], zb1[k], Gq);
-                }
-                // Below the Shields threshold G is 0 and every Exner flux is 0 (q = G |u|^2 u):
-                // a warp whose rows q and q-1 carry no G skips the Exner faces, their shuffles
-                // and activity tests; xe3 and Fy keep their +0.  Exact in both precisions: the
-                // skipped fluxes are +-0, which leave z_b unchanged bit for bit, and a NaN G
-                // (NaN depth or velocity in the MPM factor) is not 0, so it still propagates.
-                bool anyG = false;
-#pragma unroll
-                for (int k = 0; k < CPT; ++k) anyG = anyG || !(e3[k].G == T(0)) || !(e4[k].G == T(0));
-                if (__any_sync(FULL, anyG)) {
-                    ECell<T> ee[CPT];
-                    bool mqe[CPT];
-#pragma unroll
-                    for (int k = 0; k + 1 < CPT; ++k) { ee[k] = e3[k + 1]; mqe[k] = mq[k + 1]; }
-                    ee[CPT - 1] = shfl_down_ecell(e3[0]);
-                    mqe[CPT - 1] = HAS_MASK ? (__shfl_down_sync(FULL, (int)mq[0], 1) != 0) : false;
-                    T F[CPT];
-                    bool xact[CPT];
-#pragma unroll
-                    for (int k = 0; k < CPT; ++k) {
-                        xact[k] = rowD && has_e[k] && exner_active(e3[k], ee[k], mq[k], mqe[k]);
-                        const T Fx = exner_face<T, false>(e3[k], ee[k]);
-                        F[k] = xact[k] ? Fx : T(0);
-                        if (bud_item && xact[k] && out_col[k] && q >= R0 && q < R1 && q >= 1 && q <= ny - 2 &&
-                            (cb + k == 0 || cb + k == nx - 2))
-                            if constexpr (BUD) budbuf[threadIdx.x >> 5][1][lane] += cb + k == 0 ? -(double)F[k] : (double)F[k];
-                    }
-                    T Fw[CPT];
-                    bool wact[CPT];
-#pragma unroll
-                    for (int k = 1; k < CPT; ++k) { Fw[k] = F[k - 1]; wact[k] = xact[k - 1]; }
-                    Fw[0] = __shfl_up_sync(FULL, F[CPT - 1], 1);
-                    wact[0] = (__shfl_up_sync(FULL, (int)xact[CPT - 1], 1) != 0) && lane > 0;
-#pragma unroll
-                    for (int k = 0; k < CPT; ++k) {
-                        // roe_exner.py:710-711: -F of the west face first, then +F of the east face
-                        if (wact[k]) xe3[k] = xe3[k] + (-Fw[k]);
-                        if (xact[k]) xe3[k] = xe3[k] + F[k];
-                        const bool yex = rowD && (S || q - 1 >= L0) && colok[k] && exner_active(e4[k], e3[k], mq1[k], mq[k]);
-                        const T Fyv = exner_face<T, true>(e4[k], e3[k]);
-                        Fy[k] = yex ? Fyv : T(0);
-                        if (bud_item && yex && out_col[k] && (q == 1 || q == ny - 1) && q >= R0 && q < R1 &&
-                            cb + k >= 1 && cb + k <= nx - 2)
-                            if constexpr (BUD) budbuf[threadIdx.x >> 5][1][lane] += q == 1 ? -(double)Fy[k] : (double)Fy[k];
-                    }
-                }
-            }
-
-            // ================= F: z_b update of row r-4
-            T zbp4[CPT], gg4[CPT];
-#pragma unroll
-            for (int k = 0; k < CPT; ++k) {
-                zbp4[k] = T(0);
-                if (S || (r - 4 >= L0 && r - 4 < L1)) {
-                    T acc = xe4[k];
-                    acc = acc + (-fn4[k]);  // north face (roe_exner.py:712)
-                    acc = acc + Fy[k];      // south face (roe_exner.py:713)
-                    if constexpr (is_f32<T>()) zbp4[k] = e4[k].zb - dtdx * acc;
-                    else zbp4[k] = e4[k].zb - dt * acc / dx;
-                }
-                gg4[k] = e4[k].G;
-            }
-
-            // ================= G: second boundary application and stores of row p = r-5
-            const int p = r - 5;
-            const bool rowG = S || ((p >= L0) && (p < L1));
-            T zfin[CPT], gfin[CPT];
-#pragma unroll
-            for (int k = 0; k < CPT; ++k) { zfin[k] = zbp5[k]; gfin[k] = gg5[k]; }
-            if (rowG && (bc_strip || (bc_rows && (p == 0 || p == ny - 1)))) {
-                unsigned flags[CPT];
-                int zdy[CPT], zdx[CPT], gdy[CPT], gdx[CPT];
-                bool anyf = false;
-#pragma unroll
-                for (int k = 0; k < CPT; ++k) {
-                    flags[k] = 0u;
-                    zdy[k] = zdx[k] = gdy[k] = gdx[k] = 0;
-                    if constexpr (ASYNC_RECIPES) {
-                        const unsigned w = zgb[(r - 2) & 3][CPT * lane + k];  // left by the first application of row p
-                        flags[k] = w & 24u;
-                        zdy[k] = (int)((w >> 8) & 15u) - 8;
-                        zdx[k] = (int)((w >> 12) & 15u) - 8;
-                        gdy[k] = (int)((w >> 16) & 15u) - 8;
-                        gdx[k] = (int)((w >> 20) & 15u) - 8;
-                    } else {
-                        const int slot = colok[k] ? ring_slot(p, cb + k, ny, nx) : -1;
-                        if (slot >= 0) {
-                            const pxb_ring_recipe& rc = a.ring[slot];
-                            flags[k] = rc.flags;
-                            zdy[k] = rc.zb_dy; zdx[k] = rc.zb_dx; gdy[k] = rc.g_dy; gdx[k] = rc.g_dx;
-                        }
-                    }
-                    anyf = anyf || ((flags[k] & 24u) != 0u);
-                }
-                if (__any_sync(FULL, anyf)) {
-                    const bool dyrow = (p == 0) || (p == ny - 1);
-                    T zv[CPT], gv[CPT];
-                    fetch_donor<CPT>(dyrow, zdy, zdx, zbp6, zbp5, zbp4, zv);
-                    fetch_donor<CPT>(dyrow, gdy, gdx, gg6, gg5, gg4, gv);
-#pragma unroll
-                    for (int k = 0; k < CPT; ++k) {
-                        if (flags[k] & 8u) zfin[k] = zv[k];
-                        if (flags[k] & 16u) gfin[k] = gv[k];
-                    }
-                }
-            }
-            if (rowG && p >= R0 && p < R1) {
-                if constexpr (ASYNC_PARTNER) {
-                    read_cols<CPT>(pb[r & 1][3], lane, pazb);
-                    if (a.oG) read_cols<CPT>(pb[r & 1][4], lane, paG);
-                }
-#pragma unroll
-                for (int k = 0; k < CPT; ++k) {
-                    if (!out_col[k]) continue;
-                    const unsigned i = (unsigned)p * upitch + (unsigned)(cb + k);
-                    T zo = zfin[k], go = gfin[k];
-                    if (AVG) {
-                        zo = T(0.5) * pazb[k] + T(0.5) * zo;
-                        if (a.oG) go = T(0.5) * paG[k] + T(0.5) * go;
-                    }
-                    a.ozb[i] = zo;
-                    if (a.oG) a.oG[i] = go;
-                    bad |= !d_isfinite(zo);
-                }
-            }
-            if (rowD && q >= R0 && q < R1) {
-                if constexpr (ASYNC_PARTNER) {
-                    read_cols<CPT>(pb[r & 1][0], lane, pah);
-                    read_cols<CPT>(pb[r & 1][1], lane, pahu);
-                    read_cols<CPT>(pb[r & 1][2], lane, pahv);
-                }
-#pragma unroll
-                for (int k = 0; k < CPT; ++k) {
-                    if (!out_col[k]) continue;
-                    const unsigned i = (unsigned)q * upitch + (unsigned)(cb + k);
-                    T oh = sbh[k], ou = sbu[k], ov = sbv[k];
-                    if (AVG) {
-                        oh = T(0.5) * pah[k] + T(0.5) * oh;
-                        ou = T(0.5) * pahu[k] + T(0.5) * ou;
-                        ov = T(0.5) * pahv[k] + T(0.5) * ov;
-                    }
-                    a.oh[i] = oh;
-                    a.ohu[i] = ou;
-                    a.ohv[i] = ov;
-                    bad |= !(d_isfinite(oh) && d_isfinite(ou) && d_isfinite(ov));
-                }
-            }
-
-            // ================= shift the windows
-#pragma unroll
-            for (int k = 0; k < CPT; ++k) {
-                pA[k] = pr[k]; hA[k] = h_r[k]; huA[k] = hu_r[k]; hvA[k] = hv_r[k];
-#pragma unroll
-                for (int m = 0; m < 3; ++m) { xfA[k][m] = xf[k][m]; nfA[k][m] = yP[k][m]; }
-                zt3[k] = zt2[k]; zt2[k] = ztA[k]; ztA[k] = zt_r[k];
-                hr3[k] = hr2[k]; hr2[k] = hr1[k]; hur2[k] = hur1[k]; hvr2[k] = hvr1[k];
-                mwin[k] = (mwin[k] << 1) | (m_r[k] ? 1u : 0u);
-                zin4[k] = zin3[k]; zin3[k] = zin2[k]; zin2[k] = zin1[k]; zin1[k] = zb_r[k];
-                if (!MPM) { gin4[k] = gin3[k]; gin3[k] = gin2[k]; gin2[k] = gin1[k]; gin1[k] = g_r[k]; }
-                hf4h[k] = hf3h[k]; hf4u[k] = hf3u[k]; hf4v[k] = hf3v[k];
-                hf3h[k] = hf2h[k]; hf3u[k] = hf2u[k]; hf3v[k] = hf2v[k];
-                e4[k] = e3[k]; xe4[k] = xe3[k]; fn4[k] = Fy[k];
-                zbp6[k] = zbp5[k]; zbp5[k] = zbp4[k];
-                gg6[k] = gg5[k]; gg5[k] = gg4[k];
-            }
+            a.oh[i] = oh;
+            a.ohu[i] = ou;
+            a.ohv[i] = ov;
+            a.ozb[i] = zo;
+            if (a.oG) a.oG[i] = go;
+            bad |= !(d_isfinite(oh) && d_isfinite(ou) && d_isfinite(ov) && d_isfinite(zo));
         };
-        const int steady0 = min(L0 + 5, L1), steady1 = L1;
-        int r = L0;
-        for (; r < steady0; ++r) iterate(r, std::false_type{});
-        PXB_UNROLL(PXB_STAGE_UNROLL)
-        for (; r < steady1; ++r) iterate(r, std::true_type{});
-        // drain until phase G has stored the band's last row (p = R1 - 1 at r = R1 + 4);
-        // later iterations would only advance the halo rows below the band
-        for (; r < R1 + 5; ++r) iterate(r, std::false_type{});
-        cp_async_wait<0>();  // the buffers are reused by the next item
-        if constexpr (BUD) {  // this item's outflow: the warp's slots in a fixed order
-            double bh = budbuf[threadIdx.x >> 5][0][lane], bz = budbuf[threadIdx.x >> 5][1][lane];
+        // z_b (and G) entering the Exner update: the input's, or on ring cells the values of
+        // the first boundary application
+        auto ring_at = [&](int r) __attribute__((always_inline)) {  // slot of a ring cell, -1 elsewhere
+            if (INTERIOR || idx < lo - 1 || idx > hi + 1 || !(r == 0 || r == ny - 1 || c == 0 || c == nx - 1)) return -1;
+            return r == 0 ? idx : (r == ny - 1 ? pw + idx : 2 * pw + (c == 0 ? 0 : sr) + r - (R0 - 2));
+        };
+        auto bed = [&](int r) __attribute__((always_inline)) {
+            const int s = ring_at(r);
+            return s >= 0 ? slot_zb[s] : __ldg(a.zb + ((unsigned)r * upitch + (unsigned)c));
+        };
+        auto g_in = [&](int r) __attribute__((always_inline)) {
+            const int s = ring_at(r);
+            return s >= 0 ? slot_g[s] : __ldg(a.G + ((unsigned)r * upitch + (unsigned)c));
+        };
+        auto nod = [&](int r) __attribute__((always_inline)) {
+            return HAS_MASK && colok && __ldg(a.nodata + ((unsigned)r * upitch + (unsigned)c)) != 0;
+        };
+        // Below the Shields threshold G is 0 and every Exner flux is 0 (q = G |u|^2 u): a warp
+        // none of whose cells (its rows and the ones next to them) carries sediment leaves z_b
+        // as it is.  Exact in both precisions: the skipped fluxes are +-0, and a NaN G is not 0.
+        bool sediment = false;
+        if (p0 < p1) {
+            for (int r = max(p0 - 1, 0); r < min(p1 + 1, ny); ++r) {
+                const int k = sidx(r, idx);
+                if constexpr (MPM) sediment = sediment || (colok && mpm_may_move(Sh[k], Su[k], Sv[k], a.sed));
+                else sediment = sediment || (colok && !(const_grass(Sh[k], g_in(r), nod(r)) == T(0)));
+            }
+            sediment = __any_sync(FULL, sediment);
+        }
+        if (!sediment) {
+            if (out_col) {
+                T zn[U];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                bh += __shfl_down_sync(FULL, bh, o);
-                bz += __shfl_down_sync(FULL, bz, o);
+                for (int u = 0; u < U; ++u) zn[u] = p0 + u < p1 ? bed(p0 + u) : T(0);
+#pragma unroll 1
+                for (int p = p0; p < p1; p += U) {  // the next U rows' loads are in flight while U rows are stored
+                    Partner<T> q[U];
+                    T zb[U];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        q[u] = qn[u];
+                        zb[u] = zn[u];
+                        qn[u] = partner(p + U + u);
+                        zn[u] = p + U + u < p1 ? bed(p + U + u) : T(0);
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+                        if (p + u < p1) {
+                            const int k = sidx(p + u, idx);
+                            finish(p + u, Sh[k], Su[k], Sv[k], zb[u], T(0), q[u]);
+                        }
+                }
             }
-            if (lane == 0) {
-                a.bud[2 * item] = bh;
-                a.bud[2 * item + 1] = bz;
+        } else {
+            T cu = T(0), cv = T(0), nu = T(0), nv = T(0);  // hu, hv of the current and the next row
+            struct Bed { T zb, g; bool m; };  // what a row's cell needs from HBM, read a row ahead
+            auto fetch = [&](int r) __attribute__((always_inline)) {
+                Bed b{T(0), T(0), false};
+                if ((INTERIOR || colok) && r < ny) {
+                    b.zb = bed(r);
+                    if (!MPM) b.g = g_in(r);
+                    b.m = nod(r);
+                }
+                return b;
+            };
+            auto ecell = [&](int r, const Bed& b, T& hu, T& hv) __attribute__((always_inline)) {
+                T h = T(0);
+                hu = hv = T(0);
+                if (INTERIOR || colok) {
+                    const int k = sidx(r, idx);
+                    h = Sh[k];
+                    hu = Su[k];
+                    hv = Sv[k];
+                }
+                const T G = MPM ? mpm_grass(h, hu, hv, b.m, a.sed) : const_grass(h, b.g, b.m);
+                return make_ecell(h, hu, hv, b.zb, G);
+            };
+            int p = max(p0 - 1, 0);
+            bool m = false, mnext = false;
+            Bed b = fetch(p), bn = fetch(p + 1);
+            Partner<T> q = qn[0];  // row p0
+            ECell<T> e = ecell(p, b, cu, cv);
+            m = b.m;
+            T fn = T(0);
+#pragma unroll 1
+            for (; p < p1; ++p) {
+                // in flight during this row's faces: the bed of row p+2, the partner of row p+1
+                b = bn;
+                mnext = b.m;
+                if (p + 1 < p1) bn = fetch(p + 2);
+                const Partner<T> qp = q;
+                if (p >= p0) q = partner(p + 1);
+                ECell<T> es{};
+                const bool south = p + 1 < ny;
+                if (south) es = ecell(p + 1, b, nu, nv);
+                T fs = T(0);
+                if (south) {
+                    const bool act = colok && exner_active(e, es, m, mnext);
+                    const T F = exner_face<T, true>(e, es);
+                    fs = act ? F : T(0);
+                    if constexpr (BUD && !INTERIOR) {
+                        const int ps = p + 1;
+                        if (act && out_col && (ps == 1 || ps == ny - 1) && ps >= p0 && ps < p1 && c >= 1 && c <= nx - 2)
+                            budz += ps == 1 ? -(double)fs : (double)fs;
+                    }
+                }
+                if (p >= p0) {
+                    T xe = T(0);
+                    const ECell<T> ee = shfl_down_ecell(e);
+                    const bool me = HAS_MASK ? (__shfl_down_sync(FULL, (int)m, 1) != 0) : false;
+                    const bool act = has_e && exner_active(e, ee, m, me);
+                    const T Fx = exner_face<T, false>(e, ee);
+                    const T F = act ? Fx : T(0);
+                    if constexpr (BUD && !INTERIOR) {
+                        if (act && out_col && p >= 1 && p <= ny - 2 && (c == 0 || c == nx - 2))
+                            budz += c == 0 ? -(double)F : (double)F;
+                    }
+                    const T Fw = __shfl_up_sync(FULL, F, 1);
+                    const bool wact = (__shfl_up_sync(FULL, (int)act, 1) != 0) && lane > 0;
+                    // roe_exner.py:710-711: -F of the west face first, then +F of the east face
+                    if (wact) xe = xe + (-Fw);
+                    if (act) xe = xe + F;
+                    T acc = xe;
+                    acc = acc + (-fn);  // north face (roe_exner.py:712)
+                    acc = acc + fs;     // south face (roe_exner.py:713)
+                    T zo;
+                    if constexpr (is_f32<T>()) zo = e.zb - dtdx * acc;
+                    else zo = e.zb - dt * acc / dx;
+                    finish(p, e.h, cu, cv, zo, e.G, qp);
+                }
+                fn = fs;
+                e = es;
+                cu = nu;
+                cv = nv;
+                m = mnext;
             }
+        }
+    }
+
+    // ================= second boundary application and stores of the owned ring cells
+    if (ring_tile) {
+        __syncthreads();
+        for (int k = threadIdx.x; k < nslots; k += blockDim.x) {
+            int r, j;
+            if (!slot_cell(k, r, j) || r < R0 || r >= R1 || j < lo || j > hi) continue;
+            const pxb_ring_recipe rc = recipe(r, j);
+            T oh, ou, ov;
+            // a donor in the same row contributes its first-pass value; a donor in another
+            // row is never a hydro boundary cell (checked at plan creation)
+            apply_hydro(rc, sidx(r, j), oh, ou, ov);
+            // position of the cell among the edge rows / columns, and its donors' positions
+            int at, dz = 0, dg = 0;
+            if (k < 2 * pw) {
+                at = (r == 0 ? 0 : 3) * pw + j;
+                dz = rc.zb_dy * pw + rc.zb_dx;
+                dg = rc.g_dy * pw + rc.g_dx;
+            } else {  // side columns: donors lie in the same row
+                at = 4 * pw + (cstart + j == 0 ? 0 : 3) * sr + r - (R0 - 2);
+                dz = rc.zb_dx * sr;
+                dg = rc.g_dx * sr;
+            }
+            T zo = edge_z[(rc.flags & 8u) ? at + dz : at], go = edge_g[(rc.flags & 16u) ? at + dg : at];
+            const unsigned i = (unsigned)r * upitch + (unsigned)(cstart + j);
+            if (AVG) {
+                oh = T(0.5) * a.ah[i] + T(0.5) * oh;
+                ou = T(0.5) * a.ahu[i] + T(0.5) * ou;
+                ov = T(0.5) * a.ahv[i] + T(0.5) * ov;
+                zo = T(0.5) * a.azb[i] + T(0.5) * zo;
+                if (a.oG) go = T(0.5) * a.aG[i] + T(0.5) * go;
+            }
+            a.oh[i] = oh;
+            a.ohu[i] = ou;
+            a.ohv[i] = ov;
+            a.ozb[i] = zo;
+            if (a.oG) a.oG[i] = go;
+            bad |= !(d_isfinite(oh) && d_isfinite(ou) && d_isfinite(ov) && d_isfinite(zo));
+        }
+    }
+    if constexpr (BUD) {  // this tile's outflow: warps in order, each summed in a fixed order
+        __shared__ double part[2][32];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            budh += __shfl_down_sync(FULL, budh, o);
+            budz += __shfl_down_sync(FULL, budz, o);
+        }
+        if (lane == 0) {
+            part[0][warp] = budh;
+            part[1][warp] = budz;
+        }
+        __syncthreads();
+        if (threadIdx.x < 2) {
+            double s = 0.0;
+            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += part[threadIdx.x][w];
+            a.bud[2 * (size_t)tile + threadIdx.x] = s;
         }
     }
 }
 
-// Whether an item lies away from the grid's boundary: an interior strip (boundary strips
-// are the first two and the last two items of a band, as half-height items) of an
-// interior band, or any item of a grid without boundary recipes.  Such items take the
-// re_stage_item instantiation without boundary code, whose columns are all inside the
-// grid (the same bits, fewer instructions per row).
+// Whether a tile lies away from the grid's boundary (see re_stage_tile).
 template <class T>
-__device__ __forceinline__ bool stage_item_interior(const REStageArgs<T>& a, const int item) {
-    const int ipb = pxb_stage_items_per_band(a.nstrips);
-    const int band = item / ipb, kb = item - band * ipb;
-    return a.ring == nullptr || (ipb > 1 && kb >= 2 && kb < a.nstrips && band > 0 && band < a.nbands - 1);
+__device__ __forceinline__ bool stage_tile_interior(const REStageArgs<T>& a, const int tile) {
+    const int band = tile / a.nstrips, strip = tile - band * a.nstrips;
+    return strip > 0 && strip < a.nstrips - 1 && band > 0 && band < a.nbands - 1;
 }
 
-// Work-queue order of the items: those that run the generic instantiation (the first and
-// the last band, then in every band its boundary strips) come first, so that the items
-// handed out last, which set the kernel's tail, are the uniform interior ones.  A
-// permutation of the item numbers: the results do not depend on it.
 template <class T>
-__device__ __forceinline__ int stage_item_order(const REStageArgs<T>& a, const int q) {
-    const int ipb = pxb_stage_items_per_band(a.nstrips);
-    const int bq = q / ipb, k = q - bq * ipb;
-    const int nb = a.nbands;
-    const int band = (nb < 2 || bq == 0) ? 0 : (bq == 1 ? nb - 1 : bq - 1);
-    // boundary items of a band: kb 0, 1 (first strip) and ipb-2, ipb-1 (last strip)
-    const int kb = (ipb < 4 || k < 2) ? k : (k < 4 ? ipb - 4 + k : k - 2);
-    return band * ipb + kb;
+__device__ __forceinline__ T* stage_shared() {
+    extern __shared__ __align__(16) unsigned char stage_smem_raw[];
+    return reinterpret_cast<T*>(stage_smem_raw);
 }
 
-// The grid is sized to the resident capacity of the device.  A warp's first item is its
-// warp index; further items come from a grid-wide queue (one atomic per item), so warps
-// on lightly loaded SMs take more of them and no SM waits on a fixed share.  The last
-// block to finish resets the queue for the next launch on the stream.
 template <class T, bool MPM, bool HAS_MASK, bool AVG, bool BUD = false>
-__global__ void __launch_bounds__(128, PXB_STAGE_BOUNDS(T, AVG)) re_stage_kernel(const REStageArgs<T> a) {
-    const int lane = threadIdx.x & 31;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    const int nitems = pxb_stage_items_per_band(a.nstrips) * a.nbands;
+__global__ void __launch_bounds__(stage_max_threads(sizeof(T)), stage_min_blocks(sizeof(T)))
+    re_stage_kernel(const __grid_constant__ REStageArgs<T> a) {
     bool bad = false;
-    int item = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    while (item < nitems) {
-        const int it = stage_item_order(a, item);
-        if (stage_item_interior(a, it)) re_stage_item<T, MPM, HAS_MASK, AVG, BUD, true>(a, it, bad);
-        else re_stage_item<T, MPM, HAS_MASK, AVG, BUD, false>(a, it, bad);
-        unsigned next = 0;
-        if (lane == 0) next = atomicAdd(&a.queue[0], 1u);
-        item = nw + (int)__shfl_sync(FULL, next, 0);
-    }
+    const int tile = blockIdx.x;
+    if (stage_tile_interior(a, tile)) re_stage_tile<T, MPM, HAS_MASK, AVG, BUD, true>(a, tile, stage_shared<T>(), bad);
+    else re_stage_tile<T, MPM, HAS_MASK, AVG, BUD, false>(a, tile, stage_shared<T>(), bad);
     if (bad) atomicOr(a.err, 1);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd(&a.queue[1], 1u) == gridDim.x - 1) {
-            atomicExch(&a.queue[0], 0u);
-            atomicExch(&a.queue[1], 0u);
-        }
-    }
 }
 
 }  // namespace pxb
