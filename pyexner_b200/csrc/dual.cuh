@@ -56,6 +56,15 @@ __device__ inline Dual d_pow(Dual x, Dual y) {
     if (y.d != 0.0) t += log(x.v) * p * y.d;
     return Dual(p, t);
 }
+// x^(4/3), x^(3/2): the values of d_pow43 / d_pow32, the derivatives without a second power
+__device__ inline Dual d_pow43(Dual x) {
+    const double c = cbrt(x.v);
+    return Dual(x.v * c, chain(x.d, (4.0 / 3.0) * c));
+}
+__device__ inline Dual d_pow32(Dual x) {
+    const double s = sqrt(x.v);
+    return Dual(x.v * s, chain(x.d, 1.5 * s));
+}
 __device__ inline Dual d_acos(Dual x) { return Dual(acos(x.v), chain(x.d, -1.0 / sqrt(1.0 - x.v * x.v))); }
 __device__ inline Dual d_cos(Dual x) { return Dual(cos(x.v), chain(x.d, -sin(x.v))); }
 __device__ inline Dual fabs(Dual x) { return Dual(::fabs(x.v), x.v > 0.0 ? x.d : (x.v < 0.0 ? -x.d : 0.0)); }
