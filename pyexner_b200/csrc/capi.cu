@@ -295,8 +295,10 @@ void berthon_constants(const double* v, DevHandler& d) {
     d.q = q;
 }
 
+// Work items of the CFL reduction.
 struct Geometry {
     int band_rows = 0, nstrips = 0, nbands = 0, grid = 0;
+    bool wide = false;
 };
 
 // Tiles of the stage kernel: warps side by side and on top of one another, rows in shared
@@ -305,16 +307,6 @@ struct StageGeometry {
     int wx = 1, wy = 1, srows = 0, band_rows = 0, nstrips = 0, nbands = 0, grid = 0, threads = 0;
     size_t smem = 0;
 };
-
-// CFL work items per resident warp and the shortest band that rule may give (tuning knobs;
-// 4 and 64 against 2 and 32: the same at 2048^2, 10 % faster CFL at 8192^2 with bedload
-// everywhere, where the cubic's cost varies from item to item)
-#ifndef PXB_CFL_ITEMS_PER_WARP
-#define PXB_CFL_ITEMS_PER_WARP 4
-#endif
-#ifndef PXB_CFL_MIN_ROWS
-#define PXB_CFL_MIN_ROWS 64
-#endif
 
 // Dynamic shared memory a stage block may ask for (of 227 KB a block can have; the budget
 // instantiation also has 1 KB of its own).
@@ -395,23 +387,19 @@ StageGeometry stage_geometry(int ny, int nx, int esize, int sm_count, int want_r
     return best;
 }
 
-Geometry cfl_geometry(int ny, int nx, int resident_warps) {
+// Work items of the CFL reduction, about 32 warps of them per SM (16: 24 to 30 % slower at
+// 2048^2, 64 as well).  Below the line a wide item's bounds cost more than evaluating every
+// face of narrow items (float32 731 x 1203: 15.7 us narrow, 27.5 wide; 1024^2 11.2 both;
+// 2048^2 43.8 and 19.3.  float64 512^2: 22.8 and 33; 1024^2 76 and 48).
+Geometry cfl_geometry(int ny, int nx, int esize, int sm_count) {
     Geometry g;
-    g.nstrips = std::max(1, (nx + 30) / 31);
-    // about PXB_CFL_ITEMS_PER_WARP items per resident warp, handed out by the kernel's queue
-    // so that the SMs finish together; where that would make bands shorter than
-    // PXB_CFL_MIN_ROWS rows (each band re-reads one row for its first y-faces) one item per
-    // warp is faster
-    const int target_bands = std::max(1, PXB_CFL_ITEMS_PER_WARP * resident_warps / g.nstrips);
-    g.band_rows = (ny + target_bands - 1) / target_bands;
-    if (g.band_rows < PXB_CFL_MIN_ROWS) {
-        const int one = std::max(1, resident_warps / g.nstrips);
-        g.band_rows = std::max(8, (ny + one - 1) / one);
-    }
-    g.nbands = std::max(1, (ny + g.band_rows - 1) / g.band_rows);
-    const int items = g.nstrips * g.nbands;
-    const int need = std::max(1, (items + 7) / 8), cap = std::max(1, resident_warps / 8);
-    g.grid = need >= cap / 4 ? std::min(need, cap) : need;
+    g.wide = (long long)ny * nx > (esize == 8 ? 500000 : 1200000);
+    g.nstrips = g.wide ? (nx + pxb::CFL_WIDE - 1) / pxb::CFL_WIDE : (nx + pxb::CFL_NARROW - 1) / pxb::CFL_NARROW;
+    const int want = std::max(1, 32 * sm_count / g.nstrips);
+    g.band_rows = std::max(2, (ny + want - 1) / want);
+    if (g.wide) g.band_rows = std::min(pxb::CFL_MAX_ROWS, std::max(4, g.band_rows));
+    g.nbands = (ny + g.band_rows - 1) / g.band_rows;
+    g.grid = (int)(((long long)g.nstrips * g.nbands + 7) / 8);
     return g;
 }
 
@@ -866,6 +854,7 @@ int re_cfl_impl(pxb_re_plan* P, const pxb_re_fields* f, double cfl, void* dt_out
     a.band_rows = P->c.cfl.band_rows;
     a.nstrips = P->c.cfl.nstrips;
     a.nbands = P->c.cfl.nbands;
+    a.wide = P->c.cfl.wide;
     PXB_CUDA(pxb::launch_re_cfl<T>(a, P->nodata != nullptr, P->c.cfl.grid, s));
     return PXB_OK;
 }
@@ -1239,8 +1228,6 @@ const pxb::SedTable<float>& ens_sed<float>(const pxb_re_ens* E) { return E->sedf
 template <>
 const pxb::SedTable<double>& ens_sed<double>(const pxb_re_ens* E) { return E->sedd; }
 
-constexpr int ENS_CFL_ROWS = 32;  // rows per CFL work item
-
 template <class T>
 pxb::REStageArgs<T> ens_stage_args(const pxb_re_ens* E, int k, const pxb_re_fields* in, const pxb_re_fields* out,
                                    const pxb_re_fields* avg, const pxb_re_fields* statics) {
@@ -1335,6 +1322,10 @@ template <class T>
 int ens_build_cfl_tables(pxb_re_ens* E, double cfl, void* dt_log) {
     std::vector<pxb::CflArgs<T>> t[2];
     std::vector<int> base(1, 0);
+    // bands for about 32 warps on every SM, members together
+    long long strip_rows = 0;
+    for (const EnsMember& mb : E->m) strip_rows += (long long)mb.ny * ((mb.nx + pxb::CFL_NARROW - 1) / pxb::CFL_NARROW);
+    const int rows = (int)std::min(64LL, std::max(4LL, strip_rows / (32LL * E->sm_count) + 1));
     for (int k = 0; k < E->nm; ++k) {
         const EnsMember& mb = E->m[(size_t)k];
         for (int v = 0; v < 2; ++v) {
@@ -1354,9 +1345,9 @@ int ens_build_cfl_tables(pxb_re_ens* E, double cfl, void* dt_log) {
             a.scr = E->scr + k;
             a.dt_out = (T*)E->dt + k;
             a.dt_log = (T*)dt_log;
-            a.band_rows = ENS_CFL_ROWS;
-            a.nstrips = std::max(1, (mb.nx + 30) / 31);
-            a.nbands = std::max(1, (mb.ny + ENS_CFL_ROWS - 1) / ENS_CFL_ROWS);
+            a.band_rows = rows;
+            a.nstrips = (mb.nx + pxb::CFL_NARROW - 1) / pxb::CFL_NARROW;
+            a.nbands = (mb.ny + rows - 1) / rows;
             t[v].push_back(a);
         }
         base.push_back(base.back() + t[0].back().nstrips * t[0].back().nbands);
@@ -1391,8 +1382,7 @@ int ens_cfl_launch(pxb_re_ens* E, int v, cudaStream_t s) {
     a.base = E->cfl_base;
     a.nmembers = E->nm;
     a.log_stride = E->nm;
-    const int grid = std::max(1, std::min((E->cfl_total + 7) / 8, 8 * E->sm_count));
-    PXB_CUDA(pxb::launch_ens_cfl<T>(a, E->has_mask, grid, s));
+    PXB_CUDA(pxb::launch_ens_cfl<T>(a, E->has_mask, (E->cfl_total + 7) / 8, s));
     return PXB_OK;
 }
 
@@ -2223,9 +2213,7 @@ int re_plan_create(const pxb_re_config* cfg, DevArena* A, pxb_re_plan** out) {
         delete P;
         return fail(PXB_ERR_CUDA, std::string("stage kernel shared memory: ") + cudaGetErrorString(es));
     }
-    const int cb = f64 ? pxb::re_cfl_blocks_per_sm<double>(cfg->nodata != nullptr)
-                       : pxb::re_cfl_blocks_per_sm<float>(cfg->nodata != nullptr);
-    P->c.cfl = cfl_geometry(cfg->ny, cfg->nx, std::max(1, cb) * 8 * P->c.sm_count);
+    P->c.cfl = cfl_geometry(cfg->ny, cfg->nx, f64 ? 8 : 4, P->c.sm_count);
     *out = P;
     return PXB_OK;
 }

@@ -67,14 +67,6 @@ cudaError_t launch_re_cfl(const CflArgs<T>& a, bool hm, int grid, cudaStream_t s
 }
 
 template <class T>
-int re_cfl_blocks_per_sm(bool hm) {
-    int n = 0;
-    if (hm) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, re_cfl_kernel<T, true>, 256, 0);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, re_cfl_kernel<T, false>, 256, 0);
-    return n;
-}
-
-template <class T>
 cudaError_t launch_re_init(const InitArgs<T>& a, cudaStream_t s) {
     dim3 b(32, 8), g((a.nx + 31) / 32, (a.ny + 7) / 8);
     re_init_kernel<T><<<g, b, 0, s>>>(a);
@@ -155,7 +147,6 @@ cudaError_t launch_roe_cfl(const CflArgs<T>& a, int grid, cudaStream_t s) {
     template cudaError_t launch_re_stage<T>(const REStageArgs<T>&, bool, bool, bool, int, int, size_t, cudaStream_t); \
     template cudaError_t stage_allow_smem<T>(bool, bool, StageUse, size_t);                             \
     template cudaError_t launch_re_cfl<T>(const CflArgs<T>&, bool, int, cudaStream_t);                  \
-    template int re_cfl_blocks_per_sm<T>(bool);                                                         \
     template cudaError_t launch_re_init<T>(const InitArgs<T>&, cudaStream_t);                           \
     template cudaError_t launch_bc<T>(const BcArgs<T>&, cudaStream_t);                                  \
     template cudaError_t launch_re_general<T>(const GenArgs<T>&, int, cudaStream_t);                    \

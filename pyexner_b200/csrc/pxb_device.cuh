@@ -611,7 +611,8 @@ __device__ __forceinline__ T face_speed_nog(const CCell<T>& I, const CCell<T>& J
         ut = (uhi * I.sq + uhj * J.sq) / den;
         ct = d_sqrt(T(G_ACC) * ht);
     }
-    return nan_max(fabs(ut - ct), fabs(ut + ct));
+    // max(|u - c|, |u + c|) is the rounded |u| + c in either sign of u
+    return fabs(ut) + ct;
 }
 
 // Order-preserving map of a non-negative (or NaN) float to unsigned bits for atomicMax.

@@ -35,8 +35,6 @@ template <class T>
 cudaError_t stage_allow_smem(bool mpm, bool has_mask, StageUse use, size_t bytes);
 template <class T>
 cudaError_t launch_re_cfl(const CflArgs<T>& a, bool has_mask, int grid, cudaStream_t s);
-template <class T>
-int re_cfl_blocks_per_sm(bool has_mask);
 // Volume budget (budget.cuh): one stage's boundary outflow into the accumulator; the
 // water and bed volumes of a state into out[2] (device).
 template <class T>

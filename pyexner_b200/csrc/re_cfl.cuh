@@ -10,11 +10,25 @@
 // into dt = max(cfl * dx / smax, 1e-6),
 // resets the accumulator and logs dt.  Deterministic and free of host round trips.
 //
-// Work layout: a warp covers 32 columns and the 31 x-faces between them (strips overlap
-// by one column) and marches down a band of rows; y-faces (r | r+1) belong to row r's band.
+// Work layout: a warp takes an item, a strip of a band of rows.  Narrow items (small grids)
+// evaluate every face of 31 columns.  Wide items (124 columns, four per lane) read every
+// cell once, 16 bytes per lane and plane, and form for each row an upper bound of the speeds
+// of its faces: the largest over the lanes, each from the extremes of h, |u|, |v| and G
+// among the ten cells its faces join.  Exact speeds of one row of 31 columns per item,
+// spread over the grid, give a lower bound of the maximum; only rows whose bound is not
+// below what is known by then are evaluated face by face, shared out over the block's warps
+// (they lie close together: left to the warp that found them, one warp's rows set the
+// kernel's time).  A face that is left out cannot be the fastest, so dt keeps its bits.
+//
+// Bound by the read of h, hu, hv and G (8192^2: 5.9 TB/s) and, on small grids, by the chain
+// of launch, loads, reduction and last block.  Evaluating every face took 125 to 300
+// instructions per row of 31.  us, before -> after: float32 256^2 7.8 -> 5.3, 2048^2 24.6 ->
+// 19.3 and with bedload 51 -> 26, 8192^2 293 -> 185; float64 256^2 36 -> 13, 1024^2 with
+// bedload 64 -> 48.
 #pragma once
+#include <type_traits>
+
 #include "pxb_device.cuh"
-#include "re_stage.cuh"  // cp.async helpers
 
 namespace pxb {
 
@@ -26,8 +40,6 @@ struct CflScratch {
     int pad;
     double t_step;               // simulation time at the start of the current step
     double t_next;               // t_step + dt: the time the next dt is added to
-    unsigned int cfl_queue;      // CFL kernel work queue: items handed out (reset by the last block)
-    unsigned int pad2;
 };
 
 // Start of a fixed-step run at time t0 (the first CFL launch moves it into t_step).
@@ -48,291 +60,361 @@ struct CflArgs {
     T* dt_out;   // device scalar
     T* dt_log;   // optional: dt_log[scr->step++] = dt
     int band_rows, nstrips, nbands;
+    int wide;  // items are 124 columns wide with bounds (else 31, every face)
 };
 
-// Rows in flight ahead of the one the float32 CFL item evaluates (tuning knob; the item
-// does little arithmetic per row, so the copies must cover the memory latency).
-#ifndef PXB_CFL_AHEAD
-#define PXB_CFL_AHEAD 2
-#endif
+constexpr int CFL_WIDE = 124, CFL_NARROW = 31;  // columns of an item
+constexpr int CFL_MAX_ROWS = 64;                // rows of a wide item (a lane keeps two bounds)
 
-// Float32 work item of the CFL reduction (a 31-column strip of one band; the 32nd lane
-// is the first column of the next strip, for the strip's last x-face).  Rows arrive in
-// shared slots of this warp, PXB_CFL_AHEAD rows ahead.  With 16-byte aligned planes and a
-// pitch that is a multiple of 4 elements (VEC), one 16-byte cp.async per lane copies a
-// whole row of the four planes (9 chunks of 4 columns per plane, starting from lane 0's
-// column rounded down to a multiple of 4; the 36 chunks are lanes 0-31 plus lanes 0-3
-// again), so lanes read columns that other lanes copied, after a warp barrier; otherwise
-// each lane copies its own column of each plane, 4 bytes at a time.  Two rows per loop
-// iteration: the cells of the previous row stay where they are.  Columns beyond the grid
-// read as G = 0 (the warp vote below) and never enter a face.
-constexpr int PXB_CFL_RW = 36;  // floats per plane row in a shared slot of the float32 CFL item
-constexpr int PXB_CFL_SLOTS = PXB_CFL_AHEAD < 4 ? 4 : (PXB_CFL_AHEAD < 8 ? 8 : 16);  // a power of two above AHEAD
+// Resident 256-thread blocks per SM: 4 (64 registers; the spills are in the exact rows of wide
+// items) against 2 and 3 is 15 to 30 % faster at 8192^2 in float32.
+constexpr int cfl_min_blocks(int esize) { return esize == 8 ? 2 : 4; }
 
-// cb: this warp's slots (PXB_CFL_SLOTS rows of the four planes, PXB_CFL_RW floats each)
-template <bool HAS_MASK, bool VEC>
-__device__ __forceinline__ void re_cfl_item_f32(const CflArgs<float>& a, const int item, unsigned& best,
-                                                float (*cb)[4][PXB_CFL_RW]) {
-    constexpr int RW = PXB_CFL_RW;
-    const int lane = threadIdx.x & 31;
-    const int ny = a.ny, nx = a.nx;
-    const float DRY = float(DRY_TOL);
-    const int band = item / a.nstrips;
-    const int strip = item - band * a.nstrips;
-    const int c0 = strip * 31;
-    const int c = c0 + lane;
-    const bool colok = c < nx;
-    const bool has_e = colok && (c + 1 < nx) && lane < 31;
-    const int R0 = band * a.band_rows;
-    const int R1 = min(ny, R0 + a.band_rows);
-    const int rend = min(ny, R1 + 1);
-    const unsigned upitch = (unsigned)a.pitch;  // planes are < 2^31 elements
-    constexpr int AHEAD = PXB_CFL_AHEAD;
-    constexpr int SLOTS = PXB_CFL_SLOTS;
-    const int al = VEC ? (c0 & ~3) : c0;
-    const int off = c0 - al;
-    // VEC: this lane's chunks k = lane and k = 32 + lane (lanes 0-3): plane k / 9, columns al + 4 (k % 9)
-    const float* csrc[2];
-    unsigned cdst[2], cbytes[2];
+template <class T>
+using speed_bits_t = typename std::conditional<sizeof(T) == 4, unsigned, unsigned long long>::type;
+
+__device__ __forceinline__ unsigned warp_max_bits(unsigned v) { return __reduce_max_sync(FULL, v); }
+__device__ __forceinline__ unsigned long long warp_max_bits(unsigned long long v) {
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-        const int k = lane + 32 * q;
-        const int pl = min(k / 9, 3), j = k - 9 * (k / 9);
-        const float* base = pl == 0 ? a.h : (pl == 1 ? a.hu : (pl == 2 ? a.hv : a.G));
-        const int col = al + 4 * j;
-        const bool ok = k < 36 && col + 4 <= (int)upitch;  // a chunk never straddles two rows
-        csrc[q] = base + (ok ? col : 0);
-        cbytes[q] = ok ? 16u : 0u;
-        cdst[q] = (unsigned)__cvta_generic_to_shared(&cb[0][pl][4 * (j < 9 ? j : 0)]);
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long w = __shfl_xor_sync(FULL, v, o);
+        v = w > v ? w : v;
     }
-    constexpr unsigned SLOT = 4 * RW * sizeof(float);
-    auto issue = [&](int rr) __attribute__((always_inline)) {  // row rr into slot rr % SLOTS
-        if (rr < rend) {
-            const unsigned ro = (unsigned)rr * upitch;
-            const unsigned so = (unsigned)(rr & (SLOTS - 1)) * SLOT;
-            if constexpr (VEC) {
-                cp_async16_zfill(cdst[0] + so, csrc[0] + ro, cbytes[0]);
-                if (lane < 4) cp_async16_zfill(cdst[1] + so, csrc[1] + ro, cbytes[1]);
-            } else if (colok) {
-                float* d = &cb[rr & (SLOTS - 1)][0][lane];
-                cp_async_elem(d, a.h + ro + c);
-                cp_async_elem(d + RW, a.hu + ro + c);
-                cp_async_elem(d + 2 * RW, a.hv + ro + c);
-                cp_async_elem(d + 3 * RW, a.G + ro + c);
-            }
-        }
-        cp_async_commit();
-    };
-    bool nm = false;
-    auto fetch_mask = [&](int rr) __attribute__((always_inline)) {
-        nm = false;
-        if (HAS_MASK && colok && rr < rend) nm = __ldg(a.nodata + (unsigned)rr * upitch + (unsigned)c) != 0;
-    };
-    auto row = [&](const int r, CCell<float>& cur, bool& mc, const CCell<float>& prev, const bool mp)
-                   __attribute__((always_inline)) {
-        cp_async_wait<AHEAD - 1>();  // row r landed (rows r+1 .. r+AHEAD-1 may be in flight)
-        if constexpr (VEC) __syncwarp();  // chunks copied by other lanes
-        const float* sr = &cb[r & (SLOTS - 1)][0][off + lane];
-        const float h = sr[0], hu = sr[RW], hv = sr[2 * RW];
-        const float g = colok ? sr[3 * RW] : 0.f;
-        issue(r + AHEAD);
-        mc = nm;
-        fetch_mask(r + 1);
-        cur = make_ccell(h, hu, hv, g);
-        // rows r-1 and r of the warp without G (below the Shields threshold) take
-        // face_speed_nog, the same value without a~ and the cubic (a NaN G is not 0)
-        const bool nog = !__any_sync(FULL, !(g == 0.f) || !(prev.G == 0.f));
-        if (r < R1) {  // x-face (c | c+1) of row r
-            CCell<float> e;
-            e.h = __shfl_down_sync(FULL, cur.h, 1);
-            e.sq = __shfl_down_sync(FULL, cur.sq, 1);
-            e.u = __shfl_down_sync(FULL, cur.u, 1);
-            e.v = __shfl_down_sync(FULL, cur.v, 1);
-            const bool me = HAS_MASK ? (__shfl_down_sync(FULL, (int)mc, 1) != 0) : false;
-            // cur.h = max(h, DRY_TOL) > DRY_TOL exactly when h > DRY_TOL (false for NaN)
-            const bool act = has_e && ((cur.h > DRY) || (e.h > DRY)) && !(mc || me);
-            if (nog) {  // branch-free: every lane evaluates, inactive ones are masked
-                const unsigned b = __float_as_uint(face_speed_nog<float, false>(cur, e));
-                best = (act && b > best) ? b : best;
-            } else {
-                e.G = __shfl_down_sync(FULL, cur.G, 1);
-                e.rs = __shfl_down_sync(FULL, cur.rs, 1);
-                // only active faces enter the cubic: a lane without a face (the strip's last, or
-                // beyond the grid) could otherwise send the warp into the float64 fallback
-                if (act) {
-                    const unsigned b = __float_as_uint(face_speed<float, false>(cur, e));
-                    best = b > best ? b : best;
-                }
-            }
-        }
-        if (r > R0) {  // y-face (r-1 | r)
-            const bool act = colok && ((prev.h > DRY) || (cur.h > DRY)) && !(mp || mc);
-            if (nog) {
-                const unsigned b = __float_as_uint(face_speed_nog<float, true>(prev, cur));
-                best = (act && b > best) ? b : best;
-            } else if (act) {
-                const unsigned b = __float_as_uint(face_speed<float, true>(prev, cur));
-                best = b > best ? b : best;
-            }
-        }
-    };
-#pragma unroll
-    for (int k = 0; k < AHEAD; ++k) issue(R0 + k);
-    fetch_mask(R0);
-    CCell<float> pa = make_ccell(1.f, 0.f, 0.f, 0.f), pb = pa;
-    bool ma = false, mb = false;
-    int r = R0;
-    for (; r + 1 < rend; r += 2) {
-        row(r, pb, mb, pa, ma);
-        row(r + 1, pa, ma, pb, mb);
-    }
-    if (r < rend) row(r, pb, mb, pa, ma);
-    cp_async_wait<0>();  // the slots are reused by the next item
-    __syncwarp();
+    return v;
 }
 
-// Largest face-speed bit pattern seen by this lane over one work item (a 32-column strip
-// of one band) folded into `best`; shared by the single-grid and the ensemble kernels.
+// The x-faces (c | c+1) of rows r0 .. r1-1 and the y-faces (r | r+1) below them, for the 31
+// columns from c0 (the 32nd lane is the east neighbour of the last).
+template <class T, bool HAS_MASK>
+__device__ __forceinline__ void cfl_rows(const CflArgs<T>& a, const int c0, const int r0, const int r1,
+                                         speed_bits_t<T>& best) {
+    const int lane = threadIdx.x & 31;
+    const int ny = a.ny, nx = a.nx, c = c0 + lane;
+    const bool colok = c < nx, has_e = lane < 31 && c + 1 < nx;
+    const T DRY = T(DRY_TOL);
+    struct Raw { T h, hu, hv, g; bool m; };
+    auto load = [&](int r) __attribute__((always_inline)) {
+        Raw x{T(1), T(0), T(0), T(0), false};
+        if (colok && r < ny) {
+            const long long i = (long long)r * a.pitch + c;
+            x.h = __ldg(a.h + i);
+            x.hu = __ldg(a.hu + i);
+            x.hv = __ldg(a.hv + i);
+            x.g = __ldg(a.G + i);
+            if (HAS_MASK) x.m = __ldg(a.nodata + i) != 0;
+        }
+        return x;
+    };
+    auto fold = [&](bool act, T s) __attribute__((always_inline)) {
+        const speed_bits_t<T> b = (speed_bits_t<T>)speed_bits(s);
+        best = act && b > best ? b : best;
+    };
+    Raw x = load(r0), nx_ = load(r0 + 1);
+    CCell<T> cur = make_ccell(x.h, x.hu, x.hv, x.g);
+    bool m = x.m;
+    for (int r = r0; r < r1; ++r) {
+        const CCell<T> s = make_ccell(nx_.h, nx_.hu, nx_.hv, nx_.g);
+        const bool ms = nx_.m;
+        if (r + 1 < r1) nx_ = load(r + 2);  // in flight during this row's faces
+        // rows r and r+1 without G (below the Shields threshold) take face_speed_nog, the
+        // same value without a~ and the cubic (a NaN G is not 0)
+        const bool nog = !__any_sync(FULL, !(cur.G == T(0)) || !(s.G == T(0)));
+        CCell<T> e;
+        e.h = __shfl_down_sync(FULL, cur.h, 1);
+        e.sq = __shfl_down_sync(FULL, cur.sq, 1);
+        e.u = __shfl_down_sync(FULL, cur.u, 1);
+        e.v = __shfl_down_sync(FULL, cur.v, 1);
+        const bool me = HAS_MASK ? (__shfl_down_sync(FULL, (int)m, 1) != 0) : false;
+        // cur.h = max(h, DRY_TOL) > DRY_TOL exactly when h > DRY_TOL (false for NaN)
+        const bool ax = has_e && ((cur.h > DRY) || (e.h > DRY)) && !(m || me);
+        const bool ay = colok && r + 1 < ny && ((cur.h > DRY) || (s.h > DRY)) && !(m || ms);
+        if (nog) {
+            fold(ax, face_speed_nog<T, false>(cur, e));
+            fold(ay, face_speed_nog<T, true>(cur, s));
+        } else {
+            e.G = __shfl_down_sync(FULL, cur.G, 1);
+            e.rs = __shfl_down_sync(FULL, cur.rs, 1);
+            // only active faces enter the cubic: a lane without a face could otherwise send
+            // the whole warp into the float64 fallback of the float32 solve
+            if (ax) fold(true, face_speed<T, false>(cur, e));
+            if (ay) fold(true, face_speed<T, true>(cur, s));
+        }
+        cur = s;
+        m = ms;
+    }
+}
+
+// max / min that propagate NaN (max only: a NaN minimum goes with a NaN maximum)
+__device__ __forceinline__ float fmax_nan(float a, float b) { float y; asm("max.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b)); return y; }
+
+// Upper bound of the face speeds among cells with depths (clamped at DRY_TOL) in [hm, hM],
+// velocity components up to U and grass factors up to G, with a margin for the rounding of
+// the bound and of the speeds.  Without G the speeds are |u~| + c~ with u~ between the
+// cells' velocities and c~ <= sqrt(g hM).  With G the speeds are the roots of
+//   l ((l - u)^2 - c^2) = a c^2 (l + u),  a <= A = 4 G U^2 / hm
+// (the sign of l turned).  A root with |l| > |u| has (|l| - |u|)^2 <= c^2 (1 + 2 a), so
+// |l| <= |u| + c sqrt(1 + 2 a).  The trigonometric solution gives the roots when all three
+// are real; at l = -(c - u)/2 (u >= 0) the left side less the right is at least
+// (c - u)^2 (3 c + u) / 8 - a c^2 u, which is positive, and all three are, when
+// A cM^2 U < 0.375 (cm - U)^2 cm.  Otherwise its argument is clipped and its values are
+// within 4/3 |u| + 2/sqrt(3) c sqrt(1 + a).  A NaN makes the bound NaN.
+__device__ __forceinline__ float cfl_bound(float U, float hM, float hm, float G) {
+    const float cM = f_sqrt(9.81f * hM);
+    if (G == 0.f) return (U + cM) * 1.00002f;
+    const float A = 4.f * G * U * U / hm * 1.0001f, cm = f_sqrt(9.81f * hm) - U;
+    const bool three = cm > 0.f && A * cM * cM * U < 0.374f * cm * cm * (cm + U);
+    const float tight = U + cM * f_sqrt(1.f + 2.f * A);
+    const float loose = 1.3334f * U + 1.1548f * cM * f_sqrt(1.f + A);
+    return (three ? tight : loose) * 1.0002f;
+}
+
+// A wide item: strip, rows, and this lane's four columns.
+template <class T>
+struct CflStrip {
+    int c, R0, R1;  // this lane's first column (lane 31: the next strip's), rows
+    bool inner;     // every column of the strip lies in the grid
+    __device__ __forceinline__ CflStrip(const CflArgs<T>& a, int item) {
+        const int band = item / a.nstrips, c0 = (item - band * a.nstrips) * CFL_WIDE;
+        c = c0 + 4 * (threadIdx.x & 31);
+        R0 = band * a.band_rows;
+        R1 = min(a.ny, R0 + a.band_rows);
+        inner = c0 + 128 <= a.nx;
+    }
+};
+template <class T>
+struct CflRow {
+    T h[4], hu[4], hv[4], g[4];
+};
+
+template <class T>
+__device__ __forceinline__ void cfl_load4(const T* p, T (&v)[4]) {
+    if constexpr (sizeof(T) == 4) {
+        const float4 t = __ldg(reinterpret_cast<const float4*>(p));
+        v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w;
+    } else {
+        const double2 t = __ldg(reinterpret_cast<const double2*>(p)), w = __ldg(reinterpret_cast<const double2*>(p) + 1);
+        v[0] = t.x, v[1] = t.y, v[2] = w.x, v[3] = w.y;
+    }
+}
+
+// Row r of a lane's four columns.  VEC: 16-byte aligned planes and a pitch of whole groups
+// of four elements.  Columns beyond the grid: still water of no depth, without G.
+template <class T, bool VEC>
+__device__ __forceinline__ void cfl_load(const CflArgs<T>& a, const CflStrip<T>& st, int r, CflRow<T>& x) {
+    const long long i = (long long)r * a.pitch + st.c;
+    if (VEC && (st.inner || st.c + 4 <= a.pitch)) {
+        cfl_load4(a.h + i, x.h);
+        cfl_load4(a.hu + i, x.hu);
+        cfl_load4(a.hv + i, x.hv);
+        cfl_load4(a.G + i, x.g);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const bool ok = st.c + k < a.nx;
+            x.h[k] = ok ? __ldg(a.h + i + k) : T(0);
+            x.hu[k] = ok ? __ldg(a.hu + i + k) : T(0);
+            x.hv[k] = ok ? __ldg(a.hv + i + k) : T(0);
+            x.g[k] = ok ? __ldg(a.G + i + k) : T(0);
+        }
+    }
+    if (!st.inner) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (st.c + k >= a.nx) x.h[k] = x.hu[k] = x.hv[k] = x.g[k] = T(0);
+    }
+}
+
+// Bounds of the rows of a wide item (x-faces of row r, y-faces (r | r+1)): lane k gets those
+// of rows R0 + k and R0 + 32 + k.
+template <class T, bool VEC>
+__device__ __forceinline__ void cfl_wide_bounds(const CflArgs<T>& a, const CflStrip<T>& st, float& bound0, float& bound1) {
+    const int lane = threadIdx.x & 31, R0 = st.R0, R1 = st.R1, rend = min(a.ny, R1 + 1);
+    using Row = CflRow<T>;
+    auto load = [&](int r, Row& x) __attribute__((always_inline)) { cfl_load<T, VEC>(a, st, r, x); };
+    // extremes of this lane's four cells of a row and the next column's
+    struct Ext { float U, hM, hm, G; };
+    auto extremes = [&](const Row& x) __attribute__((always_inline)) {
+        Ext e{0.f, 0.f, 3e38f, 0.f};
+        float h0 = 0.f, u0 = 0.f, g = 0.f, g0 = 0.f;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float h = clamp_lo((float)x.h[k], (float)DRY_TOL);
+            const float u = fmax_nan(fabsf((float)x.hu[k]), fabsf((float)x.hv[k])) * f_rcp(h);
+            if (k == 0) h0 = h, u0 = u;
+            e.U = fmax_nan(e.U, u);
+            e.hM = fmax_nan(e.hM, h);
+            e.hm = fminf(e.hm, h);
+            g = fmax_nan(g, fabsf((float)x.g[k]));
+            if (k == 0) g0 = g;
+        }
+        e.G = fmax_nan(g, __shfl_down_sync(FULL, g0, 1));
+        const float he = __shfl_down_sync(FULL, h0, 1);
+        e.U = fmax_nan(e.U, __shfl_down_sync(FULL, u0, 1));
+        e.hM = fmax_nan(e.hM, he);
+        e.hm = fminf(e.hm, he);
+        return e;
+    };
+    Row cur, nxt;
+    load(R0, cur);
+    if (R0 + 1 < rend) load(R0 + 1, nxt);
+    Ext pe = extremes(cur);
+    for (int r = R0; r < R1; ++r) {
+        Ext ce = pe;
+        if (r + 1 < rend) {
+            cur = nxt;
+            if (r + 2 < rend) load(r + 2, nxt);
+            ce = extremes(cur);
+        }
+        const float b = cfl_bound(fmax_nan(pe.U, ce.U), fmax_nan(pe.hM, ce.hM), fminf(pe.hm, ce.hm), fmax_nan(pe.G, ce.G));
+        const float w = __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(b)));  // (NaN above all numbers)
+        const int k = r - R0;
+        if (lane == (k & 31)) (k < 32 ? bound0 : bound1) = w;
+        pe = ce;
+    }
+}
+
+// The exact speeds of one row of a wide item, largest bits folded into `best`.
+template <class T, bool HAS_MASK, bool VEC>
+__device__ __forceinline__ void cfl_wide_row(const CflArgs<T>& a, const CflStrip<T>& st, const int r, speed_bits_t<T>& best) {
+    const int lane = threadIdx.x & 31, ny = a.ny, nx = a.nx, c = st.c;
+    using Row = CflRow<T>;
+    auto load = [&](int q, Row& x) __attribute__((always_inline)) { cfl_load<T, VEC>(a, st, q, x); };
+    auto fold = [&](T v) __attribute__((always_inline)) {
+        const speed_bits_t<T> b = (speed_bits_t<T>)speed_bits(v);
+        best = b > best ? b : best;
+    };
+    const bool south = r + 1 < ny;
+    Row x, y;
+    load(r, x);
+    if (south) load(r + 1, y);
+    else y = x;
+    CCell<T> p[5], q[4];
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+        p[n] = make_ccell(x.h[n], x.hu[n], x.hv[n], x.g[n]);
+        q[n] = make_ccell(y.h[n], y.hu[n], y.hv[n], y.g[n]);
+    }
+    p[4].h = __shfl_down_sync(FULL, p[0].h, 1);
+    p[4].sq = __shfl_down_sync(FULL, p[0].sq, 1);
+    p[4].u = __shfl_down_sync(FULL, p[0].u, 1);
+    p[4].v = __shfl_down_sync(FULL, p[0].v, 1);
+    p[4].G = __shfl_down_sync(FULL, p[0].G, 1);
+    p[4].rs = __shfl_down_sync(FULL, p[0].rs, 1);
+    const T DRY = T(DRY_TOL);
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+        bool m = false, me = false, ms = false;
+        if (HAS_MASK) {
+            const long long i = (long long)r * a.pitch + c + n;
+            m = c + n < nx && __ldg(a.nodata + i) != 0;
+            me = c + n + 1 < nx && __ldg(a.nodata + i + 1) != 0;
+            ms = south && c + n < nx && __ldg(a.nodata + i + a.pitch) != 0;
+        }
+        const bool ax = c + n + 1 < nx && (n < 3 || lane < 31) && (p[n].h > DRY || p[n + 1].h > DRY) && !(m || me);
+        const bool ay = south && c + n < nx && (p[n].h > DRY || q[n].h > DRY) && !(m || ms);
+        // without G the same value without the cubic; only active faces enter that (see cfl_rows)
+        if (ax) fold(p[n].G == T(0) && p[n + 1].G == T(0) ? face_speed_nog<T, false>(p[n], p[n + 1])
+                                                            : face_speed<T, false>(p[n], p[n + 1]));
+        if (ay) fold(p[n].G == T(0) && q[n].G == T(0) ? face_speed_nog<T, true>(p[n], q[n])
+                                                      : face_speed<T, true>(p[n], q[n]));
+    }
+}
+
+// Rows left to evaluate by a block of 8 warps.
+struct CflTasks {
+    int count;
+    float bound[8 * CFL_MAX_ROWS];
+    unsigned short who[8 * CFL_MAX_ROWS];  // warp * CFL_MAX_ROWS + row of its item
+};
+
+// Wide items of a block, one per warp (`item`: this warp's, negative for none; `items`: all
+// warps').  Every warp forms its rows' bounds; the rows that
+// may hold the maximum, which tend to lie in few items, are shared out over the block.
+// Returns with `best` covering whatever the block's warps could not rule out.
+template <class T, bool HAS_MASK, bool VEC>
+__device__ __forceinline__ void cfl_wide_block(const CflArgs<T>& a, const int item, const int* items, CflTasks& tasks) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) tasks.count = 0;
+    __syncthreads();
+    if (item >= 0) {
+        const CflStrip<T> st(a, item);
+        speed_bits_t<T> best = 0;
+        {  // the faces of a row of 31 columns somewhere in the grid: items in order step through
+           // the rows, and through the columns by the golden ratio
+            const int r = (int)((long long)a.ny * item / (a.nstrips * a.nbands));
+            const int cs = (int)(((unsigned)item * 2654435769u >> 8) * (unsigned long long)max(1, a.nx - 31) >> 24);
+            cfl_rows<T, HAS_MASK>(a, cs, r, r + 1, best);
+            best = warp_max_bits(best);
+            if (lane == 0 && best) atomicMax(&a.scr->maxbits, (unsigned long long)best);
+        }
+        float b0 = 0.f, b1 = 0.f;
+        cfl_wide_bounds<T, VEC>(a, st, b0, b1);
+        unsigned long long seen = 0ull;
+        if (lane == 0) seen = *(volatile unsigned long long*)&a.scr->maxbits;
+        const float known = (float)bits_speed(__shfl_sync(FULL, seen, 0), T(0));
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+            const float b = n ? b1 : b0;
+            const bool todo = !(b < known) && st.R0 + 32 * n + lane < st.R1;  // (a NaN bound is not below it)
+            const unsigned vote = __ballot_sync(FULL, todo);
+            int at = 0;
+            if (lane == 0 && vote) at = atomicAdd(&tasks.count, __popc(vote));
+            at = __shfl_sync(FULL, at, 0) + __popc(vote & ((1u << lane) - 1u));
+            if (todo) {
+                tasks.bound[at] = b;
+                tasks.who[at] = (unsigned short)(warp * CFL_MAX_ROWS + 32 * n + lane);
+            }
+        }
+    }
+    __syncthreads();
+    for (int t = warp; t < tasks.count; t += 8) {
+        const int w = tasks.who[t] / CFL_MAX_ROWS, k = tasks.who[t] - w * CFL_MAX_ROWS;
+        unsigned long long seen = 0ull;
+        if (lane == 0) seen = *(volatile unsigned long long*)&a.scr->maxbits;
+        seen = __shfl_sync(FULL, seen, 0);
+        if (tasks.bound[t] < (float)bits_speed(seen, T(0))) continue;
+        const CflStrip<T> st(a, items[w]);
+        speed_bits_t<T> best = 0;
+        cfl_wide_row<T, HAS_MASK, VEC>(a, st, st.R0 + k, best);
+        best = warp_max_bits(best);
+        if (lane == 0 && (unsigned long long)best > seen) atomicMax(&a.scr->maxbits, (unsigned long long)best);
+    }
+}
+
+template <class T>
+__device__ __forceinline__ bool cfl_aligned(const CflArgs<T>& a) {
+    return ((((uintptr_t)a.h | (uintptr_t)a.hu | (uintptr_t)a.hv | (uintptr_t)a.G) & 15u) == 0) && ((a.pitch & 3) == 0);
+}
+
+// A narrow item: every face of 31 columns of a band, for this lane.
 template <class T, bool HAS_MASK>
 __device__ __forceinline__ void re_cfl_item(const CflArgs<T>& a, const int item, unsigned long long& best) {
-  if constexpr (is_f32<T>()) {
-    const bool vec = ((((uintptr_t)a.h | (uintptr_t)a.hu | (uintptr_t)a.hv | (uintptr_t)a.G) & 15u) == 0) &&
-                     ((a.pitch & 3) == 0);
-    unsigned b = 0u;
-    __shared__ __align__(16) float cbuf[8][PXB_CFL_SLOTS][4][PXB_CFL_RW];
-    float(*cb)[4][PXB_CFL_RW] = cbuf[(threadIdx.x >> 5) & 7];
-    if (vec) re_cfl_item_f32<HAS_MASK, true>(a, item, b, cb);
-    else re_cfl_item_f32<HAS_MASK, false>(a, item, b, cb);
+    speed_bits_t<T> b = 0;
+    const int band = item / a.nstrips, strip = item - band * a.nstrips;
+    const int R0 = band * a.band_rows;
+    cfl_rows<T, HAS_MASK>(a, strip * CFL_NARROW, R0, min(a.ny, R0 + a.band_rows), b);
     best = (unsigned long long)b > best ? (unsigned long long)b : best;
-  } else {
-    const int lane = threadIdx.x & 31;
-    const int ny = a.ny, nx = a.nx;
-    const T DRY = T(DRY_TOL);
-    {
-        const int band = item / a.nstrips;
-        const int strip = item - band * a.nstrips;
-        const int c = strip * 31 + lane;
-        const bool colok = c < nx;
-        const bool has_e = colok && (c + 1 < nx) && lane < 31;
-        const int R0 = band * a.band_rows;
-        const int R1 = min(ny, R0 + a.band_rows);
-        CCell<T> prev = make_ccell(T(1), T(0), T(0), T(0));
-        T hprev = 0;
-        bool mprev = false;
-        const int rend = min(ny, R1 + 1);
-        // float32: rows arrive by cp.async in this warp's shared slots two rows ahead (the
-        // kernel is memory-latency bound with one row of register prefetch); float64 keeps
-        // the register prefetch of row r+1.  The nodata byte is a register prefetch.
-        constexpr bool ASYNC = is_f32<T>();
-        __shared__ T cbuf[8][ASYNC ? 3 : 1][4][32];
-        T(*cb)[4][32] = cbuf[(threadIdx.x >> 5) & 7];
-        T nh = 1, nhu = 0, nhv = 0, ng = 0;
-        bool nm = false;
-        auto issue = [&](int rr) __attribute__((always_inline)) {  // float32: row rr into slot rr % 3
-            T* d = &cb[rr % 3][0][lane];
-            if (colok && rr < rend) {
-                const long long i = (long long)rr * a.pitch + c;
-                cp_async_elem(d, a.h + i);
-                cp_async_elem(d + 32, a.hu + i);
-                cp_async_elem(d + 64, a.hv + i);
-                cp_async_elem(d + 96, a.G + i);
-            } else {
-                d[0] = T(1);
-                d[32] = d[64] = d[96] = T(0);
-            }
-            cp_async_commit();
-        };
-        auto fetch = [&](int rr) __attribute__((always_inline)) {
-            nm = false;
-            if constexpr (!ASYNC) {
-                nh = 1;
-                nhu = nhv = ng = 0;
-            }
-            if (colok && rr < rend) {
-                const long long i = (long long)rr * a.pitch + c;
-                if constexpr (!ASYNC) {
-                    nh = __ldg(a.h + i);
-                    nhu = __ldg(a.hu + i);
-                    nhv = __ldg(a.hv + i);
-                    ng = __ldg(a.G + i);
-                }
-                if (HAS_MASK) nm = __ldg(a.nodata + i) != 0;
-            }
-        };
-        if constexpr (ASYNC) {
-            issue(R0);
-            issue(R0 + 1);
-        }
-        fetch(R0);
-        for (int r = R0; r < rend; ++r) {
-            T h = nh, hu = nhu, hv = nhv, g = ng;
-            if constexpr (ASYNC) {
-                cp_async_wait<1>();  // row r landed (row r+1 may be in flight); each lane reads its own slots
-                const T* sr = &cb[r % 3][0][lane];
-                h = sr[0];
-                hu = sr[32];
-                hv = sr[64];
-                g = sr[96];
-                issue(r + 2);
-            }
-            const bool m = nm;
-            fetch(r + 1);
-            const CCell<T> cur = make_ccell(h, hu, hv, g);
-            // rows r-1 and r of the warp without G (below the Shields threshold) take
-            // face_speed_nog, the same value without a~ and the cubic (a NaN G is not 0)
-            const bool nog = !__any_sync(FULL, !(g == T(0)) || !(prev.G == T(0)));
-            if (r < R1) {  // x-face (c | c+1) of row r
-                CCell<T> e;
-                e.h = __shfl_down_sync(FULL, cur.h, 1);
-                e.sq = __shfl_down_sync(FULL, cur.sq, 1);
-                e.u = __shfl_down_sync(FULL, cur.u, 1);
-                e.v = __shfl_down_sync(FULL, cur.v, 1);
-                e.G = __shfl_down_sync(FULL, cur.G, 1);
-                e.rs = __shfl_down_sync(FULL, cur.rs, 1);
-                const T he = __shfl_down_sync(FULL, h, 1);
-                const bool me = HAS_MASK ? (__shfl_down_sync(FULL, (int)m, 1) != 0) : false;
-                if (has_e && ((h > DRY) || (he > DRY)) && !(m || me)) {
-                    const unsigned long long b =
-                        speed_bits(nog ? face_speed_nog<T, false>(cur, e) : face_speed<T, false>(cur, e));
-                    best = b > best ? b : best;
-                }
-            }
-            if (r > R0 && colok && ((hprev > DRY) || (h > DRY)) && !(mprev || m)) {  // y-face (r-1 | r)
-                const unsigned long long b =
-                    speed_bits(nog ? face_speed_nog<T, true>(prev, cur) : face_speed<T, true>(prev, cur));
-                best = b > best ? b : best;
-            }
-            prev = cur;
-            hprev = h;
-            mprev = m;
-        }
-        if constexpr (ASYNC) cp_async_wait<0>();  // the slots are reused by the next item
-    }
-  }
 }
 
-// Resident 256-thread blocks per SM the CFL kernel is compiled for (tuning knob; by
-// default the compiler's register choice sets it).
-#ifdef PXB_CFL_MIN_BLOCKS
-#define PXB_CFL_BOUNDS __launch_bounds__(256, PXB_CFL_MIN_BLOCKS)
-#else
-#define PXB_CFL_BOUNDS __launch_bounds__(256)
-#endif
-
+// One item per warp.  Wide items of one block lie far apart (the block number runs fastest),
+// so that rows near the fastest faces end up in many blocks.
 template <class T, bool HAS_MASK>
-__global__ void PXB_CFL_BOUNDS re_cfl_kernel(const CflArgs<T> a) {
+__global__ void __launch_bounds__(256, cfl_min_blocks(sizeof(T))) re_cfl_kernel(const __grid_constant__ CflArgs<T> a) {
     const int lane = threadIdx.x & 31;
-    const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    unsigned long long best = 0ull;
     const int nitems = a.nstrips * a.nbands;
-    // first item by warp index, the rest from a grid-wide queue (faster warps take more)
-    int item = wid;
-    while (item < nitems) {
-        re_cfl_item<T, HAS_MASK>(a, item, best);
-        unsigned next = 0;
-        if (lane == 0) next = atomicAdd(&a.scr->cfl_queue, 1u);
-        item = nw + (int)__shfl_sync(FULL, next, 0);
+    unsigned long long best = 0ull;
+    if (a.wide) {
+        __shared__ CflTasks tasks;
+        __shared__ int items[8];
+        const int w = threadIdx.x >> 5, n = w * gridDim.x + blockIdx.x;
+        const int item = n < nitems ? n : -1;
+        if (lane == 0) items[w] = item;
+        if (cfl_aligned(a)) cfl_wide_block<T, HAS_MASK, true>(a, item, items, tasks);
+        else cfl_wide_block<T, HAS_MASK, false>(a, item, items, tasks);
+        __syncthreads();  // the block's maxima before its ticket
+    } else {
+        const int item = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+        if (item < nitems) re_cfl_item<T, HAS_MASK>(a, item, best);
     }
     // warp max, block max through shared memory, one atomic and one fence per block
     for (int o = 16; o > 0; o >>= 1) {
@@ -365,7 +447,6 @@ __global__ void PXB_CFL_BOUNDS re_cfl_kernel(const CflArgs<T> a) {
         if (!d_isfinite(dt)) a.scr->err |= 2;
         a.scr->maxbits = 0ull;
         a.scr->done = 0u;
-        a.scr->cfl_queue = 0u;  // every warp has left its item loop
         __threadfence();
     }
 }

@@ -107,22 +107,6 @@ struct REStageArgs {
     double* bud;
 };
 
-// Asynchronous global -> shared copies of one element (cp.async, completion by group).
-template <class T>
-__device__ __forceinline__ void cp_async_elem(T* smem, const T* gmem) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    if constexpr (sizeof(T) == 4) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
-    else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-// cp.async of 16 bytes with zero fill: the first src_bytes (0-16) bytes are read, the
-// rest of the 16 is set to zero; with src_bytes = 0 nothing is read.
-__device__ __forceinline__ void cp_async16_zfill(unsigned smem, const void* gmem, unsigned src_bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem), "l"(gmem), "r"(src_bytes) : "memory");
-}
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-
 template <class T>
 __device__ __forceinline__ HCell<T> shfl_down_hcell(const HCell<T>& p) {
     HCell<T> q;
