@@ -261,38 +261,30 @@ __global__ void __launch_bounds__(256) adj_hydro_kernel(const AdjArgs a) {
 
 // ---------------------------------------------------------------- handlers backwards
 
-// pass 1: the boundary cells' adjoints of the fields the handler writes
-__global__ void adj_bc_read_kernel(const AdjBcArgs a) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= a.count) return;
-    const unsigned fm = bc_field_mask(a.kind);
-    const long long b = a.cells[k];
-    for (int s = 0; s < 6; ++s) a.tmp[s * a.count + k] = ((fm >> s) & 1u) && a.f[s] ? a.f[s][b] : 0.0;
+// The adjoint of one boundary cell's fields that the handler writes, saved and cleared (they
+// were overwritten).
+__device__ __forceinline__ void adj_bc_take(const AdjBcSet& a, const AdjBcHandler& h, const int k) {
+    const unsigned fm = bc_field_mask(h.kind);
+    const long long b = h.cells[k];
+#pragma unroll
+    for (int s = 0; s < 6; ++s) {
+        const bool w = ((fm >> s) & 1u) && a.f[s];
+        a.tmp[s * h.count + k] = w ? __ldcg(a.f[s] + b) : 0.0;  // (past the L1: atomics of the handler before)
+        if (w) a.f[s][b] = 0.0;
+    }
 }
 
-// pass 2: the overwritten fields of the boundary cells lose their adjoint
-__global__ void adj_bc_zero_kernel(const AdjBcArgs a) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= a.count) return;
-    const unsigned fm = bc_field_mask(a.kind);
-    const long long b = a.cells[k];
-    for (int s = 0; s < 6; ++s)
-        if (((fm >> s) & 1u) && a.f[s]) a.f[s][b] = 0.0;
-}
-
-// pass 3: donors receive the transposed Jacobian of the handler times the saved adjoints
-__global__ void adj_bc_scatter_kernel(const AdjBcArgs a) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= a.count) return;
-    const long long d = a.donors[k];
+// The donor receives the transposed Jacobian of the handler times the saved adjoints.
+__device__ __forceinline__ void adj_bc_give(const AdjBcSet& a, const AdjBcHandler& h, const int k) {
+    const long long d = h.donors[k];
     const double* t = a.tmp;
-    const int n = a.count;
+    const int n = h.count;
     auto add = [&](int s, double v) {
         if (a.f[s] && v != 0.0) atomicAdd(a.f[s] + d, v);
     };
-    switch (a.kind) {
+    switch (h.kind) {
         case PXB_BC_RE_REFLECTIVE: {  // hu' = (-nx^2 + ny^2) hu - 2 nx ny hv, hv' = -2 nx ny hu + (nx^2 - ny^2) hv
-            const double nx = a.nx, ny = a.ny;
+            const double nx = h.nx, ny = h.ny;
             // forward: mom_n = hu nx + hv ny, mom_t = -hu ny + hv nx, hu' = -mom_n nx - mom_t ny,
             // hv' = -mom_n ny + mom_t nx
             const double bu = t[1 * n + k], bv = t[2 * n + k];
@@ -318,17 +310,30 @@ __global__ void adj_bc_scatter_kernel(const AdjBcArgs a) {
             add(2, t[2 * n + k]);
             break;
         case PXB_BC_RE_ZEROMOMENTUM:  // NaN values keep the cell's own momentum (its donor)
-            if (a.c0 != a.c0) add(1, t[1 * n + k]);
-            if (a.c1 != a.c1) add(2, t[2 * n + k]);
+            if (h.c0 != h.c0) add(1, t[1 * n + k]);
+            if (h.c1 != h.c1) add(2, t[2 * n + k]);
             break;
         case PXB_BC_RE_CONSTANTINFLUX:  // prescribed hu = q values[1], hv = q values[2]: the adjoint of q
-            if (a.qbar) {
-                const double v = t[1 * n + k] * a.vx + t[2 * n + k] * a.vy;
-                if (v != 0.0) atomicAdd(a.qbar, v);
+            if (h.qbar) {
+                const double v = t[1 * n + k] * h.vx + t[2 * n + k] * h.vy;
+                if (v != 0.0) atomicAdd(h.qbar, v);
             }
             break;
         default:  // Berthon: prescribed values
             break;
+    }
+}
+
+// Handlers backwards, the last one first, by one block (three launches per handler took 2 us
+// each).  Atomics of one handler are complete, as seen by the block, before the next takes.
+__global__ void __launch_bounds__(1024) adj_bc_set_kernel(const __grid_constant__ AdjBcSet a) {
+    for (int q = a.n - 1; q >= 0; --q) {
+        const AdjBcHandler& h = a.h[q];
+        for (int k = threadIdx.x; k < h.count; k += blockDim.x) adj_bc_take(a, h, k);
+        __syncthreads();
+        for (int k = threadIdx.x; k < h.count; k += blockDim.x) adj_bc_give(a, h, k);
+        __threadfence();
+        __syncthreads();
     }
 }
 

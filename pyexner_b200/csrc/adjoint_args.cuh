@@ -26,17 +26,22 @@ struct AdjArgs {
     double* tbar;   // MPM table of the one sediment class: np2, sm1d, thc, np3sg, sm1, frac, 1 - porosity
 };
 
-// Field slots as BcArgs: 0 h, 1 hu, 2 hv, 3 z_b, 4 n (not carried), 5 G.
-struct AdjBcArgs {
-    double* f[6];
+// Field slots as BcFields: 0 h, 1 hu, 2 hv, 3 z_b, 4 n (not carried), 5 G.
+struct AdjBcHandler {
     const long long* cells;
     const long long* donors;
     int count, kind;
     double nx, ny;
     double c0, c1;  // ZeroMomentum values (NaN: identity)
-    double* tmp;    // 6 * count
     double vx, vy;  // ConstantInflux: d(hu, hv) / d values[0] = (values[1], values[2])
     double* qbar;   // ConstantInflux: adjoint of its values[0] (accumulated; null: not requested)
+};
+constexpr int ADJ_BC_SET_MAX = 16;
+struct AdjBcSet {  // in the order of application; run backwards
+    double* f[6];
+    double* tmp;  // 6 * the largest count
+    int n;
+    AdjBcHandler h[ADJ_BC_SET_MAX];
 };
 
 struct AdjCflArgs {

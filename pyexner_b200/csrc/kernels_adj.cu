@@ -39,12 +39,13 @@ cudaError_t launch_adj_compute_n(int ny, int nx, long long pitch, int mpm, const
     return cudaGetLastError();
 }
 
-cudaError_t launch_adj_bc(const AdjBcArgs& a, cudaStream_t s) {
-    if (a.count <= 0) return cudaSuccess;
-    const int g = (a.count + 255) / 256;
-    adj_bc_read_kernel<<<g, 256, 0, s>>>(a);
-    adj_bc_zero_kernel<<<g, 256, 0, s>>>(a);
-    adj_bc_scatter_kernel<<<g, 256, 0, s>>>(a);
+cudaError_t launch_adj_bc(const AdjBcSet& a, cudaStream_t s) {
+    if (a.n <= 0) return cudaSuccess;
+    int most = 0;
+    for (int k = 0; k < a.n; ++k) most = a.h[k].count > most ? a.h[k].count : most;
+    const int threads = most >= 1024 ? 1024 : (most + 31) / 32 * 32;
+    if (threads == 0) return cudaSuccess;
+    adj_bc_set_kernel<<<1, threads, 0, s>>>(a);
     return cudaGetLastError();
 }
 

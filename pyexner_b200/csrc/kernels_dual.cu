@@ -29,6 +29,7 @@ cudaError_t launch_dual_unpack(int ny, int nx, long long pitch, const Dual* in, 
 
 template cudaError_t launch_re_general<Dual>(const GenArgs<Dual>&, int, cudaStream_t);
 template cudaError_t launch_bc<Dual>(const BcArgs<Dual>&, cudaStream_t);
+template cudaError_t launch_bc_set<Dual>(const BcSet<Dual>&, cudaStream_t);
 template cudaError_t launch_re_init<Dual>(const InitArgs<Dual>&, cudaStream_t);
 
 }  // namespace pxb

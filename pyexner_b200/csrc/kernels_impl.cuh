@@ -1,5 +1,6 @@
 // Launchers shared by the float and double translation units.
 #pragma once
+#include <algorithm>
 #include <type_traits>
 
 #include "pxb_launch.h"
@@ -75,10 +76,23 @@ cudaError_t launch_re_init(const InitArgs<T>& a, cudaStream_t s) {
 
 template <class T>
 cudaError_t launch_bc(const BcArgs<T>& a, cudaStream_t s) {
-    if (a.count <= 0) return cudaSuccess;
-    const int g = (a.count + 255) / 256;
+    if (a.h.count <= 0) return cudaSuccess;
+    const int g = (a.h.count + 255) / 256;
     bc_gather_kernel<T><<<g, 256, 0, s>>>(a);
     bc_scatter_kernel<T><<<g, 256, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
+template <class T>
+cudaError_t launch_bc_set(const BcSet<T>& a, cudaStream_t s) {
+    if (a.n <= 0) return cudaSuccess;
+    // a warp for every 32 cells of the largest level, up to the block's 32
+    int most = 0, level = 0;
+    for (int k = 0; k < a.n; ++k) {
+        level = (a.h[k].level ? 0 : level) + (a.h[k].count + 31) / 32;
+        most = std::max(most, level);
+    }
+    bc_set_kernel<T><<<1, 32 * std::max(1, std::min(32, most)), 0, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -149,6 +163,7 @@ cudaError_t launch_roe_cfl(const CflArgs<T>& a, int grid, cudaStream_t s) {
     template cudaError_t launch_re_cfl<T>(const CflArgs<T>&, bool, int, cudaStream_t);                  \
     template cudaError_t launch_re_init<T>(const InitArgs<T>&, cudaStream_t);                           \
     template cudaError_t launch_bc<T>(const BcArgs<T>&, cudaStream_t);                                  \
+    template cudaError_t launch_bc_set<T>(const BcSet<T>&, cudaStream_t);                               \
     template cudaError_t launch_re_general<T>(const GenArgs<T>&, int, cudaStream_t);                    \
     template cudaError_t launch_ens_stage<T>(const EnsStageArgs<T>&, bool, bool, bool, int, int, size_t, \
                                              cudaStream_t);                                             \

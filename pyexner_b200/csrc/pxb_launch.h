@@ -46,7 +46,9 @@ cudaError_t launch_volume(int ny, int nx, long long pitch, const T* h, const T* 
 template <class T>
 cudaError_t launch_re_init(const InitArgs<T>& a, cudaStream_t s);
 template <class T>
-cudaError_t launch_bc(const BcArgs<T>& a, cudaStream_t s);
+cudaError_t launch_bc(const BcArgs<T>& a, cudaStream_t s);      // one handler
+template <class T>
+cudaError_t launch_bc_set(const BcSet<T>& a, cudaStream_t s);   // several, in one launch
 // Phases of the general stage path (re_general.cuh).
 enum GenPhase { GEN_HYDRO = 0, GEN_CORR = 1, GEN_GRASS = 2, GEN_EXNER = 3, GEN_STORE = 4 };
 template <class T>
@@ -56,12 +58,12 @@ cudaError_t launch_set_time(CflScratch* scr, double t0, cudaStream_t s);
 
 // Reverse mode (kernels_adj.cu); the argument structs are in adjoint_args.cuh.
 struct AdjArgs;
-struct AdjBcArgs;
+struct AdjBcSet;
 struct AdjCflArgs;
 cudaError_t launch_adj_store(int ny, int nx, long long pitch, double scale, const double* const o[5], double* const S[5],
                              double* const A[5], cudaStream_t s);
 cudaError_t launch_adj_stage(const AdjArgs& a, int phase, cudaStream_t s);
-cudaError_t launch_adj_bc(const AdjBcArgs& a, cudaStream_t s);
+cudaError_t launch_adj_bc(const AdjBcSet& a, cudaStream_t s);
 cudaError_t launch_adj_cfl(const AdjCflArgs& a, cudaStream_t s);
 cudaError_t launch_adj_compute_n(int ny, int nx, long long pitch, int mpm, const double* zb, double* nbbar,
                                  double* nbar, double* npbar, cudaStream_t s);
