@@ -127,10 +127,9 @@ cudaError_t launch_set_time(CflScratch* scr, double t0, cudaStream_t s) {
 
 template <class T>
 cudaError_t launch_roe_stage(const RoeArgs<T>& a, bool avg, cudaStream_t s) {
-    const long long threads = 4LL * a.ny * a.nx;  // four threads per cell
-    const int g = (int)((threads + 255) / 256);
-    if (avg) roe_stage_kernel<T, true><<<g, 256, 0, s>>>(a);
-    else roe_stage_kernel<T, false><<<g, 256, 0, s>>>(a);
+    const int g = roe_tiles(a.nx, ROE_TX) * roe_tiles(a.ny, ROE_TY);
+    if (avg) roe_stage_kernel<T, true><<<g, ROE_THREADS, 0, s>>>(a);
+    else roe_stage_kernel<T, false><<<g, ROE_THREADS, 0, s>>>(a);
     return cudaGetLastError();
 }
 

@@ -1,11 +1,14 @@
 // Plain Roe shallow-water step (no Exner): PyExner src/PyExner/solvers/kernels/roe.py
 // and src/PyExner/solvers/roe_solver.py.
 //
-// Four threads per cell, one face each (every face is evaluated by both of its cells).
-// Ring cells with boundary recipes recompute the update of their donor cell instead of
-// reading it, so the stage is one launch with no global synchronisation.  The plain Roe
-// configuration is small (258 x 258) and latency-bound; the Roe-Exner stage is the one
-// built for bandwidth.
+// A block computes a tile of 16 x 8 cells: one thread per face of the tile into shared
+// memory, then one thread per cell sums its four faces; ring cells with boundary recipes
+// take their donor's update from shared memory, so the stage is one launch.  The
+// configuration this solver is used for is small (258 x 258, float64): four threads per cell
+// evaluated every face twice (and the donors' faces again), and a face's seven quotients and
+// power took 64 registers with spills.  Bound by the float64 pipe and the length of a face's
+// chain; us per SSPRK2 step with its dt, before -> after: float64 256^2 72 -> 29, 700^2 299 ->
+// 112; float32 256^2 39 -> 21, 1000^2 299 -> 145.
 #pragma once
 #include "pxb_device.cuh"
 
@@ -34,17 +37,19 @@ __device__ __forceinline__ void roe_plain_face(T hi, T hui, T hvi, T zi, T ni, T
     hi = hi > DRY ? hi : T(0);
     hj = hj > DRY ? hj : T(0);
     const T sqi = d_sqrt(hi), sqj = d_sqrt(hj);
-    const T ui = hi > T(0) ? hui / hi : T(0);
-    const T vi = hi > T(0) ? hvi / hi : T(0);
-    const T uj = hj > T(0) ? huj / hj : T(0);
-    const T vj = hj > T(0) ? hvj / hj : T(0);
+    const DivBy<T> by_hi(hi), by_hj(hj);
+    const T ui = hi > T(0) ? by_hi(hui) : T(0);
+    const T vi = hi > T(0) ? by_hi(hvi) : T(0);
+    const T uj = hj > T(0) ? by_hj(huj) : T(0);
+    const T vj = hj > T(0) ? by_hj(hvj) : T(0);
     const T uhi = YF ? -vi : ui, vhi = YF ? ui : vi;
     const T uhj = YF ? -vj : uj, vhj = YF ? uj : vj;
     const T hsum = T(0.5) * (hi + hj);
     const T ht = hsum > DRY ? hsum : T(0);
     const T ct = d_sqrt(T(G_ACC) * ht);
-    const T ut = (uhi * sqi + uhj * sqj) / (sqi + sqj);
-    const T vt = (vhi * sqi + vhj * sqj) / (sqi + sqj);
+    const DivBy<T> by_sq(sqi + sqj);
+    const T ut = by_sq(uhi * sqi + uhj * sqj);
+    const T vt = by_sq(vhi * sqi + vhj * sqj);
     T l1 = ut - ct;
     const T l2 = ut;
     T l3 = ut + ct;
@@ -67,9 +72,11 @@ __device__ __forceinline__ void roe_plain_face(T hi, T hui, T hvi, T zi, T ni, T
         }
     }
     const T den = l1 - l3 + T(VEL_TOL);
-    const T p00 = -l3 / den, p01 = T(1) / den;
-    const T p10 = -vt / ct, p12 = T(1) / ct;
-    const T p20 = l1 / den, p21 = T(-1) / den;
+    // (with ct = 0 the second wave is not a number, whichever way p10 comes out: b2 below)
+    const DivBy<T> by_den(den), by_ct(ct);
+    const T p00 = by_den(-l3), p01 = by_den(T(1));
+    const T p10 = by_ct(-vt), p12 = T(1) / ct;
+    const T p20 = by_den(l1), p21 = -p01;
     const T dh = hj - hi;
     const T dhu = hj * uhj - hi * uhi;
     const T dhv = hj * vhj - hi * vhi;
@@ -89,7 +96,7 @@ __device__ __forceinline__ void roe_plain_face(T hi, T hui, T hvi, T zi, T ni, T
     const bool mt = (dz * dd >= T(0)) && (ut * dz > T(0));
     const T thrust = mt ? nan_max(thrust_a, thrust_b) : thrust_b;
     const T nt = T(0.5) * (ni + nj);
-    const T sf = (nt * nt * d_sqrt(ut * ut + vt * vt) * ut) / clamp_lo(d_pow(ht, T(4.0 / 3.0)), T(DRY_TOL));
+    const T sf = (nt * nt * d_sqrt(ut * ut + vt * vt) * ut) / clamp_lo(d_pow43(ht), T(DRY_TOL));
     const T tau = T(G_ACC) * ht * sf * dx;
     const T T1 = thrust - tau;
     // P^-1 (0, T1, 0) (roe.py:159-165)
@@ -98,18 +105,24 @@ __device__ __forceinline__ void roe_plain_face(T hi, T hui, T hvi, T zi, T ni, T
     T b3 = p20 * T(0) + p21 * T1 + T(0) * T(0);
     const T hs1 = hi + a1 - (b1 / l1);
     const T hs3 = hj - a3 + (b3 / l3);
-    const T b1min = -(hi + a1) * fabs(l1);
-    const T b3min = -(hi - a1) * fabs(l3);
-    const T dtf = dx / nan_max(nan_max(fabs(l1), fabs(l2)), fabs(l3));
-    const T dt1s = (dx / T(2) * l1) * (hi / (hi - hs1 + T(VEL_TOL)));
-    const T dt3s = (dx / T(2) * l3) * (hj / (hj - hs3 + T(VEL_TOL)));
-    if ((hs1 < T(0)) && (hs3 > T(0)) && (dt1s < dtf)) {
-        b1 = (-b1min >= b3min) ? b1min : b1;
-        b3 = -b1;
-    }
-    if ((hs1 > T(0)) && (hs3 < T(0)) && (dt3s < dtf)) {
-        b3 = (-b3min >= b3min) ? b1min : b3;
-        b1 = -b3;
+    const bool neg1 = (hs1 < T(0)) && (hs3 > T(0)), neg3 = (hs1 > T(0)) && (hs3 < T(0));
+    if (neg1 || neg3) {
+        const T b1min = -(hi + a1) * fabs(l1);
+        const T b3min = -(hi - a1) * fabs(l3);
+        const T dtf = dx / nan_max(nan_max(fabs(l1), fabs(l2)), fabs(l3));
+        if (neg1) {
+            const T dt1s = (dx / T(2) * l1) * (hi / (hi - hs1 + T(VEL_TOL)));
+            if (dt1s < dtf) {
+                b1 = (-b1min >= b3min) ? b1min : b1;
+                b3 = -b1;
+            }
+        } else {
+            const T dt3s = (dx / T(2) * l3) * (hj / (hj - hs3 + T(VEL_TOL)));
+            if (dt3s < dtf) {
+                b3 = (-b3min >= b3min) ? b1min : b3;
+                b1 = -b3;
+            }
+        }
     }
     const bool mk1 = (hi < DRY) && (hs1 < T(0));
     const bool mk2 = (hj < DRY) && (hs3 < T(0));
@@ -145,46 +158,6 @@ __device__ __forceinline__ void roe_plain_face(T hi, T hui, T hvi, T zi, T ni, T
         P[0] = p0; P[1] = p1; P[2] = p2;
         M[0] = n0; M[1] = n1; M[2] = n2;
     }
-}
-
-// Update of cell (r, c) from its four faces (roe.py:251-315), order of roe.py:296-299.
-// Update of cell (r, c) by the four threads of its quad (adjacent lanes qbase..qbase+3):
-// thread q evaluates face q of the cell (0 east, 1 west, 2 south = row + 1, 3 north =
-// row - 1) and the sums run in that order, the scatter order of roe.py (east upwM, west
-// upwP, south upwM, north upwP).  One face per thread: the 66 k-cell configuration of
-// this path is latency-bound, and four threads per cell keep four times as many in
-// flight as one thread evaluating the four faces in turn.
-template <class T>
-__device__ __forceinline__ void roe_quad_update(const RoeArgs<T>& a, int r, int c, T dt, int q, unsigned qmask,
-                                                int qbase, T out[3]) {
-    const long long p = a.pitch;
-    const long long i = (long long)r * p + c;
-    const bool first = (q & 1) == 0;  // the cell is the face's i side (east, south faces)
-    const bool yf = q >= 2;
-    const bool has = q == 0 ? (c + 1 < a.nx) : q == 1 ? (c >= 1) : q == 2 ? (r + 1 < a.ny) : (r >= 1);
-    const long long j = q == 0 ? i + 1 : q == 1 ? i - 1 : q == 2 ? i + p : i - p;
-    T v[3] = {T(0), T(0), T(0)};
-    if (has) {
-        const long long ii = first ? i : j, jj = first ? j : i;
-        T P[3], M[3];
-        roe_plain_face<T>(a.h[ii], a.hu[ii], a.hv[ii], a.z[ii], a.n[ii], a.h[jj], a.hu[jj], a.hv[jj], a.z[jj], a.n[jj],
-                          a.dx, yf, P, M);
-#pragma unroll
-        for (int m = 0; m < 3; ++m) v[m] = first ? M[m] : P[m];
-    }
-    T f[3] = {T(0), T(0), T(0)};
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const bool hk = __shfl_sync(qmask, (int)has, qbase + k) != 0;
-#pragma unroll
-        for (int m = 0; m < 3; ++m) {
-            const T vk = __shfl_sync(qmask, v[m], qbase + k);
-            if (hk) f[m] = f[m] + vk;
-        }
-    }
-    out[0] = a.h[i] - dt * f[0] / a.dx;
-    out[1] = a.hu[i] - dt * f[1] / a.dx;
-    out[2] = a.hv[i] - dt * f[2] / a.dx;
 }
 
 // The larger of the two speeds of compute_dt for plain Roe (roe.py:13-30) at one cell,
@@ -239,96 +212,110 @@ __device__ __forceinline__ void roe_dt_reduce(unsigned long long best, CflScratc
     __threadfence();
 }
 
-// One stage; four threads per cell.  Ring cells with boundary recipes recompute the
-// update of their donor cell instead of reading it, so the stage is one launch with no
-// global synchronisation.
-// Resident 256-thread blocks per SM the stage is register-limited to (tuning knob): 4
-// (64 registers, a few hundred bytes of spills) runs the 256^2 dam break's 266 k threads
-// in 2 waves instead of 2.3, 3 % faster than 3 (80 registers) and 8 % faster than 2.
+// Tile of a block: at most ROE_TX x ROE_TY cells; the tiles of a row or column of tiles
+// differ by at most one cell and have at least two, so that a ring cell and its donors
+// share one.
+constexpr int ROE_TX = 16, ROE_TY = 8;
+constexpr int ROE_XF = (ROE_TX + 1) * ROE_TY, ROE_YF = ROE_TX * (ROE_TY + 1);  // x-faces, y-faces
+constexpr int ROE_THREADS = (ROE_XF + ROE_YF + 31) / 32 * 32;
+static inline __host__ __device__ int roe_tiles(int n, int t) { return n > t ? (n + t - 1) / t : 1; }
+
+// Resident blocks per SM the stage is register-limited to (tuning knob): 4 (56 registers) takes
+// 29.1 us per step at 256^2 and 112 at 700^2 in float64, 3: 31.1 and 117, 2: 31.1 and 138.
 #ifndef PXB_ROE_MIN_BLOCKS
 #define PXB_ROE_MIN_BLOCKS 4
 #endif
 
+// One stage (roe_solver.py:40-54): update (roe.py:251-315), then the handlers.
 template <class T, bool AVG>
-__global__ void __launch_bounds__(256, PXB_ROE_MIN_BLOCKS) roe_stage_kernel(const RoeArgs<T> a) {
-    const int lane = threadIdx.x & 31;
-    const int qbase = lane & ~3;
-    const unsigned qmask = 0xFu << qbase;
-    const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const long long cell = tid >> 2;
-    const int q = (int)(tid & 3);
-    if (cell >= (long long)a.ny * a.nx) return;  // whole quads leave together
-    const int r = (int)(cell / a.nx), c = (int)(cell - (long long)r * a.nx);
+__global__ void __launch_bounds__(ROE_THREADS, PXB_ROE_MIN_BLOCKS) roe_stage_kernel(const __grid_constant__ RoeArgs<T> a) {
+    __shared__ T fx[6][ROE_XF], fy[6][ROE_YF], up[3][ROE_TX * ROE_TY];  // faces: upwP, upwM
+    const int ntx = roe_tiles(a.nx, ROE_TX), nty = roe_tiles(a.ny, ROE_TY);
+    const int by = blockIdx.x / ntx, bx = blockIdx.x - by * ntx;
+    const int c0 = (int)((long long)a.nx * bx / ntx), c1 = (int)((long long)a.nx * (bx + 1) / ntx);
+    const int r0 = (int)((long long)a.ny * by / nty), r1 = (int)((long long)a.ny * (by + 1) / nty);
     const T dt = *a.dt;
-    const long long i = (long long)r * a.pitch + c;
-    const bool on_ring = (r == 0) || (r == a.ny - 1) || (c == 0) || (c == a.nx - 1);
-    // The same for the four threads of the quad: Roe handlers write h, z and n from one
-    // donor (flags bit 0) and the momentum from another (bit 1: a 2x2 map of the donor's,
-    // or constants with bit 2).
-    unsigned flags = 0u;
-    int hdy = 0, hdx = 0, mdy = 0, mdx = 0;
-    T m0 = T(0), m1 = T(0), m2 = T(0), m3 = T(0);
-    if (on_ring && a.ring != nullptr) {
-        const pxb_ring_recipe& rc = a.ring[ring_slot(r, c, a.ny, a.nx)];
-        flags = rc.flags;
-        hdy = rc.h_dy, hdx = rc.h_dx, mdy = rc.m_dy, mdx = rc.m_dx;
-        m0 = T(rc.m[0]), m1 = T(rc.m[1]), m2 = T(rc.m[2]), m3 = T(rc.m[3]);
-    }
-    // Updates evaluated in turn by one inlined copy of the quad update: the cell itself
-    // (unless both of its parts come from donors), the h donor, the momentum donor.
-    T u[3] = {T(0), T(0), T(0)}, dh[3] = {T(0), T(0), T(0)}, dm[3] = {T(0), T(0), T(0)};
-#pragma unroll 1
-    for (int pass = 0; pass < 3; ++pass) {
-        int rr = r, cc = c;
-        if (pass == 0 && (flags & 3u) == 3u) continue;
-        if (pass == 1) {
-            if (!(flags & 1u)) continue;
-            rr = r + hdy, cc = c + hdx;
-        }
-        if (pass == 2) {
-            if (!(flags & 2u) || (flags & 4u)) continue;
-            rr = r + mdy, cc = c + mdx;
-        }
-        T d[3];
-        roe_quad_update(a, rr, cc, dt, q, qmask, qbase, d);
+    const int t = threadIdx.x;
+    // x-face f of a row lies west of column c0 + f, y-face f of a column north of row r0 + f
+    const bool yf = t >= ROE_XF;
+    const int k = yf ? t - ROE_XF : t;
+    const int row = yf ? k / ROE_TX : k / (ROE_TX + 1), col = yf ? k - row * ROE_TX : k - row * (ROE_TX + 1);
+    const int rj = r0 + row, cj = c0 + col, ri = yf ? rj - 1 : rj, ci = yf ? cj : cj - 1;
+    const bool face = t < ROE_XF + ROE_YF && (yf ? (cj < c1 && rj <= r1 && ri >= 0 && rj < a.ny)
+                                                 : (rj < r1 && cj <= c1 && ci >= 0 && cj < a.nx));
+    if (face) {
+        const long long i = (long long)ri * a.pitch + ci, j = (long long)rj * a.pitch + cj;
+        T P[3], M[3];
+        roe_plain_face<T>(a.h[i], a.hu[i], a.hv[i], a.z[i], a.n[i], a.h[j], a.hu[j], a.hv[j], a.z[j], a.n[j], a.dx, yf, P, M);
 #pragma unroll
         for (int m = 0; m < 3; ++m) {
-            u[m] = pass == 0 ? d[m] : u[m];
-            dh[m] = pass == 1 ? d[m] : dh[m];
-            dm[m] = pass == 2 ? d[m] : dm[m];
+            (yf ? fy[m][k] : fx[m][k]) = P[m];
+            (yf ? fy[3 + m][k] : fx[3 + m][k]) = M[m];
         }
     }
-    T zo = a.z[i], no = a.n[i];
-    if (flags & 1u) {
-        u[0] = dh[0];
-        const long long j = (long long)(r + hdy) * a.pitch + (c + hdx);
-        zo = a.z[j];
-        no = a.n[j];
-    }
-    if (flags & 2u) {
-        if (flags & 4u) {
-            u[1] = m0;
-            u[2] = m1;
-        } else {
-            u[1] = m0 * dm[1] + m1 * dm[2];
-            u[2] = m2 * dm[1] + m3 * dm[2];
+    __syncthreads();
+    const int tr = t / ROE_TX, tc = t - tr * ROE_TX, r = r0 + tr, c = c0 + tc;
+    const bool cell = t < ROE_TX * ROE_TY && r < r1 && c < c1;
+    const long long i = (long long)r * a.pitch + c;
+    T u[3] = {T(0), T(0), T(0)};
+    if (cell) {
+        // scatter order of roe.py:296-299: east upwM, west upwP, south upwM, north upwP
+        T f[3] = {T(0), T(0), T(0)};
+        const int xw = tr * (ROE_TX + 1) + tc, yn = tr * ROE_TX + tc;
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+            if (c + 1 < a.nx) f[m] = f[m] + fx[3 + m][xw + 1];
+            if (c >= 1) f[m] = f[m] + fx[m][xw];
+            if (r + 1 < a.ny) f[m] = f[m] + fy[3 + m][yn + ROE_TX];
+            if (r >= 1) f[m] = f[m] + fy[m][yn];
         }
+        const DivBy<T> by_dx(a.dx);
+        u[0] = a.h[i] - by_dx(dt * f[0]);
+        u[1] = a.hu[i] - by_dx(dt * f[1]);
+        u[2] = a.hv[i] - by_dx(dt * f[2]);
+#pragma unroll
+        for (int m = 0; m < 3; ++m) up[m][t] = u[m];
     }
-    if (q != 0) return;  // the quad's first thread writes the cell
+    __syncthreads();
+    if (!cell) return;
+    // Roe handlers write h, z and n from one donor (flags bit 0) and the momentum from
+    // another (bit 1: a 2x2 map of the donor's, or constants with bit 2).
+    const bool on_ring = (r == 0) || (r == a.ny - 1) || (c == 0) || (c == a.nx - 1);
+    if (on_ring) {
+        T zo = a.z[i], no = a.n[i];
+        if (a.ring != nullptr) {
+            const pxb_ring_recipe& rc = a.ring[ring_slot(r, c, a.ny, a.nx)];
+            if (rc.flags & 1u) {
+                u[0] = up[0][t + rc.h_dy * ROE_TX + rc.h_dx];
+                const long long j = (long long)(r + rc.h_dy) * a.pitch + (c + rc.h_dx);
+                zo = a.z[j];
+                no = a.n[j];
+            }
+            if (rc.flags & 4u) {
+                u[1] = T(rc.m[0]);
+                u[2] = T(rc.m[1]);
+            } else if (rc.flags & 2u) {
+                const int d = t + rc.m_dy * ROE_TX + rc.m_dx;
+                const T du = up[1][d], dv = up[2][d];
+                u[1] = T(rc.m[0]) * du + T(rc.m[1]) * dv;
+                u[2] = T(rc.m[2]) * du + T(rc.m[3]) * dv;
+            }
+        }
+        if (AVG) {
+            zo = T(0.5) * a.az[i] + T(0.5) * zo;
+            no = T(0.5) * a.an[i] + T(0.5) * no;
+        }
+        a.oz[i] = zo;
+        a.on[i] = no;
+    }
     if (AVG) {
         u[0] = T(0.5) * a.ah[i] + T(0.5) * u[0];
         u[1] = T(0.5) * a.ahu[i] + T(0.5) * u[1];
         u[2] = T(0.5) * a.ahv[i] + T(0.5) * u[2];
-        zo = T(0.5) * a.az[i] + T(0.5) * zo;
-        no = T(0.5) * a.an[i] + T(0.5) * no;
     }
     a.oh[i] = u[0];
     a.ohu[i] = u[1];
     a.ohv[i] = u[2];
-    if (on_ring) {
-        a.oz[i] = zo;
-        a.on[i] = no;
-    }
     if (!(d_isfinite(u[0]) && d_isfinite(u[1]) && d_isfinite(u[2]))) atomicOr(a.err, 1);
 }
 
