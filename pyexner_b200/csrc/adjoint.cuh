@@ -125,66 +125,79 @@ __device__ __forceinline__ void adj_sum_add(double* dst, const double (&v)[N]) {
     }
 }
 
+// Derivatives of the Meyer-Peter & Mueller grass factor of one cell (roe_exner.py:85-130):
+// G = sum_k frac g1 g2 d / (1 - porosity) with d = theta - theta_c, g1 = n_p^3 sqrt(g) /
+// ((s-1) sqrt(h)), g2 = 8 sqrt(d) / (theta^1.5 + 1e-5), theta = n_p^2 |u|^2 / ((s-1) d50
+// h^(1/3)).  dh, dhu, dhv: with respect to the cell's planes; par[7] (PAR): with respect to
+// the constants of the one class (n_p^2, (s-1) d50, theta_c, n_p^3 sqrt(g), s-1, fraction,
+// 1 - porosity).  Zero at and below the threshold and in dry cells, as the clamps give.
+template <bool PAR>
+__device__ __forceinline__ void mpm_gradient(double h, double hu, double hv, const SedTable<double>& S, double& dh,
+                                             double& dhu, double& dhv, double (&par)[7]) {
+    dh = dhu = dhv = 0.0;
+#pragma unroll
+    for (int q = 0; q < 7; ++q) par[q] = 0.0;
+    if (!(h > DRY_TOL)) return;
+    const DivBy<double> by_h(h);
+    const double u = by_h(hu), v = by_h(hv), vel2 = u * u + v * v, cb = cbrt(h), sqh = sqrt(h);
+    for (int k = 0; k < S.n; ++k) {
+        const SedT<double>& c = S.s[k];
+        const double per = c.np2 / (c.sm1d * cb);  // theta per |u|^2
+        const double theta = per * vel2, d = theta - c.thc;
+        if (!(d > 0.0)) {  // (a NaN stays in the value, not in the derivatives of other cells)
+            if (d != d) dh = dhu = dhv = d;
+            continue;
+        }
+        const double rt = sqrt(theta), rd = sqrt(d), den = 1.0 / (theta * rt + 1e-5);
+        const double g1 = c.np3sg / (c.sm1 * sqh), amp = c.frac * g1 * 8.0 / S.one_minus_por;
+        const double G = amp * rd * d * den;
+        const double g_d = 1.5 * amp * rd * den;                 // through d
+        const double g_t = g_d - 1.5 * G * rt * den;             // through theta
+        const double t_h = by_h(theta) * (-7.0 / 3.0), t_u = per * 2.0 * by_h(1.0) * g_t;
+        dh += g_t * t_h - 0.5 * by_h(G);
+        dhu += t_u * u;
+        dhv += t_u * v;
+        if (PAR) {
+            par[0] = g_t * theta / c.np2;
+            par[1] = -g_t * theta / c.sm1d;
+            par[2] = -g_d;
+            par[3] = G / c.np3sg;
+            par[4] = -G / c.sm1;
+            par[5] = amp / c.frac * rd * d * den;
+            par[6] = -G / S.one_minus_por;
+        }
+    }
+}
+
 // grass factor backwards, in place on T (G of the state after handlers 1 -> h, hu, hv);
-// PAR: also the adjoint of the MPM constants of the single sediment class (a.tbar), from
-// one evaluation on dual numbers seeded in the cell's h, hu, hv and in those constants
+// PAR: also the adjoint of the MPM constants of the single sediment class (a.tbar).  The
+// derivatives are written out instead of taken from dual numbers with ten tangents.
 template <bool PAR>
 __global__ void __launch_bounds__(256) adj_grass_kernel(const AdjArgs a) {
     int r, c;
     long long i;
     const bool in = adj_cell(a.ny, a.nx, a.pitch, r, c, i);
-    if constexpr (PAR) {
-        double tb[7] = {0, 0, 0, 0, 0, 0, 0};
-        if (in && a.mpm) {
-            using D = DualN<10>;
-            const bool m = adj_nodata(a.nodata, i);
-            SedTable<D> sd;
-            sd.n = 1;
-            sd.s[0].np2 = D::seed(a.sed.s[0].np2, 3);
-            sd.s[0].sm1d = D::seed(a.sed.s[0].sm1d, 4);
-            sd.s[0].thc = D::seed(a.sed.s[0].thc, 5);
-            sd.s[0].np3sg = D::seed(a.sed.s[0].np3sg, 6);
-            sd.s[0].sm1 = D::seed(a.sed.s[0].sm1, 7);
-            sd.s[0].frac = D::seed(a.sed.s[0].frac, 8);
-            sd.one_minus_por = D::seed(a.sed.one_minus_por, 9);
-            const D G = mpm_grass(D::seed(a.sh[i], 0), D::seed(a.shu[i], 1), D::seed(a.shv[i], 2), m, sd);
-            const double gbar = a.TG[i];
-            a.Th[i] += gbar * G.d[0];
-            a.Thu[i] += gbar * G.d[1];
-            a.Thv[i] += gbar * G.d[2];
-            a.TG[i] = 0.0;
+    double tb[7] = {0, 0, 0, 0, 0, 0, 0};
+    if (in) {
+        const bool m = adj_nodata(a.nodata, i);
+        const double gbar = a.TG[i];
+        if (a.mpm) {
+            if (!m) {
+                double dh, dhu, dhv, par[7];
+                mpm_gradient<PAR>(a.sh[i], a.shu[i], a.shv[i], a.sed, dh, dhu, dhv, par);
+                a.Th[i] += gbar * dh;
+                a.Thu[i] += gbar * dhu;
+                a.Thv[i] += gbar * dhv;
+                if (PAR)
 #pragma unroll
-            for (int q = 0; q < 7; ++q) tb[q] = gbar * G.d[3 + q];
-        } else if (in) {
-            a.TG[i] = (!adj_nodata(a.nodata, i) && a.sh[i] > DRY_TOL) ? a.TG[i] : 0.0;
+                    for (int q = 0; q < 7; ++q) tb[q] = gbar * par[q];
+            }
+            a.TG[i] = 0.0;  // MPM recomputes G: the incoming G has no influence
+        } else {
+            a.TG[i] = (!m && a.sh[i] > DRY_TOL) ? gbar : 0.0;
         }
-        adj_sum_add<7>(a.tbar, tb);
-        return;
     }
-    if (!in) return;
-    const bool m = adj_nodata(a.nodata, i);
-    const double gbar = a.TG[i];
-    if (a.mpm) {
-        using D = DualN<3>;
-        SedTable<D> sd;  // the sediment constants as (constant) dual numbers
-        sd.n = a.sed.n;
-        for (int k = 0; k < a.sed.n; ++k) {
-            sd.s[k].np2 = a.sed.s[k].np2;
-            sd.s[k].sm1d = a.sed.s[k].sm1d;
-            sd.s[k].thc = a.sed.s[k].thc;
-            sd.s[k].np3sg = a.sed.s[k].np3sg;
-            sd.s[k].sm1 = a.sed.s[k].sm1;
-            sd.s[k].frac = a.sed.s[k].frac;
-        }
-        sd.one_minus_por = a.sed.one_minus_por;
-        const D G = mpm_grass(D::seed(a.sh[i], 0), D::seed(a.shu[i], 1), D::seed(a.shv[i], 2), m, sd);
-        a.Th[i] += gbar * G.d[0];
-        a.Thu[i] += gbar * G.d[1];
-        a.Thv[i] += gbar * G.d[2];
-        a.TG[i] = 0.0;  // MPM recomputes G: the incoming G has no influence
-    } else {
-        a.TG[i] = (!m && a.sh[i] > DRY_TOL) ? gbar : 0.0;
-    }
+    if constexpr (PAR) adj_sum_add<7>(a.tbar, tb);
 }
 
 // momentum corrections backwards, in place on T (interior cells)
@@ -205,58 +218,211 @@ __global__ void adj_corr_kernel(const AdjArgs a) {
     if (!(active && !stop_v)) a.Thv[i] = 0.0;
 }
 
-// hydro update backwards: I += T (identity paths) + face terms; dt adjoint.  NB: a fifth
-// tangent in the cell's n_b (Manning friction of its faces) adds its adjoint to a.nbbar.
+// Adjoints of the values of one cell that a Roe-Exner face reads (HCell).
+struct HBar {
+    double h, u, v, z, nb;  // clamped depth (with its square root and celerity), velocities, bed, n_b
+};
+
+// One face backwards (roe_exner_face): Pb, Mb are the adjoints of upwP and upwM; bI, bJ
+// receive those of the two cells' values, P and M the fluctuations.  Branches (entropy fix,
+// signs of the speeds, the floor of h^(4/3)) are the forward ones.
+template <bool YF>
+__device__ __forceinline__ void adj_exner_hydro_face(const HCell<double>& I, const HCell<double>& J, const double dx,
+                                                     const double (&Pb)[3], const double (&Mb)[3], HBar& bI, HBar& bJ,
+                                                     double (&P)[3], double (&M)[3]) {
+    const double uI = YF ? -I.v : I.u, vI = YF ? I.u : I.v, uJ = YF ? -J.v : J.u, vJ = YF ? J.u : J.v;
+    const double ht = 0.5 * (I.h + J.h), ct = sqrt(G_ACC * ht);
+    const DivBy<double> by_den(I.sq + J.sq), by_c(ct);
+    const double ut = by_den(uI * I.sq + uJ * J.sq), vt = by_den(vI * I.sq + vJ * J.sq);
+    const double l1r = ut - ct, l3r = ut + ct;
+    const double ei = uI - I.c, ej = uJ - J.c, fi = uI + I.c, fj = uJ + J.c;
+    const bool m1 = ei < 0.0 && ej > 0.0, m3 = fi < 0.0 && fj > 0.0;
+    double l1 = l1r, l3 = l3r, lE1 = 0.0, lE3 = 0.0;
+    if (m1) {
+        l1 = ei * (ej - l1r) / (ej - ei);
+        lE1 = l1r - l1;
+    }
+    if (m3) {
+        const double num = fj * (l3r - fi);
+        lE3 = l3r - num / (fj - fi);
+        l3 = num / ((fj - fi) + VEL_TOL);
+    }
+    const double dh = J.h - I.h, dhu = J.h * uJ - I.h * uI, dhv = J.h * vJ - I.h * vI, dz = J.zt - I.zt;
+    const double a1 = -0.5 * by_c(-l3r * dh + dhu), a2 = by_c(-vt * dh + dhv), a3 = -0.5 * by_c(l1r * dh - dhu);
+    const double nt = 0.5 * (I.nb + J.nb), speed = sqrt(ut * ut + vt * vt), cb = cbrt(ht);
+    const double D43 = ht * cb;
+    const bool floored = D43 < DRY_TOL;
+    const double rD = 1.0 / (floored ? DRY_TOL : D43);
+    const double sf = nt * nt * speed * ut * rD;
+    const double thrust = -G_ACC * ht * dz, tau = G_ACC * ht * sf * dx;
+    const double b1 = -0.5 * by_c(thrust - tau);
+    const double w1 = l1 * a1 - b1, w2 = ut * a2, w3 = l3 * a3 + b1;
+    // fluctuations and their adjoints in the face's frame (1: normal, 2: tangential)
+    const double pb0 = Pb[0], pb1 = YF ? -Pb[2] : Pb[1], pb2 = YF ? Pb[1] : Pb[2];
+    const double nb0 = Mb[0], nb1 = YF ? -Mb[2] : Mb[1], nb2 = YF ? Mb[1] : Mb[2];
+    double p0 = 0, p1 = 0, p2 = 0, n0 = 0, n1 = 0, n2 = 0;
+    double l1b = 0, l3b = 0, a1b = 0, a3b = 0, vtb = 0, b1b = 0, lE1b = 0, lE3b = 0;
+    auto wave = [&](bool pos, double w, double l, double& lb) __attribute__((always_inline)) {  // -> adjoint of w
+        (pos ? p0 : n0) += w;
+        (pos ? p1 : n1) += w * l;
+        (pos ? p2 : n2) += w * vt;
+        const double B0 = pos ? pb0 : nb0, B1 = pos ? pb1 : nb1, B2 = pos ? pb2 : nb2;
+        lb += B1 * w;
+        vtb += B2 * w;
+        return B0 + B1 * l + B2 * vt;
+    };
+    const double w1b = wave(l1 > 0.0, w1, l1, l1b);
+    const double w3b = wave(l3 > 0.0, w3, l3, l3b);
+    l1b += w1b * a1;
+    a1b += w1b * l1;
+    l3b += w3b * a3;
+    a3b += w3b * l3;
+    b1b += w3b - w1b;
+    const bool s2 = ut > 0.0;
+    (s2 ? p2 : n2) += w2 * ct;
+    const double B2 = s2 ? pb2 : nb2, w2b = B2 * ct;
+    double ctb = B2 * w2, utb = w2b * a2, l1rb = 0.0, l3rb = 0.0;
+    const double a2b = w2b * ut;
+    double uIb = 0, uJb = 0, cIb = 0, cJb = 0;
+    if (m1) {
+        const double eb = wave(lE1 > 0.0, lE1 * a1, l1, l1b);
+        lE1b = eb * a1;
+        a1b += eb * lE1;
+        const double dd = 1.0 / (ej - ei), tb = l1b - lE1b;
+        const double eib = tb * ((ej - l1r) + l1) * dd, ejb = tb * (ei - l1) * dd;
+        l1rb += lE1b - tb * ei * dd;
+        uIb += eib, cIb -= eib, uJb += ejb, cJb -= ejb;
+    } else {
+        l1rb += l1b;
+    }
+    if (m3) {
+        const double eb = wave(lE3 > 0.0, lE3 * a3, l3, l3b);
+        lE3b = eb * a3;
+        a3b += eb * lE3;
+        const double d0 = 1.0 / (fj - fi), d1 = 1.0 / ((fj - fi) + VEL_TOL), q = l3r - lE3;
+        const double numb = l3b * d1 - lE3b * d0, d0b = lE3b * q * d0 - l3b * l3 * d1;
+        const double fjb = numb * (l3r - fi) + d0b, fib = -numb * fj - d0b;
+        l3rb += lE3b + numb * fj;
+        uIb += fib, cIb += fib, uJb += fjb, cJb += fjb;
+    } else {
+        l3rb += l3b;
+    }
+    // wave strengths and the source
+    const double y1 = -0.5 * by_c(a1b), y2 = by_c(a2b), y3 = -0.5 * by_c(a3b), yb = -0.5 * by_c(b1b);
+    ctb -= by_c(a1b * a1 + a2b * a2 + a3b * a3 + b1b * b1);
+    l3rb -= y1 * dh;
+    l1rb += y3 * dh;
+    vtb -= y2 * dh;
+    const double dhb = -y1 * l3r - y2 * vt + y3 * l1r, dhub = y1 - y3, dhvb = y2;
+    double htb = -yb * G_ACC * dz - yb * G_ACC * sf * dx;
+    const double dzb = -yb * G_ACC * ht, sfb = -yb * G_ACC * ht * dx;
+    const double ntb = sfb * 2.0 * nt * speed * ut * rD, spb = sfb * nt * nt * ut * rD;
+    utb += sfb * nt * nt * speed * rD;
+    if (!floored) htb -= sfb * sf * rD * (4.0 / 3.0) * cb;
+    if (speed > 0.0) {
+        const double k = spb / speed;
+        utb += k * ut;
+        vtb += k * vt;
+    }
+    utb += l1rb + l3rb;
+    ctb += l3rb - l1rb;
+    htb += 0.5 * G_ACC * by_c(ctb);
+    const double yu = by_den(utb), yv = by_den(vtb);
+    uIb += yu * I.sq - dhub * I.h;
+    uJb += yu * J.sq + dhub * J.h;
+    const double vIb = yv * I.sq - dhvb * I.h, vJb = yv * J.sq + dhvb * J.h;
+    const double sIb = yu * (uI - ut) + yv * (vI - vt), sJb = yu * (uJ - ut) + yv * (vJ - vt);
+    // sqrt(h) and sqrt(g h) of the cells back to their depths
+    bI.h = 0.5 * htb - dhb - dhub * uI - dhvb * vI + 0.5 * sIb / I.sq + 0.5 * G_ACC * cIb / I.c;
+    bJ.h = 0.5 * htb + dhb + dhub * uJ + dhvb * vJ + 0.5 * sJb / J.sq + 0.5 * G_ACC * cJb / J.c;
+    bI.u = YF ? vIb : uIb;
+    bI.v = YF ? -uIb : vIb;
+    bJ.u = YF ? vJb : uJb;
+    bJ.v = YF ? -uJb : vJb;
+    bI.z = -dzb;
+    bJ.z = dzb;
+    bI.nb = bJ.nb = 0.5 * ntb;
+    P[0] = p0, P[1] = YF ? p2 : p1, P[2] = YF ? -p1 : p2;
+    M[0] = n0, M[1] = YF ? n2 : n1, M[2] = YF ? -n1 : n2;
+}
+
+// Tile of adj_hydro_kernel: at most 16 x 8 cells, one thread per face.
+constexpr int ADJ_TX = 16, ADJ_TY = 8;
+constexpr int ADJ_XF = (ADJ_TX + 1) * ADJ_TY, ADJ_YF = ADJ_TX * (ADJ_TY + 1);
+constexpr int ADJ_THREADS = (ADJ_XF + ADJ_YF + 31) / 32 * 32;
+
+// hydro update backwards: I += T (identity paths) + face terms; dt adjoint.  NB: also the
+// adjoint of the cells' n_b (Manning friction of their faces), added to a.nbbar.  Every face
+// of a tile is differentiated once, in reverse, for both of its cells; before, each cell
+// evaluated its four faces on dual numbers with five tangents: 528 us at 512^2, 87 now.
+// Bound by the float64 pipe.
+#ifndef PXB_ADJ_MIN_BLOCKS
+#define PXB_ADJ_MIN_BLOCKS 2
+#endif
 template <bool NB>
-__global__ void __launch_bounds__(256) adj_hydro_kernel(const AdjArgs a) {
-    int r, c;
-    long long i;
-    const bool in = adj_cell(a.ny, a.nx, a.pitch, r, c, i);
+__global__ void __launch_bounds__(ADJ_THREADS, PXB_ADJ_MIN_BLOCKS) adj_hydro_kernel(const __grid_constant__ AdjArgs a) {
+    __shared__ double fx[10][ADJ_XF], fy[10][ADJ_YF];  // adjoints of the first, then of the second cell
+    const int t = threadIdx.x, c0 = blockIdx.x * ADJ_TX, r0 = blockIdx.y * ADJ_TY;
+    const int c1 = min(a.nx, c0 + ADJ_TX), r1 = min(a.ny, r0 + ADJ_TY);
+    const double dt = *a.dt, dx = a.dx, DRY = DRY_TOL;
+    // x-face f of a row lies west of column c0 + f, y-face f of a column north of row r0 + f
+    const bool yf = t >= ADJ_XF;
+    const int k = yf ? t - ADJ_XF : t;
+    const int row = yf ? k / ADJ_TX : k / (ADJ_TX + 1), col = yf ? k - row * ADJ_TX : k - row * (ADJ_TX + 1);
+    const int rj = r0 + row, cj = c0 + col, ri = yf ? rj - 1 : rj, ci = yf ? cj : cj - 1;
+    bool face = t < ADJ_XF + ADJ_YF && (yf ? (cj < c1 && rj <= r1 && ri >= 0 && rj < a.ny)
+                                           : (rj < r1 && cj <= c1 && ci >= 0 && cj < a.nx));
+    const long long i = (long long)ri * a.pitch + ci, j = (long long)rj * a.pitch + cj;
+    if (face) face = ((a.h[i] > DRY) || (a.h[j] > DRY)) && !(adj_nodata(a.nodata, i) || adj_nodata(a.nodata, j));
     double add_dt = 0.0;
-    if (in) {
-        using D = DualN<NB ? 5 : 4>;
-        const double dt = *a.dt, dx = a.dx, DRY = DRY_TOL;
-        const HCell<D> Cd = make_hcell(D::seed(a.h[i], 0), D::seed(a.hu[i], 1), D::seed(a.hv[i], 2),
-                                       D::seed(a.zb[i], 3), D(a.z[i]), NB ? D::seed(a.nb[i], NB ? 4 : 0) : D(a.nb[i]));
-        auto hconst = [&](long long k) {
-            return make_hcell(D(a.h[k]), D(a.hu[k]), D(a.hv[k]), D(a.zb[k]), D(a.z[k]), D(a.nb[k]));
-        };
-        const bool mC = adj_nodata(a.nodata, i);
+    HBar bI{0, 0, 0, 0, 0}, bJ{0, 0, 0, 0, 0};
+    if (face) {
         const double k_ = -dt / dx;
-        double g[NB ? 5 : 4] = {};
-        double f[3] = {0, 0, 0};  // forward fluctuation sum of this cell
-        // face (I|J): M goes to I, P to J
-        auto face = [&](long long k, bool cell_is_I, bool yf) {
-            const bool mk = adj_nodata(a.nodata, k);
-            if (!(((a.h[i] > DRY) || (a.h[k] > DRY)) && !(mC || mk))) return;
-            const HCell<D> Nd = hconst(k);
-            D P[3], M[3];
-            if (yf) {
-                if (cell_is_I) roe_exner_face<D, true>(Cd, Nd, D(dx), P, M);
-                else roe_exner_face<D, true>(Nd, Cd, D(dx), P, M);
-            } else {
-                if (cell_is_I) roe_exner_face<D, false>(Cd, Nd, D(dx), P, M);
-                else roe_exner_face<D, false>(Nd, Cd, D(dx), P, M);
-            }
-            const long long I = cell_is_I ? i : k, J = cell_is_I ? k : i;
-            const double aI[3] = {a.Th[I], a.Thu[I], a.Thv[I]}, aJ[3] = {a.Th[J], a.Thu[J], a.Thv[J]};
-            for (int q = 0; q < (NB ? 5 : 4); ++q)
-                for (int m = 0; m < 3; ++m) g[q] += k_ * (aI[m] * M[m].d[q] + aJ[m] * P[m].d[q]);
-            for (int m = 0; m < 3; ++m) f[m] += cell_is_I ? M[m].v : P[m].v;
-        };
-        if (c + 1 < a.nx) face(i + 1, true, false);
-        if (c >= 1) face(i - 1, false, false);
-        if (r + 1 < a.ny) face(i + a.pitch, true, true);
-        if (r >= 1) face(i - a.pitch, false, true);
-        a.Ih[i] += a.Th[i] + g[0];
-        a.Ihu[i] += a.Thu[i] + g[1];
-        a.Ihv[i] += a.Thv[i] + g[2];
-        a.Izb[i] += a.Tzb[i] + g[3];
-        a.IG[i] += a.TG[i];
-        if constexpr (NB) a.nbbar[i] += g[NB ? 4 : 0];
-        add_dt = -(a.Th[i] * f[0] + a.Thu[i] * f[1] + a.Thv[i] * f[2]) / dx;
+        const double aI[3] = {a.Th[i], a.Thu[i], a.Thv[i]}, aJ[3] = {a.Th[j], a.Thu[j], a.Thv[j]};
+        const double Pb[3] = {k_ * aJ[0], k_ * aJ[1], k_ * aJ[2]}, Mb[3] = {k_ * aI[0], k_ * aI[1], k_ * aI[2]};
+        const HCell<double> I = make_hcell(a.h[i], a.hu[i], a.hv[i], a.zb[i], a.z[i], a.nb[i]);
+        const HCell<double> J = make_hcell(a.h[j], a.hu[j], a.hv[j], a.zb[j], a.z[j], a.nb[j]);
+        double P[3], M[3];
+        if (yf) adj_exner_hydro_face<true>(I, J, dx, Pb, Mb, bI, bJ, P, M);
+        else adj_exner_hydro_face<false>(I, J, dx, Pb, Mb, bI, bJ, P, M);
+        // the tile of the second cell counts the face
+        if (yf ? rj < r1 : cj < c1)
+            add_dt = -((aI[0] * M[0] + aI[1] * M[1] + aI[2] * M[2]) + (aJ[0] * P[0] + aJ[1] * P[1] + aJ[2] * P[2])) / dx;
+    }
+    if (t < ADJ_XF + ADJ_YF) {
+        const double v[10] = {bI.h, bI.u, bI.v, bI.z, bI.nb, bJ.h, bJ.u, bJ.v, bJ.z, bJ.nb};
+#pragma unroll
+        for (int m = 0; m < 10; ++m) (yf ? fy[m][k] : fx[m][k]) = v[m];
     }
     adj_dt_add(a.dtbar, add_dt);
+    __syncthreads();
+    const int tr = t / ADJ_TX, tc = t - tr * ADJ_TX, r = r0 + tr, c = c0 + tc;
+    if (t >= ADJ_TX * ADJ_TY || r >= r1 || c >= c1) return;
+    const int xw = tr * (ADJ_TX + 1) + tc, yn = tr * ADJ_TX + tc;
+    double g[5];
+#pragma unroll
+    for (int m = 0; m < 5; ++m) {  // faces beyond the grid hold zeros
+        g[m] = fx[m][xw + 1] + fx[5 + m][xw];
+        g[m] = g[m] + fy[m][yn + ADJ_TX];
+        g[m] = g[m] + fy[5 + m][yn];
+    }
+    // the clamps, velocities and the bed of make_hcell backwards
+    const long long o = (long long)r * a.pitch + c;
+    const double h = a.h[o], hc = clamp_lo(h, DRY);
+    double gh = g[0], ghu = 0.0, ghv = 0.0;
+    if (hc > DRY) {
+        const DivBy<double> by_h(hc);
+        ghu = by_h(g[1]);
+        ghv = by_h(g[2]);
+        gh -= ghu * by_h(a.hu[o]) + ghv * by_h(a.hv[o]);
+    }
+    if (h < DRY) gh = 0.0;
+    a.Ih[o] += a.Th[o] + gh;
+    a.Ihu[o] += a.Thu[o] + ghu;
+    a.Ihv[o] += a.Thv[o] + ghv;
+    a.Izb[o] += a.Tzb[o] + (a.zb[o] > SED_TOL ? g[3] : 0.0);
+    a.IG[o] += a.TG[o];
+    if constexpr (NB) a.nbbar[o] += g[4];
 }
 
 // ---------------------------------------------------------------- handlers backwards

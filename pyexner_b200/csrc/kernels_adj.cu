@@ -26,8 +26,11 @@ cudaError_t launch_adj_stage(const AdjArgs& a, int phase, cudaStream_t s) {
             break;
         case 2: adj_corr_kernel<<<g, b, 0, s>>>(a); break;
         default:
-            if (a.nbbar) adj_hydro_kernel<true><<<g, b, 0, s>>>(a);
-            else adj_hydro_kernel<false><<<g, b, 0, s>>>(a);
+        {
+            const dim3 t((a.nx + ADJ_TX - 1) / ADJ_TX, (a.ny + ADJ_TY - 1) / ADJ_TY);
+            if (a.nbbar) adj_hydro_kernel<true><<<t, ADJ_THREADS, 0, s>>>(a);
+            else adj_hydro_kernel<false><<<t, ADJ_THREADS, 0, s>>>(a);
+        }
             break;
     }
     return cudaGetLastError();
