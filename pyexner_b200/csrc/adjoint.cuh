@@ -22,6 +22,7 @@
 #include "init_bc.cuh"
 #include "adjoint_args.cuh"
 #include "dualn.cuh"
+#include "re_cfl.cuh"  // cfl_bound
 
 namespace pxb {
 
@@ -36,10 +37,29 @@ __device__ __forceinline__ bool adj_cell(int ny, int nx, long long pitch, int& r
 
 __device__ __forceinline__ bool adj_nodata(const uint8_t* m, long long i) { return m ? m[i] != 0 : false; }
 
-// warp sum then one atomic per warp (every lane of the warp calls this)
+// Sum over the block of each of N values, one atomic per value and block: atomics of all
+// warps of a 512^2 grid on one address took about 60 us.  Every thread of a block of up to
+// 1024 calls it once.
+template <int N>
+__device__ __forceinline__ void adj_sum_add(double* dst, const double (&v)[N]) {
+    __shared__ double part[N][32];
+    const int tid = threadIdx.x + blockDim.x * threadIdx.y, warp = tid >> 5, nw = (blockDim.x * blockDim.y) >> 5;
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+        double x = v[q];
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(FULL, x, o);
+        if ((tid & 31) == 0) part[q][warp] = x;
+    }
+    __syncthreads();
+    if (tid < N) {
+        double x = 0.0;
+        for (int w = 0; w < nw; ++w) x += part[tid][w];
+        if (x != 0.0) atomicAdd(dst + tid, x);
+    }
+}
 __device__ __forceinline__ void adj_dt_add(double* dst, double v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
-    if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(dst, v);
+    const double x[1] = {v};
+    adj_sum_add<1>(dst, x);
 }
 
 // SSPRK2 average / plain store: S = scale * out_adj; with `avg`, avg_adj = 0.5 * out_adj.
@@ -112,17 +132,6 @@ __global__ void __launch_bounds__(256) adj_exner_kernel(const AdjArgs a) {
         add_dt = a.Szb[i] * (-acc / dx);
     }
     adj_dt_add(a.dtbar, add_dt);
-}
-
-// warp sum of each of N values, one atomic per value and warp (every lane calls this)
-template <int N>
-__device__ __forceinline__ void adj_sum_add(double* dst, const double (&v)[N]) {
-#pragma unroll
-    for (int q = 0; q < N; ++q) {
-        double x = v[q];
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(FULL, x, o);
-        if ((threadIdx.x & 31) == 0 && x != 0.0) atomicAdd(dst + q, x);
-    }
 }
 
 // Derivatives of the Meyer-Peter & Mueller grass factor of one cell (roe_exner.py:85-130):
@@ -536,34 +545,32 @@ __device__ __forceinline__ bool adj_face_speed(const AdjCflArgs& a, int r, int c
     return true;
 }
 
-// pass 1: maximum speed (bits); pass 2: number of faces at it
-__global__ void __launch_bounds__(256) adj_cfl_max_kernel(const AdjCflArgs a, int pass) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    const int r = blockIdx.y * blockDim.y + threadIdx.y;
-    unsigned long long best = 0ull;
-    unsigned int ties = 0;
-    if (r < a.ny && c < a.nx) {
-        for (int yf = 0; yf < 2; ++yf) {
-            double s;
-            if (adj_face_speed(a, r, c, yf != 0, s)) {
-                const unsigned long long b = speed_bits(s);
-                if (pass == 0) best = b > best ? b : best;
-                else ties += (b == *a.maxbits) ? 1u : 0u;
-            }
-        }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long ob = __shfl_xor_sync(FULL, best, o);
-        best = ob > best ? ob : best;
-        ties += __shfl_xor_sync(FULL, ties, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        if (pass == 0 && best != 0ull) atomicMax(a.maxbits, best);
-        if (pass == 1 && ties) atomicAdd(a.nties, ties);
-    }
+// Whether a face's speed is the maximum: its bound from the two cells rules most faces out
+// (cfl_bound) before the speed itself is formed.
+__device__ __forceinline__ bool adj_at_max(const AdjCflArgs& a, int r, int c, bool yf, unsigned long long m, float smax) {
+    if (yf ? (r + 1 >= a.ny) : (c + 1 >= a.nx)) return false;
+    const long long i = (long long)r * a.pitch + c, j = yf ? i + a.pitch : i + 1;
+    const float hi = clamp_lo((float)a.h[i], (float)DRY_TOL), hj = clamp_lo((float)a.h[j], (float)DRY_TOL);
+    const float ui = fmax_nan(fabsf((float)a.hu[i]), fabsf((float)a.hv[i])) * f_rcp(hi);
+    const float uj = fmax_nan(fabsf((float)a.hu[j]), fabsf((float)a.hv[j])) * f_rcp(hj);
+    const float b = cfl_bound(fmax_nan(ui, uj), fmax_nan(hi, hj), fminf(hi, hj), fmax_nan(fabsf((float)a.G[i]), fabsf((float)a.G[j])));
+    double s;
+    return !(b < smax) && adj_face_speed(a, r, c, yf, s) && speed_bits(s) == m;
 }
 
-// pass 3: d(dt)/d(s_max) spread over the tying faces, through their speeds' local Jacobians
+// pass 1: number of faces at the maximum speed
+__global__ void __launch_bounds__(256) adj_cfl_ties_kernel(const AdjCflArgs a) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    const int r = blockIdx.y * blockDim.y + threadIdx.y;
+    if (r >= a.ny || c >= a.nx) return;
+    const unsigned long long m = *a.maxbits;
+    const float smax = (float)bits_speed(m, 0.0);
+    unsigned int ties = 0;
+    for (int yf = 0; yf < 2; ++yf) ties += adj_at_max(a, r, c, yf != 0, m, smax) ? 1u : 0u;
+    if (ties) atomicAdd(a.nties, ties);
+}
+
+// pass 2: d(dt)/d(s_max) spread over the tying faces, through their speeds' local Jacobians
 __global__ void __launch_bounds__(256) adj_cfl_grad_kernel(const AdjCflArgs a) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     const int r = blockIdx.y * blockDim.y + threadIdx.y;
@@ -574,8 +581,7 @@ __global__ void __launch_bounds__(256) adj_cfl_grad_kernel(const AdjCflArgs a) {
     if (!(dt >= a.floor_dt) || *a.nties == 0u) return;  // the floor (or no face): dt does not depend on the state
     const double sbar = *a.dtbar * (-a.cfl * a.dx / (smax * smax)) / (double)*a.nties;
     for (int yf = 0; yf < 2; ++yf) {
-        double s;
-        if (!adj_face_speed(a, r, c, yf != 0, s) || speed_bits(s) != m) continue;
+        if (!adj_at_max(a, r, c, yf != 0, m, (float)smax)) continue;
         using D = DualN<8>;
         const long long i = (long long)r * a.pitch + c, j = yf ? i + a.pitch : i + 1;
         const CCell<D> I = make_ccell(D::seed(a.h[i], 0), D::seed(a.hu[i], 1), D::seed(a.hv[i], 2), D::seed(a.G[i], 3));

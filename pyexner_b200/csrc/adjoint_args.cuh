@@ -50,7 +50,7 @@ struct AdjCflArgs {
     const double *h, *hu, *hv, *G;
     const uint8_t* nodata;
     double dx, cfl, floor_dt;
-    unsigned long long* maxbits;
+    const unsigned long long* maxbits;  // the step's largest face speed (bits)
     unsigned int* nties;
     const double* dtbar;
     double *Ah, *Ahu, *Ahv, *AG;  // adjoint of the step input (accumulated)

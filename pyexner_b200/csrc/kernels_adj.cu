@@ -54,8 +54,7 @@ cudaError_t launch_adj_bc(const AdjBcSet& a, cudaStream_t s) {
 
 cudaError_t launch_adj_cfl(const AdjCflArgs& a, cudaStream_t s) {
     const dim3 g = adj_grid(a.ny, a.nx), b(32, 8);
-    adj_cfl_max_kernel<<<g, b, 0, s>>>(a, 0);
-    adj_cfl_max_kernel<<<g, b, 0, s>>>(a, 1);
+    adj_cfl_ties_kernel<<<g, b, 0, s>>>(a);
     adj_cfl_grad_kernel<<<g, b, 0, s>>>(a);
     return cudaGetLastError();
 }

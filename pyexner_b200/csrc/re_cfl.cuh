@@ -34,6 +34,7 @@ namespace pxb {
 
 struct CflScratch {
     unsigned long long maxbits;  // running max of speed bits
+    unsigned long long last;     // the largest speed of the last completed reduction (bits)
     unsigned int done;           // finished blocks of the current launch
     unsigned int step;           // index into the dt log
     int err;                     // sticky error word
@@ -445,6 +446,7 @@ __global__ void __launch_bounds__(256, cfl_min_blocks(sizeof(T))) re_cfl_kernel(
         a.scr->t_step = a.scr->t_next;
         a.scr->t_next = a.scr->t_next + (double)dt;
         if (!d_isfinite(dt)) a.scr->err |= 2;
+        a.scr->last = bits;
         a.scr->maxbits = 0ull;
         a.scr->done = 0u;
         __threadfence();
