@@ -436,24 +436,20 @@ __global__ void __launch_bounds__(ADJ_THREADS, PXB_ADJ_MIN_BLOCKS) adj_hydro_ker
 
 // ---------------------------------------------------------------- handlers backwards
 
-// The adjoint of one boundary cell's fields that the handler writes, saved and cleared (they
-// were overwritten).
-__device__ __forceinline__ void adj_bc_take(const AdjBcSet& a, const AdjBcHandler& h, const int k) {
+// The adjoint of a boundary cell's fields that the handler writes, taken and cleared (they
+// were overwritten); read past the L1, behind the atomics of the handler before.
+__device__ __forceinline__ void adj_bc_take(const AdjBcSet& a, const AdjBcHandler& h, const long long b, double (&t)[6]) {
     const unsigned fm = bc_field_mask(h.kind);
-    const long long b = h.cells[k];
 #pragma unroll
     for (int s = 0; s < 6; ++s) {
         const bool w = ((fm >> s) & 1u) && a.f[s];
-        a.tmp[s * h.count + k] = w ? __ldcg(a.f[s] + b) : 0.0;  // (past the L1: atomics of the handler before)
+        t[s] = w ? __ldcg(a.f[s] + b) : 0.0;
         if (w) a.f[s][b] = 0.0;
     }
 }
 
-// The donor receives the transposed Jacobian of the handler times the saved adjoints.
-__device__ __forceinline__ void adj_bc_give(const AdjBcSet& a, const AdjBcHandler& h, const int k) {
-    const long long d = h.donors[k];
-    const double* t = a.tmp;
-    const int n = h.count;
+// The donor receives the transposed Jacobian of the handler times the adjoints taken.
+__device__ __forceinline__ void adj_bc_give(const AdjBcSet& a, const AdjBcHandler& h, const long long d, const double (&t)[6]) {
     auto add = [&](int s, double v) {
         if (a.f[s] && v != 0.0) atomicAdd(a.f[s] + d, v);
     };
@@ -462,35 +458,35 @@ __device__ __forceinline__ void adj_bc_give(const AdjBcSet& a, const AdjBcHandle
             const double nx = h.nx, ny = h.ny;
             // forward: mom_n = hu nx + hv ny, mom_t = -hu ny + hv nx, hu' = -mom_n nx - mom_t ny,
             // hv' = -mom_n ny + mom_t nx
-            const double bu = t[1 * n + k], bv = t[2 * n + k];
+            const double bu = t[1], bv = t[2];
             const double bmn = -bu * nx - bv * ny, bmt = -bu * ny + bv * nx;
-            add(0, t[0 * n + k]);
+            add(0, t[0]);
             add(1, bmn * nx - bmt * ny);
             add(2, bmn * ny + bmt * nx);
-            add(3, t[3 * n + k]);
-            add(5, t[5 * n + k]);
+            add(3, t[3]);
+            add(5, t[5]);
             break;
         }
         case PXB_BC_RE_TRANSMISSIVE:
-            add(0, t[0 * n + k]);
-            add(1, t[1 * n + k]);
-            add(2, t[2 * n + k]);
+            add(0, t[0]);
+            add(1, t[1]);
+            add(2, t[2]);
             break;
         case PXB_BC_RE_TRANSMISSIVEBED:
         case PXB_BC_RE_STEEPFALL:
-            add(3, t[3 * n + k]);
+            add(3, t[3]);
             break;
         case PXB_BC_RE_NORMALFLOWDEPTH:  // hu, hv copied; h and z_b prescribed
-            add(1, t[1 * n + k]);
-            add(2, t[2 * n + k]);
+            add(1, t[1]);
+            add(2, t[2]);
             break;
         case PXB_BC_RE_ZEROMOMENTUM:  // NaN values keep the cell's own momentum (its donor)
-            if (h.c0 != h.c0) add(1, t[1 * n + k]);
-            if (h.c1 != h.c1) add(2, t[2 * n + k]);
+            if (h.c0 != h.c0) add(1, t[1]);
+            if (h.c1 != h.c1) add(2, t[2]);
             break;
         case PXB_BC_RE_CONSTANTINFLUX:  // prescribed hu = q values[1], hv = q values[2]: the adjoint of q
             if (h.qbar) {
-                const double v = t[1 * n + k] * h.vx + t[2 * n + k] * h.vy;
+                const double v = t[1] * h.vx + t[2] * h.vy;
                 if (v != 0.0) atomicAdd(h.qbar, v);
             }
             break;
@@ -500,15 +496,51 @@ __device__ __forceinline__ void adj_bc_give(const AdjBcSet& a, const AdjBcHandle
 }
 
 // Handlers backwards, the last one first, by one block (three launches per handler took 2 us
-// each).  Atomics of one handler are complete, as seen by the block, before the next takes.
+// each).  A thread keeps what it takes of its first ADJ_BC_KEEP cells of a handler in
+// registers, of more cells in the temporary; the next handler's first indices are read ahead.
+constexpr int ADJ_BC_KEEP = 2;
 __global__ void __launch_bounds__(1024) adj_bc_set_kernel(const __grid_constant__ AdjBcSet a) {
+    const int nt = blockDim.x;
+    long long cell[ADJ_BC_KEEP], donor[ADJ_BC_KEEP];
+    auto ahead = [&](int q) {
+#pragma unroll
+        for (int u = 0; u < ADJ_BC_KEEP; ++u) {
+            const int k = threadIdx.x + u * nt;
+            cell[u] = donor[u] = 0;
+            if (k < a.h[q].count) cell[u] = a.h[q].cells[k], donor[u] = a.h[q].donors[k];
+        }
+    };
+    ahead(a.n - 1);
     for (int q = a.n - 1; q >= 0; --q) {
         const AdjBcHandler& h = a.h[q];
-        for (int k = threadIdx.x; k < h.count; k += blockDim.x) adj_bc_take(a, h, k);
-        __syncthreads();
-        for (int k = threadIdx.x; k < h.count; k += blockDim.x) adj_bc_give(a, h, k);
-        __threadfence();
-        __syncthreads();
+        double t[ADJ_BC_KEEP][6];
+        long long d[ADJ_BC_KEEP];
+#pragma unroll
+        for (int u = 0; u < ADJ_BC_KEEP; ++u) {
+            d[u] = donor[u];
+            if ((int)threadIdx.x + u * nt < h.count) adj_bc_take(a, h, cell[u], t[u]);
+        }
+        for (int k = threadIdx.x + ADJ_BC_KEEP * nt; k < h.count; k += nt) {
+            double x[6];
+            adj_bc_take(a, h, h.cells[k], x);
+#pragma unroll
+            for (int s = 0; s < 6; ++s) a.tmp[s * h.count + k] = x[s];
+        }
+        if (q > 0) ahead(q - 1);
+        __syncthreads();  // every clear before any addition
+#pragma unroll
+        for (int u = 0; u < ADJ_BC_KEEP; ++u)
+            if ((int)threadIdx.x + u * nt < h.count) adj_bc_give(a, h, d[u], t[u]);
+        for (int k = threadIdx.x + ADJ_BC_KEEP * nt; k < h.count; k += nt) {
+            double x[6];
+#pragma unroll
+            for (int s = 0; s < 6; ++s) x[s] = a.tmp[s * h.count + k];
+            adj_bc_give(a, h, h.donors[k], x);
+        }
+        if (q > 0) {
+            __threadfence();
+            __syncthreads();
+        }
     }
 }
 

@@ -435,8 +435,8 @@ int arena_copy(DevArena* A, void* dst, const void* src, size_t bytes) {
     return PXB_OK;
 }
 
-// Boundary cells up to which one block applies all handlers: it takes about 0.6 us per level
-// and 1024 cells, two launches per handler 4.6 us and no less.
+// Boundary cells up to which a layout's handlers may be applied in one launch (each of its
+// levels must also fit: pxb::BC_SET_CHUNKS).
 constexpr int BC_SET_CELLS = 16384;
 
 // `total`: boundary cells of all handlers.
@@ -949,7 +949,12 @@ int apply_handlers(const std::vector<DevHandler>& hs, void* bc_tmp, T* const f[6
     for (auto& h : hs) F.total += h.count;
     pxb::BcSet<T> set{};
     set.f = F;
-    const bool together = F.total <= BC_SET_CELLS;
+    bool together = F.total <= BC_SET_CELLS;
+    int chunks = 0;
+    for (auto& h : hs) {
+        chunks = (h.level ? 0 : chunks) + (h.count + 31) / 32;
+        together = together && chunks <= pxb::BC_SET_CHUNKS;
+    }
     int off = 0;
     for (auto& h : hs) {
         pxb::BcHandler<T> b{};

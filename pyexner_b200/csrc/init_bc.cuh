@@ -8,6 +8,8 @@
 // handler, later handlers overwrite earlier ones).  It serves the set-up and the general
 // stage path; the fused stage kernel uses the ring recipes resolved from the same handlers.
 #pragma once
+#include <cooperative_groups.h>
+
 #include "pxb_device.cuh"
 
 namespace pxb {
@@ -64,7 +66,7 @@ struct BcFields {
     T* f[6];
     const double* tptr;   // simulation time on the device, or null: use tval
     double tval;
-    T* tmp;               // 6 * total values
+    T* tmp;               // 6 * total values (handlers in two launches)
     int total;            // boundary cells of all handlers
 };
 
@@ -74,8 +76,10 @@ struct BcArgs {  // one handler
     BcHandler<T> h;
 };
 
-// Handlers one block applies in one launch.
-constexpr int BC_SET_MAX = 16;
+// Handlers one launch applies, threads of a block and blocks of its cluster: a level has at
+// most as many warps' worth of boundary cells (chunks of 32 of a handler).
+constexpr int BC_SET_MAX = 16, BC_SET_THREADS = 512, BC_SET_BLOCKS = 8;
+constexpr int BC_SET_CHUNKS = BC_SET_THREADS / 32 * BC_SET_BLOCKS;
 template <class T>
 struct BcSet {
     BcFields<T> f;
@@ -109,73 +113,84 @@ __device__ __forceinline__ float berthon_zb(float neg_alpha, float zb0, double t
     return __fadd_rn(__fmul_rn(neg_alpha, __double2float_rn(t)), zb0);
 }
 
-// Values of boundary cell k of a handler, gathered from its donor into the temporary.
+// A value past the L1 (another SM may have written it in this launch).
 template <class T>
-__device__ __forceinline__ void bc_gather(const BcFields<T>& F, const BcHandler<T>& h, const int k) {
-    const long long d = h.donors[k];
-    auto ld = [&](int slot) { return F.f[slot] ? F.f[slot][d] : T(0); };  // null slots read as 0
-    T* t = F.tmp + h.off;
-    const int n = F.total;
+__device__ __forceinline__ T bc_load(const T* p) {
+    if constexpr (sizeof(T) == 16) {  // a dual number
+        const double2 t = __ldcg(reinterpret_cast<const double2*>(p));
+        T x;
+        x.v = t.x;
+        x.d = t.y;
+        return x;
+    } else {
+        return __ldcg(p);
+    }
+}
+
+// Values t[slot] of a boundary cell of a handler from its donor d.
+template <class T>
+__device__ __forceinline__ void bc_values(const BcFields<T>& F, const BcHandler<T>& h, const long long d, T (&t)[6]) {
+    auto ld = [&](int slot) { return F.f[slot] ? bc_load(F.f[slot] + d) : T(0); };  // null slots read as 0
     switch (h.kind) {
         case PXB_BC_RE_REFLECTIVE: {  // roeexner_reflective.py:17-63
             const T hu = ld(1), hv = ld(2);
             const T mom_n = hu * h.nx + hv * h.ny;
             const T mom_t = -hu * h.ny + hv * h.nx;
             const T mom_r = -mom_n;
-            t[(size_t)0 * n + k] = ld(0);
-            t[(size_t)1 * n + k] = mom_r * h.nx - mom_t * h.ny;
-            t[(size_t)2 * n + k] = mom_r * h.ny + mom_t * h.nx;
-            t[(size_t)3 * n + k] = ld(3);
-            t[(size_t)4 * n + k] = ld(4);
-            t[(size_t)5 * n + k] = ld(5);
+            t[0] = ld(0);
+            t[1] = mom_r * h.nx - mom_t * h.ny;
+            t[2] = mom_r * h.ny + mom_t * h.nx;
+            t[3] = ld(3);
+            t[4] = ld(4);
+            t[5] = ld(5);
             break;
         }
         case PXB_BC_RE_TRANSMISSIVE:  // roeexner_transmissive.py:17-31
-            t[(size_t)0 * n + k] = ld(0);
-            t[(size_t)1 * n + k] = ld(1);
-            t[(size_t)2 * n + k] = ld(2);
+            t[0] = ld(0);
+            t[1] = ld(1);
+            t[2] = ld(2);
             break;
         case PXB_BC_RE_TRANSMISSIVEBED:  // roeexner_transmissivebed.py:17-27
-            t[(size_t)3 * n + k] = ld(3);
+            t[3] = ld(3);
             break;
         case PXB_BC_RE_CONSTANTINFLUX:  // roeexner_constantinflux.py:18-48
-            t[(size_t)1 * n + k] = h.c0;
-            t[(size_t)2 * n + k] = h.c1;
+            t[1] = h.c0;
+            t[2] = h.c1;
             break;
         case PXB_BC_ROE_REFLECTIVE:  // roe_reflective.py:18-44
-            t[(size_t)0 * n + k] = ld(0);
-            t[(size_t)3 * n + k] = ld(3);
-            t[(size_t)4 * n + k] = ld(4);
-            t[(size_t)1 * n + k] = ld(1) * (T(1) - T(2) * h.nx * h.nx);
-            t[(size_t)2 * n + k] = ld(2) * (T(1) - T(2) * h.ny * h.ny);
+            t[0] = ld(0);
+            t[3] = ld(3);
+            t[4] = ld(4);
+            t[1] = ld(1) * (T(1) - T(2) * h.nx * h.nx);
+            t[2] = ld(2) * (T(1) - T(2) * h.ny * h.ny);
             break;
         case PXB_BC_ROE_TRANSMISSIVE:  // roe_transmissive.py:17-43
-            t[(size_t)0 * n + k] = ld(0);
-            t[(size_t)1 * n + k] = ld(1);
-            t[(size_t)2 * n + k] = ld(2);
-            t[(size_t)3 * n + k] = ld(3);
-            t[(size_t)4 * n + k] = ld(4);
+            t[0] = ld(0);
+            t[1] = ld(1);
+            t[2] = ld(2);
+            t[3] = ld(3);
+            t[4] = ld(4);
             break;
         case PXB_BC_RE_CONSTANTOUTFLUX:  // roeexner_constantoutflux.py:18-73
-            t[(size_t)0 * n + k] = outflux_depth(ld(0), ld(1), ld(2), h.q, h.vx, h.vy);
-            t[(size_t)1 * n + k] = h.c0;
-            t[(size_t)2 * n + k] = h.c1;
+            t[0] = outflux_depth(ld(0), ld(1), ld(2), h.q, h.vx, h.vy);
+            t[1] = h.c0;
+            t[2] = h.c1;
             break;
         case PXB_BC_RE_BERTHON:  // roeexner_berthon.py:19-56
-            t[(size_t)3 * n + k] = T(berthon_zb(h.neg_alpha, h.zb0, F.tptr ? *F.tptr : F.tval));
+            t[3] = T(berthon_zb(h.neg_alpha, h.zb0, F.tptr ? *F.tptr : F.tval));
             break;
         case PXB_BC_RE_NORMALFLOWDEPTH:  // roeexner_normalflowdepth.py:19-51
-            t[(size_t)0 * n + k] = h.hb;
-            t[(size_t)1 * n + k] = ld(1);
-            t[(size_t)2 * n + k] = ld(2);
-            t[(size_t)3 * n + k] = T(berthon_zb(h.neg_alpha, h.zb0, F.tptr ? *F.tptr : F.tval));
+            t[0] = h.hb;
+            t[1] = ld(1);
+            t[2] = ld(2);
+            t[3] = T(berthon_zb(h.neg_alpha, h.zb0, F.tptr ? *F.tptr : F.tval));
             break;
         case PXB_BC_RE_STEEPFALL:  // roeexner_steepfall.py:17-26
-            t[(size_t)3 * n + k] = ld(3) - T(1);
+            t[3] = ld(3) - T(1);
             break;
         case PXB_BC_RE_ZEROMOMENTUM:  // roeexner_zeromomentum.py:16-31; the donor is the cell
-            t[(size_t)1 * n + k] = (h.c0 != h.c0) ? ld(1) : h.c0;
-            t[(size_t)2 * n + k] = (h.c1 != h.c1) ? ld(2) : h.c1;
+            t[1] = (h.c0 != h.c0) ? ld(1) : h.c0;
+            t[2] = (h.c1 != h.c1) ? ld(2) : h.c1;
             break;
         default:
             break;
@@ -210,61 +225,92 @@ __host__ __device__ inline unsigned bc_read_mask(int kind) {
 }
 
 template <class T>
-__device__ __forceinline__ void bc_scatter(const BcFields<T>& F, const BcHandler<T>& h, const int k) {
-    const long long b = h.cells[k];
+__device__ __forceinline__ void bc_store(const BcFields<T>& F, const BcHandler<T>& h, const long long b, const T (&t)[6]) {
     const unsigned fm = bc_field_mask(h.kind);
 #pragma unroll
     for (int s = 0; s < 6; ++s)
-        if (((fm >> s) & 1u) && F.f[s]) F.f[s][b] = F.tmp[(size_t)s * F.total + h.off + k];
+        if (((fm >> s) & 1u) && F.f[s]) F.f[s][b] = t[s];
 }
 
+// One handler in two launches (layouts above BC_SET_CELLS): gather into the temporary,
+// scatter into the cells.
 template <class T>
 __global__ void bc_gather_kernel(const BcArgs<T> a) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < a.h.count) bc_gather(a.f, a.h, k);
+    if (k >= a.h.count) return;
+    T t[6] = {};
+    bc_values(a.f, a.h, a.h.donors[k], t);
+#pragma unroll
+    for (int s = 0; s < 6; ++s) a.f.tmp[(size_t)s * a.f.total + a.h.off + k] = t[s];
 }
 
 template <class T>
 __global__ void bc_scatter_kernel(const BcArgs<T> a) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < a.h.count) bc_scatter(a.f, a.h, k);
+    if (k >= a.h.count) return;
+    T t[6];
+#pragma unroll
+    for (int s = 0; s < 6; ++s) t[s] = a.f.tmp[(size_t)s * a.f.total + a.h.off + k];
+    bc_store(a.f, a.h, a.h.cells[k], t);
 }
 
-// All handlers by one block.  Handlers that read nothing the ones before them write form a
-// level: all of a level's values are gathered before any is scattered, and within the level
-// a later handler's values are scattered after those it overwrites (a barrier only where
-// two write the same value).  The same results as one handler after the other.  A warp
-// takes 32 cells of any handler of the level, so that their loads overlap.  Two launches per
-// handler took 4.6 us: 37 us for 8 handlers of 2500 cells, 17 us here (a chain of index,
-// value, store and barrier latencies per level); 23 -> 7 us for 5 handlers of 180 cells.
+// All handlers by one cluster of blocks, one boundary cell of a level per thread.  Handlers
+// that read nothing the ones before them write form a level: all of a level's values are
+// read before any is written, and within the level a later handler's values are written
+// after those they overwrite (a barrier only where two write the same value).  The same
+// results as one handler after the other.  A warp takes 32 cells of one handler; the next
+// level's indices are read before the barriers of this one.  Bound by the chain of value,
+// barrier and store latencies of each level.  Two launches per handler took 4.6 us, 37 us
+// for 8 handlers of 2500 cells; one block with the values in global scratch 17.3 us, this 6.9
+// (dual numbers 15.3 and 8.0).
 template <class T>
-__global__ void __launch_bounds__(1024) bc_set_kernel(const __grid_constant__ BcSet<T> a) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    // calls f(handler, cell) over the cells of handlers h0 .. h1-1, 32 of one handler per warp
-    auto cells = [&](int h0, int h1, auto f) {
-        int first = 0;  // warp chunks of the handlers before
+__global__ void __launch_bounds__(BC_SET_THREADS) bc_set_kernel(const __grid_constant__ BcSet<T> a) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int lane = threadIdx.x & 31;
+    const int warp = (int)cluster.block_rank() * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    // this thread's handler (-1: none), cell and donor among the handlers h0 .. h1-1
+    struct Item { int q; long long cell, donor; };
+    auto locate = [&](int h0, int h1) {
+        Item it{-1, 0, 0};
+        int chunk = warp;
         for (int q = h0; q < h1; ++q) {
             const int chunks = (a.h[q].count + 31) >> 5;
-            for (int ch = (warp - first % nw + nw) % nw; ch < chunks; ch += nw) {
-                const int k = 32 * ch + lane;
-                if (k < a.h[q].count) f(a.h[q], k);
+            if (chunk < chunks) {
+                const int k = 32 * chunk + lane;
+                if (k < a.h[q].count) it = Item{q, a.h[q].cells[k], a.h[q].donors[k]};
+                break;
             }
-            first += chunks;
+            chunk -= chunks;
         }
+        return it;
     };
-    for (int h0 = 0; h0 < a.n;) {
+    auto level_end = [&](int h0) {
         int h1 = h0 + 1;
         while (h1 < a.n && !a.h[h1].level) ++h1;
-        cells(h0, h1, [&](const BcHandler<T>& h, int k) { bc_gather(a.f, h, k); });
-        __syncthreads();
+        return h1;
+    };
+    int h0 = 0, h1 = level_end(0);
+    Item it = locate(h0, h1);
+    while (h0 < a.n) {
+        T t[6] = {};
+        if (it.q >= 0) bc_values(a.f, a.h[it.q], it.donor, t);
+        const int n1 = h1 < a.n ? level_end(h1) : h1;
+        const Item next = h1 < a.n ? locate(h1, n1) : Item{-1, 0, 0};
+        cluster.sync();
         for (int q = h0; q < h1;) {
             int e = q + 1;
             while (e < h1 && !a.h[e].barrier) ++e;
-            cells(q, e, [&](const BcHandler<T>& h, int k) { bc_scatter(a.f, h, k); });
-            __syncthreads();
+            if (it.q >= q && it.q < e) bc_store(a.f, a.h[it.q], it.cell, t);
             q = e;
+            if (q < h1 || h1 < a.n) {  // (nothing follows the last handlers' stores)
+                __threadfence();
+                cluster.sync();
+            }
         }
+        it = next;
         h0 = h1;
+        h1 = n1;
     }
 }
 

@@ -86,14 +86,27 @@ cudaError_t launch_bc(const BcArgs<T>& a, cudaStream_t s) {
 template <class T>
 cudaError_t launch_bc_set(const BcSet<T>& a, cudaStream_t s) {
     if (a.n <= 0) return cudaSuccess;
-    // a warp for every 32 cells of the largest level, up to the block's 32
-    int most = 0, level = 0;
+    // a warp for every 32 cells of a handler of the largest level (at most BC_SET_CHUNKS: the
+    // host splits larger layouts), in the fewest blocks
+    int most = 1, level = 0;
     for (int k = 0; k < a.n; ++k) {
         level = (a.h[k].level ? 0 : level) + (a.h[k].count + 31) / 32;
         most = std::max(most, level);
     }
-    bc_set_kernel<T><<<1, 32 * std::max(1, std::min(32, most)), 0, s>>>(a);
-    return cudaGetLastError();
+    int blocks = 1;
+    while (most > blocks * (BC_SET_THREADS / 32)) blocks *= 2;
+    if (blocks > BC_SET_BLOCKS) return cudaErrorInvalidConfiguration;
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = blocks;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(32 * ((most + blocks - 1) / blocks));
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, bc_set_kernel<T>, a);
 }
 
 template <class T>
