@@ -139,7 +139,7 @@ typedef struct pxb_re_config {
     const uint8_t* nodata;
     const pxb_bc_handler* handlers; /* in YAML order; resolved into ring recipes at plan creation */
     int32_t nhandlers;
-    int32_t band_rows;              /* rows per warp band of the stage kernel; 0 = automatic   */
+    int32_t band_rows;              /* rows per tile of the stage kernel; 0 = automatic        */
     int32_t stage_path;             /* PXB_PATH_AUTO / _FUSED / _GENERAL                       */
 } pxb_re_config;
 
@@ -333,7 +333,7 @@ typedef struct pxb_re_ens_config {
     int32_t nsed;
     const pxb_re_member* members;    /* host array                                      */
     int32_t nmembers;
-    int32_t band_rows;               /* rows per band for every member; 0 = default     */
+    int32_t band_rows;               /* rows per tile for every member; 0 = default     */
 } pxb_re_ens_config;
 
 typedef struct pxb_re_ens pxb_re_ens;

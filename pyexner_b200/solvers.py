@@ -37,7 +37,7 @@ class SolverConfig(NamedTuple):
     compute_G: object = None  # "MPM" or the constant grass factor
     compute_n: object = None
     plans: dict = None        # plan cache of the config (per dtype / mask)
-    band_rows: int = 0        # rows per warp band of the stage kernel (0 = sized to the device)
+    band_rows: int = 0        # rows per tile of the stage kernel (0 = sized to the device)
     stage_path: int = 0       # _lib.PATH_AUTO / PATH_FUSED / PATH_GENERAL
 
 
