@@ -167,6 +167,8 @@ int pxb_re_init(pxb_re_plan* plan, const pxb_re_fields* f, void* stream);
 
 /* The stage path the plan resolved to: PXB_PATH_FUSED or PXB_PATH_GENERAL. */
 int pxb_re_plan_path(const pxb_re_plan* plan);
+/* Warps side by side in a tile of the plan's fused stage kernel, 0 on the general path. */
+int pxb_re_plan_tile_warps(const pxb_re_plan* plan);
 
 /* Autotuner of the fused stage kernel's band height (no counterpart in the reference):
  * times a set of heights on stage a -> b (plain and SSPRK2-averaged with a; `a` is not

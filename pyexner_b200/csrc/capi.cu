@@ -2343,6 +2343,9 @@ int pxb_re_plan_destroy(pxb_re_plan* plan) {
 }
 
 int pxb_re_plan_path(const pxb_re_plan* plan) { return plan ? plan->path : 0; }
+int pxb_re_plan_tile_warps(const pxb_re_plan* plan) {
+    return plan && plan->path == PXB_PATH_FUSED ? plan->stage.wx : 0;
+}
 
 int pxb_re_autotune(pxb_re_plan* P, const pxb_re_fields* a, const pxb_re_fields* b, void* stream, int32_t* band_rows) {
     if (!P) return fail(PXB_ERR_ARG, "null plan");

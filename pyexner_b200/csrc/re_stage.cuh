@@ -190,9 +190,12 @@ __device__ __forceinline__ void re_stage_tile(const REStageArgs<T>& a, const int
     double budh = 0.0, budz = 0.0;
 
     // ================= phase 1: hydro faces and update of rows H0 .. H1-1
-    // the outermost index columns miss a face unless the grid ends there: they stay zero,
-    // as do the columns beyond the grid
-    const bool whole = INTERIOR ? (lane >= 1 && lane <= 30) : colok && ((lane >= 1 && lane <= 30) || c == 0 || c == nx - 1);
+    // One writer per cell: the column's owner lane, where both of its x-faces lie in the warp.
+    // Neighbouring warps overlap by two columns, so the grid's last column may also be lane 0
+    // of a warp, which lacks its west face.  The outermost index columns miss a face unless the
+    // grid ends there: they stay zero, as do the columns beyond the grid.
+    const bool inner_lane = lane >= 1 && lane <= 30;
+    const bool whole = INTERIOR ? inner_lane : lane_in && colok && (inner_lane || c == 0 || c == nx - 1);
     bool dry = false;
     {
         if (lane_in && !whole)
