@@ -199,11 +199,12 @@ __device__ __forceinline__ void cfl_load4(const T* p, T (&v)[4]) {
 }
 
 // Row r of a lane's four columns.  VEC: 16-byte aligned planes and a pitch of whole groups
-// of four elements.  Columns beyond the grid: still water of no depth, without G.
+// of four elements; a group that reaches beyond the grid is loaded element by element (a
+// plane ends with its last cell).  Columns beyond the grid: still water of no depth, without G.
 template <class T, bool VEC>
 __device__ __forceinline__ void cfl_load(const CflArgs<T>& a, const CflStrip<T>& st, int r, CflRow<T>& x) {
     const long long i = (long long)r * a.pitch + st.c;
-    if (VEC && (st.inner || st.c + 4 <= a.pitch)) {
+    if (VEC && (st.inner || st.c + 4 <= a.nx)) {
         cfl_load4(a.h + i, x.h);
         cfl_load4(a.hu + i, x.hu);
         cfl_load4(a.hv + i, x.hv);
@@ -217,11 +218,6 @@ __device__ __forceinline__ void cfl_load(const CflArgs<T>& a, const CflStrip<T>&
             x.hv[k] = ok ? __ldg(a.hv + i + k) : T(0);
             x.g[k] = ok ? __ldg(a.G + i + k) : T(0);
         }
-    }
-    if (!st.inner) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (st.c + k >= a.nx) x.h[k] = x.hu[k] = x.hv[k] = x.g[k] = T(0);
     }
 }
 
