@@ -1723,6 +1723,16 @@ int copy5(PlanCommon& C, const Planes5& dst, const Planes5& src, cudaStream_t s)
     return PXB_OK;
 }
 
+// The same from or to the caller's planes, which end with their last cell and whose columns
+// beyond nx belong to the caller.
+int copy5_cells(PlanCommon& C, const Planes5& dst, const Planes5& src, cudaStream_t s) {
+    const size_t pitch = sizeof(double) * (size_t)C.pitch;
+    for (int f = 0; f < 5; ++f)
+        PXB_CUDA(cudaMemcpy2DAsync(dst.p[f], pitch, src.p[f], pitch, sizeof(double) * (size_t)C.nx, C.ny,
+                                   cudaMemcpyDeviceToDevice, s));
+    return PXB_OK;
+}
+
 int zero5(PlanCommon& C, const Planes5& q, cudaStream_t s) {
     for (int f = 0; f < 5; ++f) PXB_CUDA(cudaMemsetAsync(q.p[f], 0, sizeof(double) * (size_t)C.ny * C.pitch, s));
     return PXB_OK;
@@ -2017,7 +2027,7 @@ int vjp_run_impl(pxb_re_plan* P, const pxb_re_fields* a0, int nsteps, int scheme
         return st == PXB_OK;
     };
     // forward sweep with checkpoints
-    chk(copy5(P->c, W.ck(0), A0, s));
+    chk(copy5_cells(P->c, W.ck(0), A0, s));
     if (st == PXB_OK && pxb::launch_set_time<double>(P->c.scr, t0, s) != cudaSuccess) st = fail(PXB_ERR_CUDA, "time");
     for (int n = 0; n < nsteps && st == PXB_OK; ++n) {
         const int k = n / W.K;
@@ -2025,7 +2035,7 @@ int vjp_run_impl(pxb_re_plan* P, const pxb_re_fields* a0, int nsteps, int scheme
             if (n > 0) chk(copy5(P->c, W.ck(k), W.seg(0), s));
             if (cudaMemcpyAsync(tck + k, &P->c.scr->t_next, 8, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
                 st = fail(PXB_ERR_CUDA, "checkpoint time");
-            if (n == 0) chk(copy5(P->c, W.seg(0), A0, s));
+            if (n == 0) chk(copy5_cells(P->c, W.seg(0), A0, s));
         }
         if (st == PXB_OK) chk(adj_step_fwd(P, W, W.seg(0), W.seg(0), scheme, a0, cfl, s));
     }
@@ -2037,7 +2047,7 @@ int vjp_run_impl(pxb_re_plan* P, const pxb_re_fields* a0, int nsteps, int scheme
     AB.p[2] = (double*)abar->hv;
     AB.p[3] = (double*)abar->z_b;
     AB.p[4] = (double*)abar->G;
-    if (st == PXB_OK) chk(copy5(P->c, W.aNext, AB, s));
+    if (st == PXB_OK) chk(copy5_cells(P->c, W.aNext, AB, s));
     for (int k = W.nck - 1; k >= 0 && st == PXB_OK; --k) {
         const int n0 = k * W.K, n1 = std::min(nsteps, n0 + W.K);
         chk(copy5(P->c, W.seg(0), W.ck(k), s));
@@ -2114,7 +2124,7 @@ int vjp_run_impl(pxb_re_plan* P, const pxb_re_fields* a0, int nsteps, int scheme
             std::swap(W.aCur, W.aNext);
         }
     }
-    if (st == PXB_OK) chk(copy5(P->c, AB, W.aNext, s));
+    if (st == PXB_OK) chk(copy5_cells(P->c, AB, W.aNext, s));
     if (st == PXB_OK) chk(apply_param_adjoints(P, pdev, pa, s));
     cudaStreamSynchronize(s);
     W.release();

@@ -21,7 +21,7 @@ import torch
 
 from . import _lib
 from .solvers import _re_plan, _roe_plan, _stream
-from .state import RoeExnerState, alloc_plane
+from .state import RoeExnerState, plane_like
 
 TIMESTEP_TOL = 5e-7  # src/utils/constants.py:25
 
@@ -65,10 +65,7 @@ def _config(cfl, end_time, out_freq, solver_bundle, solver_config, n_steps=None)
 
 
 def scratch_like(state):
-    ny, nx = state.shape
-    kw = {}
-    for f in state.PLANES:
-        kw[f] = alloc_plane(ny, nx, state.dtype, state.h.device)
+    kw = {f: plane_like(state.h) for f in state.PLANES}
     if isinstance(state, RoeExnerState):
         kw["seds"] = state.seds
     return type(state)(**kw)

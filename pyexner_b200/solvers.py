@@ -26,7 +26,7 @@ import torch
 
 from . import _lib
 from .boundaries import roe_exner_mask
-from .state import alloc_plane
+from .state import alloc_plane, plane_like
 
 
 class SolverConfig(NamedTuple):
@@ -199,10 +199,9 @@ def step_fn_roeexner(state, time, dt, mask, config, avg=None):
     """roe_exner_solver.py:80-116: one stage; with ``avg`` the SSPRK2 combination
     0.5*avg + 0.5*stage(state) is returned instead."""
     plan = _re_plan(state, mask, config)
-    ny, nx = state.shape
     # the general path carries n through the handlers; the fused path leaves it as it is
     fields = ("h", "hu", "hv", "z_b", "G") + (("n",) if plan.path == _lib.PATH_GENERAL else ())
-    new = {f: alloc_plane(ny, nx, state.dtype, state.h.device) for f in fields}
+    new = {f: plane_like(state.h) for f in fields}
     out = state.replace(**new)
     dtt = _dt_tensor(dt, state)
     _lib.call("pxb_re_stage", plan.handle, ctypes.byref(state.c_fields()), ctypes.byref(out.c_fields()),
@@ -283,7 +282,8 @@ def init_fn_roe(state, mask, config):
 def step_fn_roe(state, time, dt, mask, config, avg=None):
     """roe_solver.py:40-54: update, then the handlers."""
     plan = _roe_plan(state, config)
-    out = state.clone()  # z and n keep their interior values; ring cells are rewritten
+    # z and n keep their interior values; ring cells are rewritten
+    out = state.replace(**{f: plane_like(state.h).copy_(getattr(state, f)) for f in state.PLANES})
     dtt = _dt_tensor(dt, state)
     _lib.call("pxb_roe_stage", plan.handle, ctypes.byref(state.c_fields()), ctypes.byref(out.c_fields()),
               ctypes.byref(avg.c_fields()) if avg is not None else None, ctypes.c_void_p(dtt.data_ptr()), _stream())

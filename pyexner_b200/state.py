@@ -44,6 +44,12 @@ def alloc_plane(ny, nx, dtype, device="cuda", align=32):
     return torch.zeros((ny, pitch), dtype=dtype, device=device)[:, :nx]
 
 
+def plane_like(t):
+    """A zeroed plane of t's shape, type and row pitch (a plan's kernels address every plane
+    they are given with one pitch, the state's)."""
+    return alloc_plane(t.shape[0], t.shape[1], t.dtype, t.device, align=t.stride(0))
+
+
 def plane_from(arr, dtype, device="cuda"):
     arr = np.asarray(arr)
     t = alloc_plane(arr.shape[0], arr.shape[1], dtype, device)

@@ -43,3 +43,75 @@ def test_dt_of_a_window(nx, width, dtype):
     bundle, cfg, mask, st, win, _ = setup(1070, nx, dtype, width)
     assert win.h.stride(0) == width and win.h.storage_offset() == X0
     assert torch.equal(bundle.compute_dt_fn(win, 0.5, mask, cfg), bundle.compute_dt_fn(st, 0.5, mask, cfg))
+
+
+def same(a, b, fields=("h", "hu", "hv", "z_b", "G")):
+    for f in fields:
+        assert torch.equal(getattr(a, f), getattr(b, f)), f
+
+
+def outside_untouched(whole, nx):
+    for f, t in whole.items():
+        assert bool((t[:, :X0] == 7.0).all()) and bool((t[:, X0 + nx:] == 7.0).all()), f
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64], ids=["f32", "f64"])
+@pytest.mark.parametrize("path", ["fused", "general"])
+def test_stage_and_steps_of_a_window(path, dtype):
+    """What the wrapper allocates for a window has the window's pitch: the same bits as the
+    state's own, and nothing outside the window changes."""
+    from pyexner_b200 import run_steps
+
+    nx, width = 70, 200  # (70 columns alone would be padded to 96)
+    bundle, cfg, mask, st, win, whole = setup(41, nx, dtype, width)
+    cfg = cfg._replace(stage_path={"fused": 1, "general": 2}[path], plans={})
+    dt = float(bundle.compute_dt_fn(st, 0.5, mask, cfg))
+    same(bundle.step_fn(win, 0.0, dt, mask, cfg), bundle.step_fn(st, 0.0, dt, mask, cfg))
+    assert torch.equal(run_steps(win, mask, cfg, "FE", 3, 0.5), run_steps(st, mask, cfg, "FE", 3, 0.5))
+    same(win, st)
+    outside_untouched(whole, nx)
+
+
+def test_plain_roe_step_of_a_window():
+    from pyexner_b200 import RoeState
+
+    from bc_specs import ROE_BC_SPECS
+    from pyexner_b200 import BoundaryManager, create_solver_bundle
+
+    ny, nx, width = 41, 70, 200
+    rng = np.random.default_rng(1)
+    h = rng.uniform(0.3, 0.6, (ny, nx))
+    X, Y = grid_coords(ny, nx)
+    params = dict(flux_scheme="Roe", boundaries=ROE_BC_SPECS[sorted(ROE_BC_SPECS)[0]](ny, nx))
+    st = RoeState.from_numpy(dict(h=h, hu=0.2 * h, hv=-0.1 * h, z=0.0 * h, n=0.01 + 0.0 * h), torch.float64)
+    whole = {f: torch.full((ny, width), 7.0, dtype=torch.float64, device="cuda") for f in RoeState.PLANES}
+    win = st.replace(**{f: whole[f][:, X0:X0 + nx].copy_(getattr(st, f)) for f in RoeState.PLANES})
+    bundle = create_solver_bundle("Roe")
+    cfg = bundle.config(st, None, BoundaryManager(params, X, Y), 0.1, params)
+    mask = bundle.mask_fn(st)
+    dt = float(bundle.compute_dt_fn(st, 0.5, mask, cfg))
+    assert float(bundle.compute_dt_fn(win, 0.5, mask, cfg)) == dt
+    same(bundle.step_fn(win, 0.0, dt, mask, cfg), bundle.step_fn(st, 0.0, dt, mask, cfg), RoeState.PLANES)
+    outside_untouched(whole, nx)
+
+
+def test_reverse_mode_of_a_window():
+    """The adjoint comes back in the window's columns alone.  Its atomic sums vary in their last
+    bits: 1e-12 normwise."""
+    from pyexner_b200.tangent import vjp_run
+
+    nx, width = 70, 200
+    _, cfg, mask, st, win, whole = setup(41, nx, torch.float64, width)
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    abar = st.clone()
+    for f in FIELDS:
+        getattr(abar, f).copy_(torch.randn(st.shape, generator=gen, dtype=torch.float64, device="cuda"))
+    bars = {f: torch.full((41, width), 7.0, dtype=torch.float64, device="cuda") for f in FIELDS}
+    wbar = abar.replace(**{f: bars[f][:, X0:X0 + nx].copy_(getattr(abar, f)) for f in FIELDS})
+    vjp_run(st, abar, mask, cfg, 3, "SSPRK2", 0.5, checkpoint_every=2)
+    vjp_run(win, wbar, mask, cfg, 3, "SSPRK2", 0.5, checkpoint_every=2)
+    for f in ("h", "hu", "hv", "z_b", "G"):
+        a, b = getattr(abar, f), getattr(wbar, f)
+        assert float((a - b).abs().max()) <= 1e-12 * float(a.abs().max()), f
+    outside_untouched(whole, nx)
+    outside_untouched(bars, nx)
