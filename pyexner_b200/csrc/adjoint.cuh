@@ -158,7 +158,7 @@ __device__ __forceinline__ void mpm_gradient(double h, double hu, double hv, con
             continue;
         }
         const double rt = sqrt(theta), rd = sqrt(d), den = 1.0 / (theta * rt + 1e-5);
-        const double g1 = c.np3sg / (c.sm1 * sqh), amp = c.frac * g1 * 8.0 / S.one_minus_por;
+        const double g1 = c.np3sg / (c.sm1 * sqh), unit = g1 * 8.0 / S.one_minus_por, amp = c.frac * unit;
         const double G = amp * rd * d * den;
         const double g_d = 1.5 * amp * rd * den;                 // through d
         const double g_t = g_d - 1.5 * G * rt * den;             // through theta
@@ -172,7 +172,7 @@ __device__ __forceinline__ void mpm_gradient(double h, double hu, double hv, con
             par[2] = -g_d;
             par[3] = G / c.np3sg;
             par[4] = -G / c.sm1;
-            par[5] = amp / c.frac * rd * d * den;
+            par[5] = unit * rd * d * den;  // (not by the fraction, which may be 0)
             par[6] = -G / S.one_minus_por;
         }
     }
