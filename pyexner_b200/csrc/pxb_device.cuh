@@ -63,9 +63,11 @@ __host__ __device__ constexpr bool is_f32() { return sizeof(T) == 4; }
 // Markstein's correction (P. Markstein, "Computation of elementary functions on the IBM RISC
 // System/6000 processor", 1990): q = n r, then q + r (n - q d) with fused operations, which
 // is the correctly rounded n / d when r is the correctly rounded 1 / d and nothing over- or
-// underflows, so the results keep the bits of the divisions they replace (compared over
-// 2^30 random pairs).  Three operations instead of a division of about ten with its range
-// checks.  Other types divide.
+// underflows.  Where the remainder is 0 or not a number (exact quotients, zeros with their
+// sign, infinities, a denominator of 0) q itself is the quotient: the correction would turn
+// -0 into 0 and an infinity into a NaN.  Near the ends of the exponent range (a remainder
+// that underflows) the last bit may differ from the division's.  Four operations instead of a
+// division of about ten with its range checks.  Other types divide.
 template <class T>
 struct DivBy {
     T d;
@@ -77,13 +79,14 @@ struct DivBy<double> {
     double d, r;
     __device__ __forceinline__ explicit DivBy(double x) : d(x), r(1.0 / x) {}
     __device__ __forceinline__ double operator()(double n) const {
-        const double q = __dmul_rn(n, r);
-        return __fma_rn(__fma_rn(-q, d, n), r, q);
+        const double q = __dmul_rn(n, r), e = __fma_rn(-q, d, n);
+        return ::fabs(e) > 0.0 ? __fma_rn(e, r, q) : q;
     }
 };
 
-// x^(4/3) and x^(3/2) of x >= 0 from one root each: within 1.5 ulp (cbrt is within 1), where
-// the general power function is within 2 and costs about four times as much.
+// x^(4/3) and x^(3/2) of x >= 0 from one root each: relative errors below 1.5 * 2^-52 (cbrt is
+// within one unit in the last place) and 2^-52, where the general power function is within two
+// units and costs about four times as much.
 template <class T>
 __device__ __forceinline__ T d_pow43(T x) { return x * d_cbrt(x); }
 template <class T>
