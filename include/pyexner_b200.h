@@ -255,7 +255,8 @@ int pxb_re_jvp_run(pxb_re_plan* plan, const pxb_re_fields* a, const pxb_re_field
  * dependence of dt on the state through the fastest face.  pxb_re_vjp_init: `f` is the
  * state BEFORE init; `fbar` (in: adjoint after init, out: before) goes back through the
  * handlers and the grass factor.  Handlers of every kind but ConstantOutflux.  Allocates
- * its checkpoints for the call; synchronises `stream`. */
+ * its checkpoints for the call; synchronises `stream`.  pxb_re_vjp_run_in (declared with the
+ * parameter adjoints below) takes them in a caller-owned workspace instead. */
 int pxb_re_vjp_init(pxb_re_plan* plan, const pxb_re_fields* f, const pxb_re_fields* fbar, void* stream);
 int pxb_re_vjp_run(pxb_re_plan* plan, const pxb_re_fields* a0, int32_t nsteps, int32_t scheme, double cfl, double t0,
                    int32_t checkpoint_every, const pxb_re_fields* abar, void* stream);
@@ -283,6 +284,14 @@ int pxb_re_vjp_init_params(pxb_re_plan* plan, const pxb_re_fields* f, const pxb_
 int pxb_re_vjp_run_params(pxb_re_plan* plan, const pxb_re_fields* a0, int32_t nsteps, int32_t scheme, double cfl,
                           double t0, int32_t checkpoint_every, const pxb_re_fields* abar,
                           const pxb_re_param_adjoints* pbar, void* stream);
+/* pxb_re_vjp_run_params (pbar may be NULL) with its checkpoints and scratch in `workspace`: a
+ * 256-byte aligned device pointer to at least the bytes that pxb_re_vjp_workspace_size gives
+ * for the same step counts, untouched by others until the call returns.  NULL: allocated for
+ * the call. */
+int pxb_re_vjp_workspace_size(const pxb_re_plan* plan, int32_t nsteps, int32_t checkpoint_every, size_t* bytes);
+int pxb_re_vjp_run_in(pxb_re_plan* plan, const pxb_re_fields* a0, int32_t nsteps, int32_t scheme, double cfl,
+                      double t0, int32_t checkpoint_every, const pxb_re_fields* abar,
+                      const pxb_re_param_adjoints* pbar, void* workspace, size_t bytes, void* stream);
 
 /* Device error word of the plan (non-finite dt or state seen by a kernel): reads it
  * (synchronising `stream`), clears it, returns PXB_OK or PXB_ERR_NONFINITE. */

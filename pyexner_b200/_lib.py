@@ -169,6 +169,9 @@ SIGNATURES = {
     "pxb_re_volume": [c_void_p, POINTER(REFields), POINTER(c_double), c_void_p],
     "pxb_re_vjp_run_params": [c_void_p, POINTER(REFields), c_int32, c_int32, c_double, c_double, c_int32,
                               POINTER(REFields), c_void_p, c_void_p],
+    "pxb_re_vjp_workspace_size": [c_void_p, c_int32, c_int32, POINTER(c_size_t)],
+    "pxb_re_vjp_run_in": [c_void_p, POINTER(REFields), c_int32, c_int32, c_double, c_double, c_int32,
+                          POINTER(REFields), c_void_p, c_void_p, c_size_t, c_void_p],
     "pxb_re_vjp_init_params": [c_void_p, POINTER(REFields), POINTER(REFields), c_void_p, c_void_p],
     "pxb_re_set_budget": [c_void_p, c_void_p],
 }

@@ -760,8 +760,6 @@ struct pxb_re_plan {
     pxb::SedTable<double> sedd;
     // volume budget (pxb_re_set_budget / pxb_re_volume): per-item outflow partials of the
     // stage kernel, the caller's accumulator, and the volume reduction's scratch
-    void* adj_buf = nullptr;  // reverse mode: its buffers, kept up to ADJ_KEEP bytes
-    size_t adj_bytes = 0;
     double* bud_part = nullptr;
     long long bud_items = 0;
     pxb::BudgetAcc* bud_acc = nullptr;
@@ -1769,11 +1767,10 @@ int adj_handlers(PlanCommon& C, double* const f[6], double* tmp, cudaStream_t s,
     return PXB_OK;
 }
 
-// Largest reverse-mode buffer a plan keeps between calls.
-constexpr size_t ADJ_KEEP = (size_t)1 << 30;
-
+// Buffers of one reverse-mode run, in one block of bytes() at base: the planes, dt and its
+// adjoint with the step times, the tie count, the handlers' scratch.
 struct AdjWork {
-    double* base = nullptr;  // all planes
+    double* base = nullptr;
     size_t plane = 0;
     int nck = 0, K = 0;
     Planes5 u1, aS, aT, aCur, aNext, aU1;
@@ -1781,8 +1778,9 @@ struct AdjWork {
     double* gscr = nullptr;  // 7 planes for the general stage
     double* dev = nullptr;   // dt, dtbar, times (checkpoints then segment)
     unsigned int* nties = nullptr;
-    bool kept = false;       // base is the plan's
+    bool owned = false;      // base is this call's own allocation (else the caller's workspace)
     double* bctmp = nullptr;
+    size_t nbc = 0;          // values of bctmp
     // parameter adjoints (null: not requested): per handler the ConstantInflux discharge,
     // then the MPM table of the sediment class; the n_b adjoint plane
     double* qbar = nullptr;
@@ -1790,8 +1788,35 @@ struct AdjWork {
     double* nbbar = nullptr;
     Planes5 ck(int k) const { return planes_of(base, plane, k); }                  // checkpoint k
     Planes5 seg(int k) const { return planes_of(base, plane, nck + k); }           // segment state k
+    AdjWork(const pxb_re_plan* P, int nsteps, int every) {
+        K = every > 0 ? every : 32;
+        nck = (int)(((long long)nsteps + K - 1) / K);
+        plane = (size_t)P->c.ny * (size_t)P->c.pitch;
+        int maxcount = 1;
+        for (auto& h : P->c.handlers) maxcount = std::max(maxcount, h.count);
+        nbc = 6 * (size_t)maxcount;
+    }
+    // checkpoints, segment states (K + 1), u1, aS, aT, aCur, aNext, aU1 (5 planes each), h1, 7 scratch
+    size_t nplanes() const { return 5 * ((size_t)nck + K + 1 + 6) + 1 + 7; }
+    size_t nscal() const { return 2 + (size_t)nck + K + 1; }
+    size_t bytes() const { return sizeof(double) * (nplanes() * plane + nscal() + nbc); }
+    void place(double* block) {
+        base = block;
+        dev = base + nplanes() * plane;
+        nties = (unsigned int*)(dev + nscal() - 1);
+        bctmp = dev + nscal();
+        const int o = nck + K + 1;
+        u1 = planes_of(base, plane, o);
+        aS = planes_of(base, plane, o + 1);
+        aT = planes_of(base, plane, o + 2);
+        aCur = planes_of(base, plane, o + 3);
+        aNext = planes_of(base, plane, o + 4);
+        aU1 = planes_of(base, plane, o + 5);
+        h1 = base + (size_t)5 * (o + 6) * plane;
+        gscr = h1 + plane;
+    }
     void release() {
-        if (!kept) cudaFree(base);
+        if (owned) cudaFree(base);
         base = nullptr;
     }
 };
@@ -1953,7 +1978,8 @@ int apply_param_adjoints(pxb_re_plan* P, const double* dev, const pxb_re_param_a
 }
 
 int vjp_run_impl(pxb_re_plan* P, const pxb_re_fields* a0, int nsteps, int scheme, double cfl, double t0, int every,
-                 const pxb_re_fields* abar, const pxb_re_param_adjoints* pa, cudaStream_t s) {
+                 const pxb_re_fields* abar, const pxb_re_param_adjoints* pa, void* workspace, size_t ws_bytes,
+                 cudaStream_t s) {
     for (auto& h : P->c.handlers)
         if (h.kind == PXB_BC_RE_CONSTANTOUTFLUX)
             return fail(PXB_ERR_UNSUPPORTED, "the reverse mode does not cover ConstantOutflux handlers (nonlinear)");
@@ -1961,58 +1987,28 @@ int vjp_run_impl(pxb_re_plan* P, const pxb_re_fields* a0, int nsteps, int scheme
     PXB_CUDA(cudaStreamIsCapturing(s, &cap));
     if (cap != cudaStreamCaptureStatusNone)
         return fail(PXB_ERR_UNSUPPORTED, "the reverse mode synchronises: it cannot be captured");
+    AdjWork W(P, nsteps, every);
+    if (workspace && ws_bytes < W.bytes()) return fail(PXB_ERR_ARG, "reverse-mode workspace too small");
     double* pdev = nullptr;
     {
         const int pst = param_adjoint_buffer(P, pa, &pdev);
         if (pst != PXB_OK) return pst;
     }
-    AdjWork W;
     if (pdev) {
         W.qbar = pdev;
         if (pa->seds_bar && P->mpm) W.tbar = pdev + P->c.handlers.size();
         if (pa->seds_bar && abar->n_b) W.nbbar = (double*)abar->n_b;
     }
-    W.K = every > 0 ? every : 32;
-    W.nck = (nsteps + W.K - 1) / W.K;
-    W.plane = (size_t)P->c.ny * (size_t)P->c.pitch;
-    // checkpoints, segment states (K + 1), u1, aS, aT, aCur, aNext, aU1 (5 planes each), h1, 7 scratch
-    const size_t nplanes = (size_t)5 * (W.nck + W.K + 1 + 6) + 1 + 7;
-    int maxcount = 1;
-    for (auto& h : P->c.handlers) maxcount = std::max(maxcount, h.count);
-    auto bail = [&](int code) {
-        cudaStreamSynchronize(s);
-        W.release();
-        cudaFree(pdev);
-        return code;
-    };
-    // one block: the planes, dt and its adjoint with the step times, the tie count, the
-    // handlers' scratch.  Blocks of up to ADJ_KEEP bytes stay with the plan for its next
-    // call (allocating and freeing 200 MB took 1 to 40 ms a call).
-    const size_t nscal = 2 + (size_t)W.nck + W.K + 1, nbc = 6 * (size_t)maxcount;
-    const size_t bytes = sizeof(double) * (nplanes * W.plane + nscal + nbc);
-    W.kept = bytes <= ADJ_KEEP;
-    if (W.kept && P->adj_bytes < bytes) {
-        cudaStreamSynchronize(s);
-        cudaFree(P->adj_buf);
-        P->adj_buf = nullptr;
-        P->adj_bytes = 0;
-        if (cudaMalloc(&P->adj_buf, bytes) != cudaSuccess) return bail(fail(PXB_ERR_CUDA, "reverse-mode buffers"));
-        P->adj_bytes = bytes;
+    double* block = (double*)workspace;
+    if (!block) {
+        if (cudaMalloc(&block, W.bytes()) != cudaSuccess) {
+            cudaStreamSynchronize(s);
+            cudaFree(pdev);
+            return fail(PXB_ERR_CUDA, "reverse-mode buffers");
+        }
+        W.owned = true;
     }
-    if (W.kept) W.base = (double*)P->adj_buf;
-    else if (cudaMalloc(&W.base, bytes) != cudaSuccess) return bail(fail(PXB_ERR_CUDA, "reverse-mode buffers"));
-    W.dev = W.base + nplanes * W.plane;
-    W.nties = (unsigned int*)(W.dev + nscal - 1);
-    W.bctmp = W.dev + nscal;
-    const int o = W.nck + W.K + 1;
-    W.u1 = planes_of(W.base, W.plane, o);
-    W.aS = planes_of(W.base, W.plane, o + 1);
-    W.aT = planes_of(W.base, W.plane, o + 2);
-    W.aCur = planes_of(W.base, W.plane, o + 3);
-    W.aNext = planes_of(W.base, W.plane, o + 4);
-    W.aU1 = planes_of(W.base, W.plane, o + 5);
-    W.h1 = W.base + (size_t)5 * (o + 6) * W.plane;
-    W.gscr = W.h1 + W.plane;
+    W.place(block);
     double* tck = W.dev + 2;
     double* tseg = tck + W.nck;
     Planes5 A0;
@@ -2347,7 +2343,6 @@ int pxb_re_plan_destroy(pxb_re_plan* plan) {
     cudaFree(plan->dscr);
     cudaFree(plan->jvp_tmp);
     cudaFree(plan->bud_part);
-    cudaFree(plan->adj_buf);
     delete plan;
     return PXB_OK;
 }
@@ -2521,6 +2516,19 @@ int pxb_re_vjp_run(pxb_re_plan* P, const pxb_re_fields* a0, int32_t nsteps, int3
 int pxb_re_vjp_run_params(pxb_re_plan* P, const pxb_re_fields* a0, int32_t nsteps, int32_t scheme, double cfl,
                           double t0, int32_t checkpoint_every, const pxb_re_fields* abar,
                           const pxb_re_param_adjoints* pbar, void* stream) {
+    return pxb_re_vjp_run_in(P, a0, nsteps, scheme, cfl, t0, checkpoint_every, abar, pbar, nullptr, 0, stream);
+}
+
+int pxb_re_vjp_workspace_size(const pxb_re_plan* P, int32_t nsteps, int32_t checkpoint_every, size_t* bytes) {
+    if (!P || !bytes) return fail(PXB_ERR_ARG, "null plan or output pointer");
+    if (nsteps < 0) return fail(PXB_ERR_ARG, "nsteps < 0");
+    *bytes = AdjWork(P, nsteps, checkpoint_every).bytes();
+    return PXB_OK;
+}
+
+int pxb_re_vjp_run_in(pxb_re_plan* P, const pxb_re_fields* a0, int32_t nsteps, int32_t scheme, double cfl, double t0,
+                      int32_t checkpoint_every, const pxb_re_fields* abar, const pxb_re_param_adjoints* pbar,
+                      void* workspace, size_t bytes, void* stream) {
     if (!P) return fail(PXB_ERR_ARG, "null plan");
     if (refuse_ws(P, "the reverse mode") != PXB_OK) return PXB_ERR_UNSUPPORTED;
     if (P->c.dtype != PXB_F64) return fail(PXB_ERR_ARG, "the reverse mode runs on float64 plans");
@@ -2530,8 +2538,10 @@ int pxb_re_vjp_run_params(pxb_re_plan* P, const pxb_re_fields* a0, int32_t nstep
         return fail(PXB_ERR_ARG, "adjoint: h, hu, hv, z_b and G must be set");
     if (nsteps < 0) return fail(PXB_ERR_ARG, "nsteps < 0");
     if (scheme != PXB_FE && scheme != PXB_SSPRK2) return fail(PXB_ERR_ARG, "scheme must be PXB_FE or PXB_SSPRK2");
+    if ((uintptr_t)workspace & 255u) return fail(PXB_ERR_ARG, "the workspace must be 256-byte aligned");
     if (nsteps == 0) return PXB_OK;
-    return vjp_run_impl(P, a0, nsteps, scheme, cfl, t0, checkpoint_every, abar, pbar, (cudaStream_t)stream);
+    return vjp_run_impl(P, a0, nsteps, scheme, cfl, t0, checkpoint_every, abar, pbar, workspace, bytes,
+                        (cudaStream_t)stream);
 }
 
 int pxb_re_check(pxb_re_plan* P, void* stream) {

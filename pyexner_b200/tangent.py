@@ -182,6 +182,23 @@ class ParamAdjoints:
         return p
 
 
+# Largest reverse-mode workspace taken from torch's caching allocator, which keeps it for the
+# next call (the library's own allocation of 200 MB takes 1 to 40 ms a call).  Larger ones are
+# the library's for the call alone, so that what is kept stays small beside the device.
+WORKSPACE_MAX = 1 << 30
+
+
+def _vjp_workspace(plan, n_steps, checkpoint_every, device):
+    size = ctypes.c_size_t()
+    _lib.call("pxb_re_vjp_workspace_size", plan.handle, max(0, int(n_steps)), int(checkpoint_every), ctypes.byref(size))
+    if size.value > WORKSPACE_MAX:
+        return None
+    try:
+        return torch.empty(size.value, dtype=torch.uint8, device=device)
+    except torch.cuda.OutOfMemoryError:  # the library's call reports it
+        return None
+
+
 def vjp_run(state0, abar, mask, solver_config, n_steps, scheme="SSPRK2", cfl=0.5, t0=0.0, checkpoint_every=32,
             params=None):
     """Reverse mode of ``n_steps`` fixed steps from ``state0`` (the state after init, not
@@ -193,14 +210,13 @@ def vjp_run(state0, abar, mask, solver_config, n_steps, scheme="SSPRK2", cfl=0.5
     _check(state0, abar)
     plan = _re_plan(state0, mask, solver_config)
     code = _lib.SSPRK2 if scheme == "SSPRK2" else _lib.FE
-    if params is None:
-        _lib.call("pxb_re_vjp_run", plan.handle, ctypes.byref(state0.c_fields()), int(n_steps), code, float(cfl),
-                  float(t0), int(checkpoint_every), ctypes.byref(_adj_fields(abar)), _stream())
-    else:
-        p = params._c()
-        _lib.call("pxb_re_vjp_run_params", plan.handle, ctypes.byref(state0.c_fields()), int(n_steps), code,
-                  float(cfl), float(t0), int(checkpoint_every), ctypes.byref(_adj_fields(abar)), ctypes.byref(p),
-                  _stream())
+    p = params._c() if params is not None else None
+    work = _vjp_workspace(plan, n_steps, checkpoint_every, state0.h.device)
+    _lib.call("pxb_re_vjp_run_in", plan.handle, ctypes.byref(state0.c_fields()), int(n_steps), code, float(cfl),
+              float(t0), int(checkpoint_every), ctypes.byref(_adj_fields(abar)),
+              ctypes.byref(p) if p is not None else None,
+              ctypes.c_void_p(work.data_ptr()) if work is not None else None, work.numel() if work is not None else 0,
+              _stream())
     return abar
 
 

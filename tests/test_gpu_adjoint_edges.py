@@ -22,3 +22,54 @@ def test_parameter_adjoints_with_a_fraction_of_zero():
     assert np.all(pa.seds_bar[1:] == 0.0), pa.seds_bar
     for f in ("h", "hu", "hv", "z_b"):
         assert bool(torch.isfinite(getattr(abar, f)).all()), f
+
+
+def test_no_memory_is_kept_after_a_run():
+    """What a run needs goes back to torch's allocator: the plan holds nothing between calls."""
+    from pyexner_b200.tangent import vjp_run
+
+    def go(ny, nx, every):
+        _, cfg, mask, st = setup(*smooth_case(ny, nx))
+        abar = random_adjoint(st, np.random.default_rng(4))
+        free = []
+        for k in range(2):  # (the first call loads kernels)
+            torch.cuda.synchronize()
+            torch.cuda.empty_cache()
+            free.append(torch.cuda.mem_get_info()[0])
+            vjp_run(st, abar, mask, cfg, 4, "SSPRK2", 0.5, checkpoint_every=every)
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        return free + [torch.cuda.mem_get_info()[0]]
+
+    go(26, 34, 4)
+    free = go(400, 400, 4)  # a workspace of about 90 MB
+    assert free[0] - free[2] < 32 << 20, free
+
+
+def test_workspace_of_the_c_call():
+    """The run in a caller's workspace against the run that allocates its own (the adjoint's
+    atomic sums vary in their last bits: 1e-12 normwise), and what is refused."""
+    import ctypes
+
+    from pyexner_b200 import _lib
+    from pyexner_b200.solvers import _re_plan, _stream
+
+    _, cfg, mask, st = setup(*smooth_case(40, 50))
+    plan = _re_plan(st, mask, cfg)
+    size = ctypes.c_size_t()
+    _lib.call("pxb_re_vjp_workspace_size", plan.handle, 5, 2, ctypes.byref(size))
+    work = torch.empty(size.value + 256, dtype=torch.uint8, device="cuda")
+    a = random_adjoint(st, np.random.default_rng(4))
+    b = a.clone()
+
+    def args(bar):
+        return (plan.handle, ctypes.byref(st.c_fields()), 5, _lib.SSPRK2, 0.5, 0.0, 2, ctypes.byref(bar.c_fields()))
+
+    _lib.call("pxb_re_vjp_run", *args(a), _stream())
+    for ptr, n in ((work.data_ptr(), size.value - 1), (work.data_ptr() + 8, size.value)):
+        with pytest.raises(_lib.PxbError):
+            _lib.call("pxb_re_vjp_run_in", *args(b), None, ctypes.c_void_p(ptr), n, _stream())
+    _lib.call("pxb_re_vjp_run_in", *args(b), None, ctypes.c_void_p(work.data_ptr()), size.value, _stream())
+    for f in ("h", "hu", "hv", "z_b", "G"):
+        x, y = getattr(a, f), getattr(b, f)
+        assert float((x - y).abs().max()) <= 1e-12 * float(x.abs().max()), f
