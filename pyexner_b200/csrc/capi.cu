@@ -1724,10 +1724,8 @@ int copy5(PlanCommon& C, const Planes5& dst, const Planes5& src, cudaStream_t s)
 // The same from or to the caller's planes, which end with their last cell and whose columns
 // beyond nx belong to the caller.
 int copy5_cells(PlanCommon& C, const Planes5& dst, const Planes5& src, cudaStream_t s) {
-    const size_t pitch = sizeof(double) * (size_t)C.pitch;
-    for (int f = 0; f < 5; ++f)
-        PXB_CUDA(cudaMemcpy2DAsync(dst.p[f], pitch, src.p[f], pitch, sizeof(double) * (size_t)C.nx, C.ny,
-                                   cudaMemcpyDeviceToDevice, s));
+    const double* const o[5] = {src.p[0], src.p[1], src.p[2], src.p[3], src.p[4]};
+    PXB_CUDA(pxb::launch_adj_store(C.ny, C.nx, C.pitch, 1.0, o, dst.p, nullptr, s));
     return PXB_OK;
 }
 
@@ -2031,7 +2029,7 @@ int vjp_run_impl(pxb_re_plan* P, const pxb_re_fields* a0, int nsteps, int scheme
             if (n > 0) chk(copy5(P->c, W.ck(k), W.seg(0), s));
             if (cudaMemcpyAsync(tck + k, &P->c.scr->t_next, 8, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
                 st = fail(PXB_ERR_CUDA, "checkpoint time");
-            if (n == 0) chk(copy5_cells(P->c, W.seg(0), A0, s));
+            if (n == 0) chk(copy5(P->c, W.seg(0), W.ck(0), s));
         }
         if (st == PXB_OK) chk(adj_step_fwd(P, W, W.seg(0), W.seg(0), scheme, a0, cfl, s));
     }
