@@ -440,12 +440,13 @@ __global__ void __launch_bounds__(ADJ_THREADS, PXB_ADJ_MIN_BLOCKS) adj_hydro_ker
 // were overwritten); read past the L1, behind the atomics of the handler before.
 __device__ __forceinline__ void adj_bc_take(const AdjBcSet& a, const AdjBcHandler& h, const long long b, double (&t)[6]) {
     const unsigned fm = bc_field_mask(h.kind);
+    auto writes = [&](int s) { return ((fm >> s) & 1u) && a.f[s]; };
 #pragma unroll
-    for (int s = 0; s < 6; ++s) {
-        const bool w = ((fm >> s) & 1u) && a.f[s];
-        t[s] = w ? __ldcg(a.f[s] + b) : 0.0;
-        if (w) a.f[s][b] = 0.0;
-    }
+    for (int s = 0; s < 6; ++s) t[s] = writes(s) ? __ldcg(a.f[s] + b) : 0.0;
+    // (all loads in flight before the first store, which might alias the next plane)
+#pragma unroll
+    for (int s = 0; s < 6; ++s)
+        if (writes(s)) a.f[s][b] = 0.0;
 }
 
 // The donor receives the transposed Jacobian of the handler times the adjoints taken.
@@ -495,10 +496,14 @@ __device__ __forceinline__ void adj_bc_give(const AdjBcSet& a, const AdjBcHandle
     }
 }
 
-// Handlers backwards, the last one first, by one block (three launches per handler took 2 us
-// each).  A thread keeps what it takes of its first ADJ_BC_KEEP cells of a handler in
-// registers, of more cells in the temporary; the next handler's first indices are read ahead.
+// Handlers backwards, the last one first, by one block.  A thread keeps what it takes of a
+// handler's cells, at most ADJ_BC_KEEP, in registers; the next handler's indices are read ahead.
+// Bound by the chain of loads, barrier and atomics of each handler: 2.7 us for one of 514 cells,
+// 4.5 for 1026 and 2048.  Beyond the registers one block pays for every 1024 cells more (4096
+// cells 9 us, 65536 166 us); two launches over all cells take 3.7 to 5.5 us for any of them
+// (three took 7).
 constexpr int ADJ_BC_KEEP = 2;
+static_assert(ADJ_BC_KEEP * 1024 == ADJ_BC_SET_CELLS, "a block of 1024 threads keeps a handler's cells");
 __global__ void __launch_bounds__(1024) adj_bc_set_kernel(const __grid_constant__ AdjBcSet a) {
     const int nt = blockDim.x;
     long long cell[ADJ_BC_KEEP], donor[ADJ_BC_KEEP];
@@ -520,28 +525,37 @@ __global__ void __launch_bounds__(1024) adj_bc_set_kernel(const __grid_constant_
             d[u] = donor[u];
             if ((int)threadIdx.x + u * nt < h.count) adj_bc_take(a, h, cell[u], t[u]);
         }
-        for (int k = threadIdx.x + ADJ_BC_KEEP * nt; k < h.count; k += nt) {
-            double x[6];
-            adj_bc_take(a, h, h.cells[k], x);
-#pragma unroll
-            for (int s = 0; s < 6; ++s) a.tmp[s * h.count + k] = x[s];
-        }
         if (q > 0) ahead(q - 1);
         __syncthreads();  // every clear before any addition
 #pragma unroll
         for (int u = 0; u < ADJ_BC_KEEP; ++u)
             if ((int)threadIdx.x + u * nt < h.count) adj_bc_give(a, h, d[u], t[u]);
-        for (int k = threadIdx.x + ADJ_BC_KEEP * nt; k < h.count; k += nt) {
-            double x[6];
-#pragma unroll
-            for (int s = 0; s < 6; ++s) x[s] = a.tmp[s * h.count + k];
-            adj_bc_give(a, h, h.donors[k], x);
-        }
         if (q > 0) {
             __threadfence();
             __syncthreads();
         }
     }
+}
+
+// One handler of more cells (a.h[0]) in two launches over all of them: take, then give.
+__global__ void __launch_bounds__(256) adj_bc_take_kernel(const __grid_constant__ AdjBcSet a) {
+    const AdjBcHandler& h = a.h[0];
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= h.count) return;
+    double t[6];
+    adj_bc_take(a, h, h.cells[k], t);
+#pragma unroll
+    for (int s = 0; s < 6; ++s) a.tmp[(size_t)s * h.count + k] = t[s];
+}
+
+__global__ void __launch_bounds__(256) adj_bc_give_kernel(const __grid_constant__ AdjBcSet a) {
+    const AdjBcHandler& h = a.h[0];
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= h.count) return;
+    double t[6];
+#pragma unroll
+    for (int s = 0; s < 6; ++s) t[s] = a.tmp[(size_t)s * h.count + k];
+    adj_bc_give(a, h, h.donors[k], t);
 }
 
 // compute_n of the initialisation backwards (roe_exner.py:64-73): n_b = n_p_mix where the

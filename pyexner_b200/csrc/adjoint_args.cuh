@@ -36,10 +36,11 @@ struct AdjBcHandler {
     double vx, vy;  // ConstantInflux: d(hu, hv) / d values[0] = (values[1], values[2])
     double* qbar;   // ConstantInflux: adjoint of its values[0] (accumulated; null: not requested)
 };
-constexpr int ADJ_BC_SET_MAX = 16;
+// Handlers of one launch, and the boundary cells up to which a handler goes into one.
+constexpr int ADJ_BC_SET_MAX = 16, ADJ_BC_SET_CELLS = 2048;
 struct AdjBcSet {  // in the order of application; run backwards
     double* f[6];
-    double* tmp;  // 6 * the largest count
+    double* tmp;  // 6 * the largest count above ADJ_BC_SET_CELLS
     int n;
     AdjBcHandler h[ADJ_BC_SET_MAX];
 };

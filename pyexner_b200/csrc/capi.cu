@@ -1740,7 +1740,12 @@ int zero5(PlanCommon& C, const Planes5& q, cudaStream_t s) {
 int adj_handlers(PlanCommon& C, double* const f[6], double* tmp, cudaStream_t s, double* qbar = nullptr) {
     size_t end = C.handlers.size();
     while (end > 0) {
-        const size_t begin = end > (size_t)pxb::ADJ_BC_SET_MAX ? end - pxb::ADJ_BC_SET_MAX : 0;
+        // the last handler alone if it is large, else those before it that go into one launch
+        size_t begin = end - 1;
+        if (C.handlers[begin].count <= pxb::ADJ_BC_SET_CELLS)
+            while (begin > 0 && end - begin < (size_t)pxb::ADJ_BC_SET_MAX &&
+                   C.handlers[begin - 1].count <= pxb::ADJ_BC_SET_CELLS)
+                --begin;
         pxb::AdjBcSet set{};
         for (int k = 0; k < 6; ++k) set.f[k] = f[k];
         set.tmp = tmp;

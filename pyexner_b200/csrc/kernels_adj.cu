@@ -48,6 +48,13 @@ cudaError_t launch_adj_bc(const AdjBcSet& a, cudaStream_t s) {
     for (int k = 0; k < a.n; ++k) most = a.h[k].count > most ? a.h[k].count : most;
     const int threads = most >= 1024 ? 1024 : (most + 31) / 32 * 32;
     if (threads == 0) return cudaSuccess;
+    if (most > ADJ_BC_SET_CELLS) {
+        if (a.n != 1) return cudaErrorInvalidConfiguration;
+        const int g = (most + 255) / 256;
+        adj_bc_take_kernel<<<g, 256, 0, s>>>(a);
+        adj_bc_give_kernel<<<g, 256, 0, s>>>(a);
+        return cudaGetLastError();
+    }
     adj_bc_set_kernel<<<1, threads, 0, s>>>(a);
     return cudaGetLastError();
 }

@@ -73,3 +73,33 @@ def test_workspace_of_the_c_call():
     for f in ("h", "hu", "hv", "z_b", "G"):
         x, y = getattr(a, f), getattr(b, f)
         assert float((x - y).abs().max()) <= 1e-12 * float(x.abs().max()), f
+
+
+# the largest handler of the one-block launch and the smallest of the launches over all cells
+@pytest.mark.parametrize("rows,cols", [(23, 89), (32, 64), (41, 50)])
+def test_handlers_of_many_cells(rows, cols):
+    """<abar_0, du_0> == <abar_N, J du_0> over 3 steps (1e-9, the bound of the other layouts) with a
+    slab of rows * cols boundary cells between small handlers, one of which overwrites part of
+    it."""
+    from pyexner_b200.tangent import jvp_run, vjp_run
+    from test_gpu_tangent import inner, tangent_state
+
+    ny, nx = 60, 100
+    arrs, params, X, Y = smooth_case(ny, nx)
+
+    def rect(x0, x1, y0, y1):
+        return [[x0 - 0.5, y0 - 0.5], [x1 + 0.5, y0 - 0.5], [x1 + 0.5, y1 + 0.5], [x0 - 0.5, y1 + 0.5]]
+
+    spec = dict(params["boundaries"])
+    spec["slab"] = dict(type="Reflective", polygon=rect(4, 3 + cols, 5, 4 + rows), values=[0.0] * 4, normal=[0.0, -1.0])
+    spec["wall"] = dict(type="Transmissive", polygon=rect(6, 6, 7, 20), values=[0.0] * 4, normal=[-1.0, 0.0])
+    _, cfg, mask, st = setup(arrs, dict(params, boundaries=spec), X, Y)
+    assert cfg.boundaries.handlers[-2]["cells"][0].size == rows * cols
+    rng = np.random.default_rng(3)
+    du = tangent_state(st, rng, ("h", "hu", "hv", "z_b"))
+    s, td = st.clone(), du.clone()
+    jvp_run(s, td, mask, cfg, 3, "SSPRK2", 0.5)
+    abar = random_adjoint(st, rng)
+    rhs = inner(abar, td)
+    a0 = vjp_run(st, abar.clone(), mask, cfg, 3, "SSPRK2", 0.5, checkpoint_every=2)
+    assert abs(inner(a0, du, ("h", "hu", "hv", "z_b")) - rhs) <= 1e-9 * max(abs(rhs), 1e-30)
