@@ -296,12 +296,6 @@ void berthon_constants(const double* v, DevHandler& d) {
     d.q = q;
 }
 
-// Work items of the CFL reduction.
-struct Geometry {
-    int band_rows = 0, nstrips = 0, nbands = 0, grid = 0;
-    bool wide = false;
-};
-
 // Tiles of the stage kernel: warps side by side and on top of one another, rows in shared
 // memory (owned rows of the tallest band and two on each side), launch shape.
 struct StageGeometry {
@@ -386,22 +380,6 @@ StageGeometry stage_geometry(int ny, int nx, int esize, int sm_count, int want_r
         }
     }
     return best;
-}
-
-// Work items of the CFL reduction, about 32 warps of them per SM (16: 24 to 30 % slower at
-// 2048^2, 64 as well).  Below the line a wide item's bounds cost more than evaluating every
-// face of narrow items (float32 731 x 1203: 15.7 us narrow, 27.5 wide; 1024^2 11.2 both;
-// 2048^2 43.8 and 19.3.  float64 512^2: 22.8 and 33; 1024^2 76 and 48).
-Geometry cfl_geometry(int ny, int nx, int esize, int sm_count) {
-    Geometry g;
-    g.wide = (long long)ny * nx > (esize == 8 ? 500000 : 1200000);
-    g.nstrips = g.wide ? (nx + pxb::CFL_WIDE - 1) / pxb::CFL_WIDE : (nx + pxb::CFL_NARROW - 1) / pxb::CFL_NARROW;
-    const int want = std::max(1, 32 * sm_count / g.nstrips);
-    g.band_rows = std::max(2, (ny + want - 1) / want);
-    if (g.wide) g.band_rows = std::min(pxb::CFL_MAX_ROWS, std::max(4, g.band_rows));
-    g.nbands = (ny + g.band_rows - 1) / g.band_rows;
-    g.grid = (int)(((long long)g.nstrips * g.nbands + 7) / 8);
-    return g;
 }
 
 // Device memory of a plan: cudaMalloc'd (no arena), carved from a caller's workspace, or
@@ -597,7 +575,7 @@ struct PlanCommon {
     void* dt_dev = nullptr;
     cudaStream_t cap = nullptr;  // capture stream of the graph cache, created on first use
     bool ws = false;             // device memory carved from the caller's workspace
-    Geometry cfl;
+    pxb::CflItems cfl;
     // graph cache
     struct Cached {
         std::vector<const void*> key;
@@ -2299,7 +2277,7 @@ int re_plan_create(const pxb_re_config* cfg, DevArena* A, pxb_re_plan** out) {
         delete P;
         return fail(PXB_ERR_CUDA, std::string("stage kernel shared memory: ") + cudaGetErrorString(es));
     }
-    P->c.cfl = cfl_geometry(cfg->ny, cfg->nx, f64 ? 8 : 4, P->c.sm_count);
+    P->c.cfl = pxb::cfl_items(cfg->ny, cfg->nx, f64 ? 8 : 4, P->c.sm_count);
     *out = P;
     return PXB_OK;
 }

@@ -8,16 +8,20 @@
 // keeps its reduction scratch in a fixed array in device memory that the module owns.
 //
 // The scratch holds one partial maximum per work item (a 31-column strip times a band
-// of rows) plus the completion counter of the last-block reduction.  Work items are
+// of rows) plus the completion counter of the last-block reduction, and the plan kernel's
+// reduction state for large grids.  Work items are
 // capped at PXB_NOALLOC_MAX_ITEMS, which bounds the grid width to
 // 31 * PXB_NOALLOC_MAX_ITEMS columns; wider grids are rejected.  The array stays
 // resident on every device that loads the library until the process exits.  All calls
 // share it, so two calls whose kernels overlap on the GPU (different streams without
 // ordering between them, or different host threads on one device) race on it.
 //
-// The kernel (noalloc_kernel.cuh) runs the plan-based CFL's own work item, so both entry
-// points evaluate the same faces with the same arithmetic; its float64 instantiation is
-// compiled in noalloc_f64.cu with --fmad=false, like the other float64 kernels.
+// Up to PXB_NOALLOC_NARROW_CELLS the kernel (noalloc_kernel.cuh) evaluates every face with
+// the plan-based CFL's narrow work item, which is also what that one's wide items are checked
+// against; its float64 instantiation is compiled in noalloc_f64.cu with --fmad=false, like the
+// other float64 kernels.  Larger grids take the plan kernel with wide items (float32 at rest,
+// narrow and wide: 2050^2 31 and 20 us, 4098^2 111 and 58, 8194^2 372 and 189).  Both give the
+// same dt bit for bit.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -28,7 +32,10 @@
 #include "pxb_launch.h"
 
 #define PXB_NOALLOC_MAX_ITEMS 8192
-#define PXB_NOALLOC_WORDS (PXB_NOALLOC_MAX_ITEMS + 32)  // partials, then the counter
+#define PXB_NOALLOC_WORDS (PXB_NOALLOC_MAX_ITEMS + 32)  // partials, the counter, a CflScratch
+#define PXB_NOALLOC_SCRATCH (PXB_NOALLOC_MAX_ITEMS + 8)  // first word of the CflScratch
+#define PXB_NOALLOC_NARROW_CELLS 4000000
+static_assert(sizeof(pxb::CflScratch) <= 8 * (PXB_NOALLOC_WORDS - PXB_NOALLOC_SCRATCH), "the scratch holds a CflScratch");
 
 static __device__ __align__(256) unsigned long long pxb_noalloc_scratch[PXB_NOALLOC_WORDS];
 
@@ -53,6 +60,7 @@ struct DevSlot {
     bool ready = false;
     void* ctx = nullptr;
     unsigned long long* ptr = nullptr;
+    int sm_count = 0;
 };
 std::mutex g_mu;
 DevSlot g_slots[64];
@@ -74,7 +82,7 @@ int current_context(void** ctx) {
     return PXB_OK;
 }
 
-int scratch_for_current_device(unsigned long long** out) {
+int scratch_for_current_device(unsigned long long** out, int* sm_count) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return nfail(PXB_ERR_CUDA, std::string("cudaGetDevice: ") + cudaGetErrorString(e));
@@ -90,28 +98,26 @@ int scratch_for_current_device(unsigned long long** out) {
             return nfail(PXB_ERR_CUDA, std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
         st = current_context(&ctx);  // the context the address belongs to
         if (st != PXB_OK) return st;
+        e = cudaDeviceGetAttribute(&g_slots[dev].sm_count, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess)
+            return nfail(PXB_ERR_CUDA, std::string("cudaDeviceGetAttribute: ") + cudaGetErrorString(e));
         g_slots[dev].ptr = (unsigned long long*)p;
         g_slots[dev].ctx = ctx;
         g_slots[dev].ready = true;
     }
     *out = g_slots[dev].ptr;
+    *sm_count = g_slots[dev].sm_count;
     return PXB_OK;
 }
 
 template <class T>
 int launch(int ny, int nx, long long pitch, double dx, double cfl, const void* h, const void* hu, const void* hv,
            const void* G, const uint8_t* nodata, void* dt_out, cudaStream_t s) {
-    const int nstrips = (nx + 30) / 31;
-    int nbands = std::max(1, std::min((ny + 7) / 8, PXB_NOALLOC_MAX_ITEMS / nstrips));
-    const int band_rows = (ny + nbands - 1) / nbands;
-    nbands = (ny + band_rows - 1) / band_rows;
-    const int nitems = nstrips * nbands;
     unsigned long long* scr = nullptr;
-    int st = scratch_for_current_device(&scr);
+    int sm_count = 0;
+    int st = scratch_for_current_device(&scr, &sm_count);
     if (st != PXB_OK) return st;
-    unsigned int* done = (unsigned int*)(scr + PXB_NOALLOC_MAX_ITEMS);
-    cudaError_t e = cudaMemsetAsync(done, 0, sizeof(unsigned int), s);
-    if (e != cudaSuccess) return nfail(PXB_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
+    cudaError_t e;
     pxb::CflArgs<T> a{};
     a.ny = ny;
     a.nx = nx;
@@ -125,9 +131,27 @@ int launch(int ny, int nx, long long pitch, double dx, double cfl, const void* h
     a.cfl = (T)cfl;
     a.floor_dt = (T)pxb::DT_FLOOR;
     a.dt_out = (T*)dt_out;
-    a.band_rows = band_rows;
-    a.nstrips = nstrips;
-    a.nbands = nbands;
+    if ((long long)ny * nx > PXB_NOALLOC_NARROW_CELLS) {
+        const pxb::CflItems g = pxb::cfl_items(ny, nx, true, sm_count);
+        a.scr = (pxb::CflScratch*)(scr + PXB_NOALLOC_SCRATCH);
+        a.band_rows = g.band_rows;
+        a.nstrips = g.nstrips;
+        a.nbands = g.nbands;
+        a.wide = 1;
+        e = cudaMemsetAsync(a.scr, 0, sizeof(pxb::CflScratch), s);
+        if (e != cudaSuccess) return nfail(PXB_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
+        e = pxb::launch_re_cfl<T>(a, nodata != nullptr, g.grid, s);
+        if (e != cudaSuccess) return nfail(PXB_ERR_CUDA, std::string("cfl kernel launch: ") + cudaGetErrorString(e));
+        return PXB_OK;
+    }
+    a.nstrips = (nx + 30) / 31;
+    const int want = std::max(1, std::min((ny + 7) / 8, PXB_NOALLOC_MAX_ITEMS / a.nstrips));
+    a.band_rows = (ny + want - 1) / want;
+    a.nbands = (ny + a.band_rows - 1) / a.band_rows;
+    const int nitems = a.nstrips * a.nbands;
+    unsigned int* done = (unsigned int*)(scr + PXB_NOALLOC_MAX_ITEMS);
+    e = cudaMemsetAsync(done, 0, sizeof(unsigned int), s);
+    if (e != cudaSuccess) return nfail(PXB_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
     e = pxb::launch_cfl_noalloc<T>(a, scr, done, nitems, s);
     if (e != cudaSuccess) return nfail(PXB_ERR_CUDA, std::string("cfl kernel launch: ") + cudaGetErrorString(e));
     return PXB_OK;

@@ -26,6 +26,7 @@
 // 19.3 and with bedload 51 -> 26, 8192^2 293 -> 185; float64 256^2 36 -> 13, 1024^2 with
 // bedload 64 -> 48.
 #pragma once
+#include <algorithm>
 #include <type_traits>
 
 #include "pxb_device.cuh"
@@ -66,6 +67,31 @@ struct CflArgs {
 
 constexpr int CFL_WIDE = 124, CFL_NARROW = 31;  // columns of an item
 constexpr int CFL_MAX_ROWS = 64;                // rows of a wide item (a lane keeps two bounds)
+
+// Work items of the reduction over a grid, 8 a block.
+struct CflItems {
+    int band_rows = 0, nstrips = 0, nbands = 0, grid = 0;
+    bool wide = false;
+};
+// Items of one width, about 32 warps of them per SM (16: 24 to 30 % slower at 2048^2, 64 as
+// well).
+static inline CflItems cfl_items(int ny, int nx, bool wide, int sm_count) {
+    CflItems g;
+    g.wide = wide;
+    g.nstrips = wide ? (nx + CFL_WIDE - 1) / CFL_WIDE : (nx + CFL_NARROW - 1) / CFL_NARROW;
+    const int want = std::max(1, 32 * sm_count / g.nstrips);
+    g.band_rows = std::max(2, (ny + want - 1) / want);
+    if (wide) g.band_rows = std::min(CFL_MAX_ROWS, std::max(4, g.band_rows));
+    g.nbands = (ny + g.band_rows - 1) / g.band_rows;
+    g.grid = (int)(((long long)g.nstrips * g.nbands + 7) / 8);
+    return g;
+}
+// A plan's items.  Below the line a wide item's bounds cost more than evaluating every face of
+// narrow items (float32 731 x 1203: 15.7 us narrow, 27.5 wide; 1024^2 11.2 both; 2048^2 43.8
+// and 19.3.  float64 512^2: 22.8 and 33; 1024^2 76 and 48).
+static inline CflItems cfl_items(int ny, int nx, int esize, int sm_count) {
+    return cfl_items(ny, nx, (long long)ny * nx > (esize == 8 ? 500000 : 1200000), sm_count);
+}
 
 // Resident 256-thread blocks per SM: 4 (64 registers; the spills are in the exact rows of wide
 // items) against 2 and 3 is 15 to 30 % faster at 8192^2 in float32.
