@@ -597,9 +597,10 @@ __device__ __forceinline__ bool adj_at_max(const AdjCflArgs& a, int r, int c, bo
     if (yf ? (r + 1 >= a.ny) : (c + 1 >= a.nx)) return false;
     const long long i = (long long)r * a.pitch + c, j = yf ? i + a.pitch : i + 1;
     const float hi = clamp_lo((float)a.h[i], (float)DRY_TOL), hj = clamp_lo((float)a.h[j], (float)DRY_TOL);
-    const float ui = fmax_nan(fabsf((float)a.hu[i]), fabsf((float)a.hv[i])) * f_rcp(hi);
-    const float uj = fmax_nan(fabsf((float)a.hu[j]), fabsf((float)a.hv[j])) * f_rcp(hj);
-    const float b = cfl_bound(fmax_nan(ui, uj), fmax_nan(hi, hj), fminf(hi, hj), fmax_nan(fabsf((float)a.G[i]), fabsf((float)a.G[j])));
+    const float ri = f_rcp(hi), rj = f_rcp(hj);
+    const float U = fmax_nan(fabsf((float)a.hu[i]) * ri, fabsf((float)a.hu[j]) * rj);
+    const float V = fmax_nan(fabsf((float)a.hv[i]) * ri, fabsf((float)a.hv[j]) * rj);
+    const float b = cfl_bound(U, V, fmax_nan(hi, hj), fminf(hi, hj), fmax_nan(fabsf((float)a.G[i]), fabsf((float)a.G[j])));
     double s;
     return !(b < smax) && adj_face_speed(a, r, c, yf, s) && speed_bits(s) == m;
 }

@@ -16,15 +16,20 @@
 // of its faces: the largest over the lanes, each from the extremes of h, |u|, |v| and G
 // among the ten cells its faces join.  Exact speeds of one row of 31 columns per item,
 // spread over the grid, give a lower bound of the maximum; only rows whose bound is not
-// below what is known by then are evaluated face by face, shared out over the block's warps
-// (they lie close together: left to the warp that found them, one warp's rows set the
-// kernel's time).  A face that is left out cannot be the fastest, so dt keeps its bits.
+// below what is known by then are evaluated face by face, as narrow items of up to four rows
+// shared out over the block's warps (they lie close together: left to the warp that found
+// them, one warp's rows set the kernel's time).  A face that is left out cannot be the
+// fastest, so dt keeps its bits.
 //
 // Bound by the read of h, hu, hv and G (8192^2: 5.9 TB/s) and, on small grids, by the chain
-// of launch, loads, reduction and last block.  Evaluating every face took 125 to 300
-// instructions per row of 31.  us, before -> after: float32 256^2 7.8 -> 5.3, 2048^2 24.6 ->
-// 19.3 and with bedload 51 -> 26, 8192^2 293 -> 185; float64 256^2 36 -> 13, 1024^2 with
-// bedload 64 -> 48.
+// of launch, loads, reduction and last block.  Evaluating every face takes 125 to 300
+// instructions per row of 31.  us with every face evaluated (by 16-byte row copies in
+// float32) -> now: float32 514^2 8.1 -> 5.9 and with a constant G 11.1 -> 7.6; 2050^2 24.5 ->
+// 15.6 below the bedload threshold, 53 -> 25 with bedload or a constant G everywhere; 4098^2
+// 82 -> 55 and 192 -> 70; float64 1026^2 27 -> 17 and 77 -> 52; 2050^2 93 -> 36 and 284 -> 95.
+// In a field whose cells differ from one another like noise no row is ruled out and every
+// face is evaluated after the bounds: float32 2050^2 256 -> 225, float64 1026^2 70 -> 92,
+// 2050^2 263 -> 339.
 #pragma once
 #include <algorithm>
 #include <type_traits>
@@ -67,6 +72,8 @@ struct CflArgs {
 
 constexpr int CFL_WIDE = 124, CFL_NARROW = 31;  // columns of an item
 constexpr int CFL_MAX_ROWS = 64;                // rows of a wide item (a lane keeps two bounds)
+constexpr int CFL_CHUNK = 4;  // rows of an item that are evaluated together (4096^2 at rest, float32: 58 us with 16, 55 with 4)
+static_assert(CFL_WIDE % CFL_NARROW == 0 && 32 % CFL_CHUNK == 0, "shapes of the wide items");
 
 // Work items of the reduction over a grid, 8 a block.
 struct CflItems {
@@ -175,23 +182,26 @@ __device__ __forceinline__ void cfl_rows(const CflArgs<T>& a, const int c0, cons
 __device__ __forceinline__ float fmax_nan(float a, float b) { float y; asm("max.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b)); return y; }
 
 // Upper bound of the face speeds among cells with depths (clamped at DRY_TOL) in [hm, hM],
-// velocity components up to U and grass factors up to G, with a margin for the rounding of
-// the bound and of the speeds.  Without G the speeds are |u~| + c~ with u~ between the
-// cells' velocities and c~ <= sqrt(g hM).  With G the speeds are the roots of
-//   l ((l - u)^2 - c^2) = a c^2 (l + u),  a <= A = 4 G U^2 / hm
-// (the sign of l turned).  A root with |l| > |u| has (|l| - |u|)^2 <= c^2 (1 + 2 a), so
-// |l| <= |u| + c sqrt(1 + 2 a).  The trigonometric solution gives the roots when all three
-// are real; at l = -(c - u)/2 (u >= 0) the left side less the right is at least
+// velocity components up to U and V and grass factors up to G, with a margin for the rounding
+// of the bound and of the speeds.  With M the larger of U and V and m the other, a face's
+// normal velocities and u~ are up to M and its c~ lies between the cells' sqrt(g h).  Without
+// G the speeds are |u~| + c~.  With G they are the roots of
+//   l ((l - u)^2 - c^2) = a c^2 (l + u),  a <= A = G (3 M^2 + m^2) / hm
+// (the sign of l turned; u >= 0).  A positive root has l <= u - c, or l >= u + c and then
+// (l - u)^2 = c^2 (1 + a (1 + u / l)) with u / l <= u / (u + c) <= M / (M + cm); a negative
+// one has |l| <= c sqrt(1 + a) - u.  The trigonometric solution gives the roots when all three
+// are real; at l = -(c - u)/2 the left side less the right is at least
 // (c - u)^2 (3 c + u) / 8 - a c^2 u, which is positive, and all three are, when
-// A cM^2 U < 0.375 (cm - U)^2 cm.  Otherwise its argument is clipped and its values are
+// A cM^2 M < 0.375 (cm - M)^2 cm.  Otherwise its argument is clipped and its values are
 // within 4/3 |u| + 2/sqrt(3) c sqrt(1 + a).  A NaN makes the bound NaN.
-__device__ __forceinline__ float cfl_bound(float U, float hM, float hm, float G) {
-    const float cM = f_sqrt(9.81f * hM);
-    if (G == 0.f) return (U + cM) * 1.00002f;
-    const float A = 4.f * G * U * U / hm * 1.0001f, cm = f_sqrt(9.81f * hm) - U;
-    const bool three = cm > 0.f && A * cM * cM * U < 0.374f * cm * cm * (cm + U);
-    const float tight = U + cM * f_sqrt(1.f + 2.f * A);
-    const float loose = 1.3334f * U + 1.1548f * cM * f_sqrt(1.f + A);
+__device__ __forceinline__ float cfl_bound(float U, float V, float hM, float hm, float G) {
+    const float cM = f_sqrt(9.81f * hM), M = fmax_nan(U, V);
+    if (G == 0.f) return (M + cM) * 1.00002f;
+    const float m = fminf(U, V), cs = f_sqrt(9.81f * hm), cm = cs - M;
+    const float A = G * (3.f * M * M + m * m) / hm * 1.0001f;
+    const bool three = cm > 0.f && A * cM * cM * M < 0.374f * cm * cm * cs;
+    const float tight = M + cM * f_sqrt(1.f + A * (1.f + M * f_rcp(M + cs)));
+    const float loose = 1.3334f * M + 1.1548f * cM * f_sqrt(1.f + A);
     return (three ? tight : loose) * 1.0002f;
 }
 
@@ -255,16 +265,17 @@ __device__ __forceinline__ void cfl_wide_bounds(const CflArgs<T>& a, const CflSt
     using Row = CflRow<T>;
     auto load = [&](int r, Row& x) __attribute__((always_inline)) { cfl_load<T, VEC>(a, st, r, x); };
     // extremes of this lane's four cells of a row and the next column's
-    struct Ext { float U, hM, hm, G; };
+    struct Ext { float U, V, hM, hm, G; };
     auto extremes = [&](const Row& x) __attribute__((always_inline)) {
-        Ext e{0.f, 0.f, 3e38f, 0.f};
-        float h0 = 0.f, u0 = 0.f, g = 0.f, g0 = 0.f;
+        Ext e{0.f, 0.f, 0.f, 3e38f, 0.f};
+        float h0 = 0.f, u0 = 0.f, v0 = 0.f, g = 0.f, g0 = 0.f;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const float h = clamp_lo((float)x.h[k], (float)DRY_TOL);
-            const float u = fmax_nan(fabsf((float)x.hu[k]), fabsf((float)x.hv[k])) * f_rcp(h);
-            if (k == 0) h0 = h, u0 = u;
+            const float h = clamp_lo((float)x.h[k], (float)DRY_TOL), r = f_rcp(h);
+            const float u = fabsf((float)x.hu[k]) * r, v = fabsf((float)x.hv[k]) * r;
+            if (k == 0) h0 = h, u0 = u, v0 = v;
             e.U = fmax_nan(e.U, u);
+            e.V = fmax_nan(e.V, v);
             e.hM = fmax_nan(e.hM, h);
             e.hm = fminf(e.hm, h);
             g = fmax_nan(g, fabsf((float)x.g[k]));
@@ -273,6 +284,7 @@ __device__ __forceinline__ void cfl_wide_bounds(const CflArgs<T>& a, const CflSt
         e.G = fmax_nan(g, __shfl_down_sync(FULL, g0, 1));
         const float he = __shfl_down_sync(FULL, h0, 1);
         e.U = fmax_nan(e.U, __shfl_down_sync(FULL, u0, 1));
+        e.V = fmax_nan(e.V, __shfl_down_sync(FULL, v0, 1));
         e.hM = fmax_nan(e.hM, he);
         e.hm = fminf(e.hm, he);
         return e;
@@ -288,7 +300,8 @@ __device__ __forceinline__ void cfl_wide_bounds(const CflArgs<T>& a, const CflSt
             if (r + 2 < rend) load(r + 2, nxt);
             ce = extremes(cur);
         }
-        const float b = cfl_bound(fmax_nan(pe.U, ce.U), fmax_nan(pe.hM, ce.hM), fminf(pe.hm, ce.hm), fmax_nan(pe.G, ce.G));
+        const float b = cfl_bound(fmax_nan(pe.U, ce.U), fmax_nan(pe.V, ce.V), fmax_nan(pe.hM, ce.hM), fminf(pe.hm, ce.hm),
+                                  fmax_nan(pe.G, ce.G));
         const float w = __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(b)));  // (NaN above all numbers)
         const int k = r - R0;
         if (lane == (k & 31)) (k < 32 ? bound0 : bound1) = w;
@@ -296,67 +309,22 @@ __device__ __forceinline__ void cfl_wide_bounds(const CflArgs<T>& a, const CflSt
     }
 }
 
-// The exact speeds of one row of a wide item, largest bits folded into `best`.
-template <class T, bool HAS_MASK, bool VEC>
-__device__ __forceinline__ void cfl_wide_row(const CflArgs<T>& a, const CflStrip<T>& st, const int r, speed_bits_t<T>& best) {
-    const int lane = threadIdx.x & 31, ny = a.ny, nx = a.nx, c = st.c;
-    using Row = CflRow<T>;
-    auto load = [&](int q, Row& x) __attribute__((always_inline)) { cfl_load<T, VEC>(a, st, q, x); };
-    auto fold = [&](T v) __attribute__((always_inline)) {
-        const speed_bits_t<T> b = (speed_bits_t<T>)speed_bits(v);
-        best = b > best ? b : best;
-    };
-    const bool south = r + 1 < ny;
-    Row x, y;
-    load(r, x);
-    if (south) load(r + 1, y);
-    else y = x;
-    CCell<T> p[5], q[4];
-#pragma unroll
-    for (int n = 0; n < 4; ++n) {
-        p[n] = make_ccell(x.h[n], x.hu[n], x.hv[n], x.g[n]);
-        q[n] = make_ccell(y.h[n], y.hu[n], y.hv[n], y.g[n]);
-    }
-    p[4].h = __shfl_down_sync(FULL, p[0].h, 1);
-    p[4].sq = __shfl_down_sync(FULL, p[0].sq, 1);
-    p[4].u = __shfl_down_sync(FULL, p[0].u, 1);
-    p[4].v = __shfl_down_sync(FULL, p[0].v, 1);
-    p[4].G = __shfl_down_sync(FULL, p[0].G, 1);
-    p[4].rs = __shfl_down_sync(FULL, p[0].rs, 1);
-    const T DRY = T(DRY_TOL);
-#pragma unroll
-    for (int n = 0; n < 4; ++n) {
-        bool m = false, me = false, ms = false;
-        if (HAS_MASK) {
-            const long long i = (long long)r * a.pitch + c + n;
-            m = c + n < nx && __ldg(a.nodata + i) != 0;
-            me = c + n + 1 < nx && __ldg(a.nodata + i + 1) != 0;
-            ms = south && c + n < nx && __ldg(a.nodata + i + a.pitch) != 0;
-        }
-        const bool ax = c + n + 1 < nx && (n < 3 || lane < 31) && (p[n].h > DRY || p[n + 1].h > DRY) && !(m || me);
-        const bool ay = south && c + n < nx && (p[n].h > DRY || q[n].h > DRY) && !(m || ms);
-        // without G the same value without the cubic; only active faces enter that (see cfl_rows)
-        if (ax) fold(p[n].G == T(0) && p[n + 1].G == T(0) ? face_speed_nog<T, false>(p[n], p[n + 1])
-                                                            : face_speed<T, false>(p[n], p[n + 1]));
-        if (ay) fold(p[n].G == T(0) && q[n].G == T(0) ? face_speed_nog<T, true>(p[n], q[n])
-                                                      : face_speed<T, true>(p[n], q[n]));
-    }
-}
-
-// Rows left to evaluate by a block of 8 warps.
+// Rows left to evaluate by a block of 8 warps, in chunks of CFL_CHUNK rows of an item.
 struct CflTasks {
     int count;
-    float bound[8 * CFL_MAX_ROWS];
-    unsigned short who[8 * CFL_MAX_ROWS];  // warp * CFL_MAX_ROWS + row of its item
+    float bound[8 * CFL_MAX_ROWS / CFL_CHUNK];
+    unsigned char warp[8 * CFL_MAX_ROWS / CFL_CHUNK], first[8 * CFL_MAX_ROWS / CFL_CHUNK], last[8 * CFL_MAX_ROWS / CFL_CHUNK];
 };
 
 // Wide items of a block, one per warp (`item`: this warp's, negative for none; `items`: all
 // warps').  Every warp forms its rows' bounds; the rows that
-// may hold the maximum, which tend to lie in few items, are shared out over the block.
-// Returns with `best` covering whatever the block's warps could not rule out.
+// may hold the maximum, which tend to lie in few items, are shared out over the block: a warp
+// evaluates every face of 31 columns of a chunk's rows, as a narrow item.
+// Returns with the maximum covering whatever the block's warps could not rule out.
 template <class T, bool HAS_MASK, bool VEC>
 __device__ __forceinline__ void cfl_wide_block(const CflArgs<T>& a, const int item, const int* items, CflTasks& tasks) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned long long seen = 0ull;  // the maximum as last read, in lane 0
     if (threadIdx.x == 0) tasks.count = 0;
     __syncthreads();
     if (item >= 0) {
@@ -372,7 +340,6 @@ __device__ __forceinline__ void cfl_wide_block(const CflArgs<T>& a, const int it
         }
         float b0 = 0.f, b1 = 0.f;
         cfl_wide_bounds<T, VEC>(a, st, b0, b1);
-        unsigned long long seen = 0ull;
         if (lane == 0) seen = *(volatile unsigned long long*)&a.scr->maxbits;
         const float known = (float)bits_speed(__shfl_sync(FULL, seen, 0), T(0));
 #pragma unroll
@@ -380,27 +347,38 @@ __device__ __forceinline__ void cfl_wide_block(const CflArgs<T>& a, const int it
             const float b = n ? b1 : b0;
             const bool todo = !(b < known) && st.R0 + 32 * n + lane < st.R1;  // (a NaN bound is not below it)
             const unsigned vote = __ballot_sync(FULL, todo);
-            int at = 0;
-            if (lane == 0 && vote) at = atomicAdd(&tasks.count, __popc(vote));
-            at = __shfl_sync(FULL, at, 0) + __popc(vote & ((1u << lane) - 1u));
-            if (todo) {
-                tasks.bound[at] = b;
-                tasks.who[at] = (unsigned short)(warp * CFL_MAX_ROWS + 32 * n + lane);
+            for (int k = 0; k < 32; k += CFL_CHUNK) {
+                const unsigned bits = vote >> k & ((1u << CFL_CHUNK) - 1u);
+                if (bits == 0u) continue;
+                const bool mine = todo && lane >= k && lane < k + CFL_CHUNK;
+                const unsigned most = __reduce_max_sync(FULL, mine ? __float_as_uint(b) : 0u);
+                if (lane == 0) {
+                    const int at = atomicAdd(&tasks.count, 1);
+                    tasks.bound[at] = __uint_as_float(most);
+                    tasks.warp[at] = (unsigned char)warp;
+                    tasks.first[at] = (unsigned char)(32 * n + k + __ffs(bits) - 1);
+                    tasks.last[at] = (unsigned char)(32 * n + k + 31 - __clz(bits));
+                }
             }
         }
     }
     __syncthreads();
-    for (int t = warp; t < tasks.count; t += 8) {
-        const int w = tasks.who[t] / CFL_MAX_ROWS, k = tasks.who[t] - w * CFL_MAX_ROWS;
-        unsigned long long seen = 0ull;
-        if (lane == 0) seen = *(volatile unsigned long long*)&a.scr->maxbits;
+    constexpr int PARTS = CFL_WIDE / CFL_NARROW;
+    for (int t = warp; t < PARTS * tasks.count; t += 8) {
+        const int q = t / PARTS, part = t - PARTS * q;
         seen = __shfl_sync(FULL, seen, 0);
-        if (tasks.bound[t] < (float)bits_speed(seen, T(0))) continue;
-        const CflStrip<T> st(a, items[w]);
+        if (tasks.bound[q] < (float)bits_speed(seen, T(0))) continue;
+        const CflStrip<T> st(a, items[tasks.warp[q]]);
+        const int c = st.c - 4 * lane + CFL_NARROW * part;
+        if (c >= a.nx) continue;
+        // (the maximum for the next chunk's test, in flight during this one)
+        unsigned long long next = 0ull;
+        if (lane == 0) next = *(volatile unsigned long long*)&a.scr->maxbits;
         speed_bits_t<T> best = 0;
-        cfl_wide_row<T, HAS_MASK, VEC>(a, st, st.R0 + k, best);
+        cfl_rows<T, HAS_MASK>(a, c, st.R0 + tasks.first[q], st.R0 + tasks.last[q] + 1, best);
         best = warp_max_bits(best);
         if (lane == 0 && (unsigned long long)best > seen) atomicMax(&a.scr->maxbits, (unsigned long long)best);
+        seen = next;
     }
 }
 
