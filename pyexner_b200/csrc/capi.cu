@@ -322,6 +322,7 @@ StageGeometry stage_tiles(int ny, int nx, int esize, int wx, int wy, int rows) {
     // bands of at least two rows (a ring row and its donors' row share a tile) that fit in
     // shared memory
     const size_t cap = STAGE_SMEM_MAX / esize;
+    rows = std::min(rows, std::max(2, ny));  // (a taller band is the whole grid)
     while (rows > 2 && pxb::stage_smem_elems(wx, rows + 5) > cap) --rows;
     g.nbands = std::max(1, std::min(ny / 2, (ny + rows - 1) / rows));
     g.band_rows = (ny + g.nbands - 1) / g.nbands;

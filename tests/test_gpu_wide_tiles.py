@@ -87,3 +87,13 @@ def test_float32_stays_at_the_general_path(warps, last):
     for f in PLANES:
         x, y = a[1][f], b[1][f]
         assert np.max(np.abs(x - y)) <= 1e-6 * max(1e-3, np.max(np.abs(y))), f
+
+
+@pytest.mark.parametrize("rows", [500, 2**31 - 1])
+def test_bands_taller_than_the_grid(rows):
+    """band_rows beyond the grid's rows asks for bands as tall as they get: the same bits."""
+    arrs, params, X, Y = case(80, 70, "fast", True)
+    a = run(arrs, params, X, Y, "float64", "fused", rows, 1, 2)
+    b = run(arrs, params, X, Y, "float64", "general", 0, 0, 2)
+    for f in PLANES:
+        assert np.array_equal(a[1][f], b[1][f], equal_nan=True), f
