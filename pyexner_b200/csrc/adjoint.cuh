@@ -7,12 +7,13 @@
 //   G = grass(h, hu, hv) or the constant pass-through      (:85-140)
 //   zb2 = zb1 - dt/dx * sum of Exner face fluxes            (:665-717)
 //   handlers
-// and the SSPRK2 average for the second stage.  The adjoint runs these backwards.  Each
-// cell gathers the contributions of its faces: the derivatives of a face's outputs with
-// respect to the cell's own inputs come from one evaluation of the same face formula on
-// DualN numbers seeded with those inputs (the neighbour held constant), so no face
-// arithmetic is written twice.  Masks and branches (wet/dry, activity, upwinding, the
-// correction zeroing) are taken from the forward values and carry no derivative.
+// and the SSPRK2 average for the second stage.  The adjoint runs these backwards.  The hydro
+// faces and the MPM grass factor are differentiated by hand (adj_exner_hydro_face restates
+// roe_exner_face, mpm_gradient restates mpm_grass: a change to one belongs in the other; the
+// transpose tests compare them through the tangent model, which runs the forward formulas).
+// The Exner and CFL faces are evaluated by the forward formulas on DualN numbers seeded with
+// the cells' inputs.  Masks and branches (wet/dry, activity, upwinding, the correction
+// zeroing) are taken from the forward values and carry no derivative.
 // Handlers are linear in the state for every kind except ConstantOutflux (refused):
 // their adjoint moves the boundary cells' adjoints to the donors (scatter-add).
 #pragma once

@@ -9,7 +9,7 @@
 //     do not resolve run on the general stage path (re_general.cuh), which applies the
 //     handlers one after another on the device;
 //   * turn the sediment matrix into per-class constants;
-//   * size the warp strips / row bands of the stage and CFL kernels to the device;
+//   * choose the tiles of the stage kernel and the items of the CFL kernel for the device;
 //   * capture the fixed-step integrator loops into CUDA graphs and replay them.
 #include <cuda_runtime.h>
 
@@ -415,7 +415,8 @@ int arena_copy(DevArena* A, void* dst, const void* src, size_t bytes) {
 }
 
 // Boundary cells up to which a layout's handlers may be applied in one launch (each of its
-// levels must also fit: pxb::BC_SET_CHUNKS).
+// levels must also fit: pxb::BC_SET_CHUNKS).  Six handlers: 6 us in one launch, 26 (512 cells
+// each) to 32 us (4096 each) in two launches per handler.
 constexpr int BC_SET_CELLS = 16384;
 
 // `total`: boundary cells of all handlers.
@@ -2548,6 +2549,10 @@ int pxb_re_ens_create(const pxb_re_ens_config* cfg, pxb_re_ens** out) {
     E->dtype = cfg->dtype;
     E->mpm = cfg->mpm;
     E->nm = cfg->nmembers;
+    // (24 to 64 rows differ by a few per cent, either way: us per SSPRK2 step with 32, 40, 48 and
+    // 64 rows, float32: 24 members of 128 to 640 cells a side 316, 304, 297, 300; 8 of 512^2 222,
+    // 201, 191, 214; 2 of 2048^2 603, 622, 607, 598; float64: 1243, 1250, 1259, 1224; 946, 926,
+    // 929, 829; 2682, 2707, 2752, 2811.  pxb_re_ens_autotune times them on the members at hand.)
     E->band_rows = cfg->band_rows > 0 ? cfg->band_rows : 40;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||

@@ -50,12 +50,6 @@ __device__ inline Dual d_cbrt(Dual x) {
     const double c = cbrt(x.v);
     return Dual(c, chain(x.d, 1.0 / (3.0 * c * c)));
 }
-__device__ inline Dual d_pow(Dual x, Dual y) {
-    const double p = pow(x.v, y.v);
-    double t = chain(x.d, y.v * pow(x.v, y.v - 1.0));
-    if (y.d != 0.0) t += log(x.v) * p * y.d;
-    return Dual(p, t);
-}
 // x^(4/3), x^(3/2): the values of d_pow43 / d_pow32, the derivatives without a second power
 __device__ inline Dual d_pow43(Dual x) {
     const double c = cbrt(x.v);

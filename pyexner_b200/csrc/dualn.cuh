@@ -71,22 +71,6 @@ struct DualN {
         const double s = sqrt(x.v);
         return x.apply(s, 0.5 / s);
     }
-    friend __device__ DualN d_cbrt(const DualN& x) {
-        const double c = cbrt(x.v);
-        return x.apply(c, 1.0 / (3.0 * c * c));
-    }
-    friend __device__ DualN d_pow(const DualN& x, const DualN& y) {  // constant exponents only
-        const double p = pow(x.v, y.v);
-        return x.apply(p, y.v * pow(x.v, y.v - 1.0));
-    }
-    friend __device__ DualN d_pow43(const DualN& x) {
-        const double c = cbrt(x.v);
-        return x.apply(x.v * c, (4.0 / 3.0) * c);
-    }
-    friend __device__ DualN d_pow32(const DualN& x) {
-        const double s = sqrt(x.v);
-        return x.apply(x.v * s, 1.5 * s);
-    }
     friend __device__ DualN d_acos(const DualN& x) { return x.apply(acos(x.v), -1.0 / sqrt(1.0 - x.v * x.v)); }
     friend __device__ DualN d_cos(const DualN& x) { return x.apply(cos(x.v), -sin(x.v)); }
     friend __device__ DualN fabs(const DualN& x) {

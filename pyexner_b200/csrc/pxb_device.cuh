@@ -35,8 +35,6 @@ __device__ __forceinline__ float d_sqrt(float x) { return sqrtf(x); }
 __device__ __forceinline__ double d_sqrt(double x) { return sqrt(x); }
 __device__ __forceinline__ float d_cbrt(float x) { return cbrtf(x); }
 __device__ __forceinline__ double d_cbrt(double x) { return cbrt(x); }
-__device__ __forceinline__ float d_pow(float x, float y) { return powf(x, y); }
-__device__ __forceinline__ double d_pow(double x, double y) { return pow(x, y); }
 __device__ __forceinline__ float d_acos(float x) { return acosf(x); }
 __device__ __forceinline__ double d_acos(double x) { return acos(x); }
 __device__ __forceinline__ float d_cos(float x) { return cosf(x); }
@@ -152,8 +150,7 @@ __device__ __forceinline__ HCell<T> make_hcell(T h, T hu, T hv, T zb, T z, T nb)
 // WARP: every lane of the warp evaluates a face, so warp votes may skip work.  Where every
 // face is subcritical (both cells and the Roe state: |u| < c), no entropy fix applies, the
 // first wave goes to cell i and the third to cell j: the speeds u -+ c of the cells and the
-// wave split are left out (the same bits but for the sign of zeros; measured on the float32
-// 2048^2 Gaussian bed together with the sediment vote of the stage kernel).
+// wave split are left out (the same bits but for the sign of zeros).
 template <class T, bool YF, bool WARP = false>
 __device__ __forceinline__ void roe_exner_face(const HCell<T>& I, const HCell<T>& J, T dx, T P[3], T M[3]) {
     const T uhi = YF ? -I.v : I.u, vhi = YF ? I.u : I.v;
@@ -425,7 +422,9 @@ __device__ __forceinline__ bool mpm_may_move(T h, T hu, T hv, const SedTable<T>&
     return h > T(DRY_TOL) && !(um * um * um * S.k_move <= h);
 }
 
-// Meyer-Peter & Mueller grass factor of one cell (roe_exner.py:85-130).
+// Meyer-Peter & Mueller grass factor of one cell (roe_exner.py:85-130).  The float32 form votes
+// over the whole warp: every thread of a warp that has not exited must call it together, never
+// under a condition that only some lanes meet.
 template <class T>
 __device__ __forceinline__ T mpm_grass(T h, T hu, T hv, bool nodata, const SedTable<T>& S) {
     if constexpr (is_f32<T>()) {

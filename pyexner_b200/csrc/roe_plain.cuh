@@ -28,8 +28,8 @@ struct RoeArgs {
 };
 
 // Roe fluctuations with the wet/dry thrust and beta limiter (roe.py:32-249).  YF (the
-// y-face orientation) is a runtime flag, so that the four threads of a cell, two on
-// x-faces and two on y-faces, run one code path.
+// y-face orientation) is a runtime flag, so that the warp with both the last x-faces and the
+// first y-faces of a tile runs one code path.
 template <class T>
 __device__ __forceinline__ void roe_plain_face(T hi, T hui, T hvi, T zi, T ni, T hj, T huj, T hvj, T zj, T nj, T dx,
                                                const bool YF, T P[3], T M[3]) {
