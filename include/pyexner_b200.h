@@ -219,8 +219,8 @@ int pxb_re_run(pxb_re_plan* plan, const pxb_re_fields* a, const pxb_re_fields* b
  * each stage adds dt dx times its boundary sum, times 1/2 under SSPRK2.  Then
  * volume(end) - volume(start) + outflow vanishes to rounding.  Fused stage path only
  * (PXB_ERR_UNSUPPORTED otherwise); acc_dev = NULL switches it off.  The first call with
- * an accumulator allocates the per-item partial array (16 bytes per work item of
- * one-row bands, the most items a band geometry can have). */
+ * an accumulator allocates the per-tile partial array (16 bytes per tile of one-row bands,
+ * the most tiles a plan can have). */
 int pxb_re_volume(pxb_re_plan* plan, const pxb_re_fields* f, double* volumes, void* stream);
 int pxb_re_set_budget(pxb_re_plan* plan, double* acc_dev);
 
@@ -251,8 +251,7 @@ int pxb_re_jvp_run(pxb_re_plan* plan, const pxb_re_fields* a, const pxb_re_field
  * (dJ/du for h, hu, hv, z_b, G) and receives the adjoint of a0.  The steps are redone
  * forward with a checkpoint every `checkpoint_every` steps (0: 32) and undone segment by
  * segment: each stage backwards (handlers, Exner update, grass factor, corrections, hydro
- * update), with local Jacobians of the faces from multi-tangent dual numbers, and the
- * dependence of dt on the state through the fastest face.  pxb_re_vjp_init: `f` is the
+ * update), and the dependence of dt on the state through the fastest face.  pxb_re_vjp_init: `f` is the
  * state BEFORE init; `fbar` (in: adjoint after init, out: before) goes back through the
  * handlers and the grass factor.  Handlers of every kind but ConstantOutflux.  Allocates
  * its checkpoints for the call; synchronises `stream`.  pxb_re_vjp_run_in (declared with the

@@ -23,8 +23,8 @@
 // every cell is wet, the grass factor and the Exner update where no cell near the warp's
 // carries sediment.
 //
-// Bound by instruction issue (82 % of issue slots in the plain float32 stage at 4096^2,
-// DRAM at 35 %).  The tile replaced a warp that marched down a band with all phases in one
+// Bound by instruction issue (79 and 77 % of issue slots in the two float32 stages at 2048^2,
+// DRAM at 18 and 28 %).  The tile replaced a warp that marched down a band with all phases in one
 // register pipeline: that needed 118 registers (16 warps per SM, 74 % of issue slots),
 // moved 35 values a row between pipeline stages, repeated 1.41 times the cells (32 columns
 // for 26) and ran 11 rows before its first store, which set the time of small grids.
