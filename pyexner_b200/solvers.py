@@ -201,7 +201,8 @@ def step_fn_roeexner(state, time, dt, mask, config, avg=None):
     plan = _re_plan(state, mask, config)
     # the general path carries n through the handlers; the fused path leaves it as it is
     fields = ("h", "hu", "hv", "z_b", "G") + (("n",) if plan.path == _lib.PATH_GENERAL else ())
-    new = {f: plane_like(state.h) for f in fields}
+    (ny, nx), dtype, device, pitch = state.h.shape, state.h.dtype, state.h.device, state.pitch
+    new = {f: alloc_plane(ny, nx, dtype, device, pitch) for f in fields}  # (planes of the state's pitch)
     out = state.replace(**new)
     dtt = _dt_tensor(dt, state)
     _lib.call("pxb_re_stage", plan.handle, ctypes.byref(state.c_fields()), ctypes.byref(out.c_fields()),
