@@ -94,8 +94,10 @@ static inline CflItems cfl_items(int ny, int nx, bool wide, int sm_count) {
     return g;
 }
 // A plan's items.  Below the line a wide item's bounds cost more than evaluating every face of
-// narrow items (float32 731 x 1203: 15.7 us narrow, 27.5 wide; 1024^2 11.2 both; 2048^2 43.8
-// and 19.3.  float64 512^2: 22.8 and 33; 1024^2 76 and 48).
+// narrow items.  us narrow / wide, at rest and with bedload everywhere: float32 770^2 7.1 / 9.5
+// and 11.9 / 13.0, 1026^2 8.5 / 10.0 and 16.3 / 14.8, 1400^2 11.5 / 13.7 and 25.2 / 17.9, 2050^2
+// 19.5 / 15.8 and 47.9 / 25.6; float64 640^2 15.8 / 15.1 and 37.6 / 82, 770^2 21.1 / 16.5 and
+// 56.8 / 44.8, 1026^2 31 / 17 and 87 / 50, 2050^2 115 / 36 and 305 / 93.
 static inline CflItems cfl_items(int ny, int nx, int esize, int sm_count) {
     return cfl_items(ny, nx, (long long)ny * nx > (esize == 8 ? 500000 : 1200000), sm_count);
 }
